@@ -770,6 +770,17 @@ bool make_rtm_map(const Plan& p, CUtensorMap* map, int* mbox) {
 // quarter warp on 8 distinct 16-byte bank groups in all passes at N = 1536.
 constexpr int kFftThreadsF = 384;
 
+// Threads of one staged CTA.  Every variant fills the register file
+// (168 registers x 384 threads per SM): at N = 1536 one line takes the whole
+// shared memory, so one CTA has them all; the shorter lines leave room for
+// several CTAs per SM, whose barriers and record stores then overlap, and a
+// pass of theirs has fewer items than 384 threads could take (N / F0 or N / M
+// per pair).  FFT ms at 384 threads -> here: L = 255, Nr = 129 (N = 768)
+// 2.64 -> 2.42 (160 threads 2.53); L = 127, Nr = 65 (N = 384) 0.390 -> 0.292
+// (128 threads 0.296); L = 63, Nr = 65 (N = 192) 0.153 -> 0.081 (96 threads
+// 0.085); L = 31, Nr = 33 (N = 96) 0.034 -> 0.016 (64 threads 0.018).
+__host__ __device__ constexpr int ff_threads(int n) { return n == 768 ? 192 : n == 384 ? 96 : n == 192 ? 64 : n == 96 ? 32 : kFftThreadsF; }
+
 __host__ __device__ constexpr int ff_mid(int n) { return (n % 64 == 0 && (n / 64 == 3 || n / 64 == 6 || n / 64 == 12 || n / 64 == 24)) ? 16 : 4; }
 __host__ __device__ constexpr int ff_first(int n) { return n / (4 * ff_mid(n)); }
 __device__ __forceinline__ int swf(int i) { return i ^ (((i >> 3) ^ (i >> 6)) & 7); }
@@ -1241,7 +1252,7 @@ __device__ void ff_store_records(const double2* z, const Plan& P, double* rtm, i
 // NT threads: fewer threads leave more registers to each for the fused
 // products of many fields (the unstaged variants)
 template <int N, int MVB, int MSB, int MVF, int MSF, bool PR, int PK, bool STG = true, int NT = kFftThreadsF>
-__global__ void __launch_bounds__(NT, 1)
+__global__ void __launch_bounds__(NT, kFftThreadsF / NT)
     k_fft_cycle_f(Plan P, int line0, int nlines, const __grid_constant__ CUtensorMap tmap, int tma, int mbox) {
   extern __shared__ double4 smraw[];
   constexpr int NP = N + 1;
@@ -1336,7 +1347,7 @@ __global__ void __launch_bounds__(NT, 1)
   }
 }
 
-template <int N, int MVB, int MSB, int MVF, int MSF, bool PR, int PK, bool STG = true, int NT = kFftThreadsF>
+template <int N, int MVB, int MSB, int MVF, int MSF, bool PR, int PK, bool STG = true, int NT = ff_threads(N)>
 cudaError_t run_cycle_fk(const Plan& p, cudaStream_t s) {
   auto kern = k_fft_cycle_f<N, MVB, MSB, MVF, MSF, PR, PK, STG, NT>;
   const int npair = ((p.ncb > p.ncf ? p.ncb : p.ncf) + 1) / 2;
