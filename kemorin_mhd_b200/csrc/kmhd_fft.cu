@@ -16,12 +16,12 @@
 // Products: cal_cross_prod_w_coef_smp, cal_vec_scalar_prod_w_coef_smp,
 // cal_dot_prod_w_coef_smp (CORE_src/BASE/cal_products_smp.f90) as called by
 // nonlinear_terms_in_rtp (MHD_src/sph_MHD/cal_nonlinear_sph_MHD.f90:64-128).
-#include <algorithm>
-#include <utility>
-
 #include <cuda.h>
 
+#include <algorithm>
 #include <cstring>
+#include <type_traits>
+#include <utility>
 
 #include "kmhd_internal.cuh"
 
@@ -29,8 +29,9 @@ namespace kmhd {
 namespace {
 
 constexpr int kFftThreads = 256;
+constexpr int kRtmOrders = 1 << kRtmShift;
 
-// mbarrier + TMA tensor load (staging of a line's spectra)
+// mbarrier + bulk copies (staging of a line's spectra)
 constexpr long long kFftSpinCap = 1ll << 22;  // try_wait rounds (each may suspend for microseconds)
 __device__ __forceinline__ unsigned ssa(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ bool fbar_wait(unsigned long long* b, unsigned parity, long long cap = kFftSpinCap) {
@@ -158,647 +159,83 @@ struct TwiddleRun {
   }
 };
 
-// One in-place DIF (+) pass over npair sequences: butterfly, then twiddle.
-template <int R>
-__device__ void dif_pass(double2* z, int npair, int N, int span, const double2* __restrict__ tw) {
-  const int s = span / R, nbf = N / R, stw = N / span;
-  for (int it = threadIdx.x; it < npair * nbf; it += blockDim.x) {
-    const int pp = it / nbf, rem = it % nbf;
-    const int j = rem % s, b = rem / s;
-    double2* base = z + pp * N + b * span + j;
-    double2 x[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) x[r] = base[r * s];
-    DFT<R, +1>::run(x);
-    base[0] = x[0];
-#pragma unroll
-    for (int q = 1; q < R; ++q) base[q * s] = cmul(x[q], twd<+1>(tw, j * q * stw));
-  }
-}
+// ---------------------------------------------------------------------------
+// Passes of run-time N: the radices P.fac (composite, at most 16) over nseq
+// sequences zs entries apart.  Entry i of a sequence sits at index i ^ ((i >> 3
+// ^ i >> 6) & 7) where N is a multiple of eight (power-of-two strides would
+// meet in few banks), at i otherwise.
+struct Seqs {
+  double2* z;
+  int n, zs, N, msk;
+  __device__ Seqs(double2* z_, int n_, int zs_, int N_) : z(z_), n(n_), zs(zs_), N(N_), msk(N_ % 8 == 0 ? 7 : 0) {}
+  __device__ __forceinline__ int ix(int i) const { return i ^ (((i >> 3) ^ (i >> 6)) & msk); }
+};
 
-// One in-place DIT (-) pass, the transpose of dif_pass.
-template <int R>
-__device__ void dit_pass(double2* z, int npair, int N, int span, const double2* __restrict__ tw) {
-  const int s = span / R, nbf = N / R, stw = N / span;
-  for (int it = threadIdx.x; it < npair * nbf; it += blockDim.x) {
-    const int pp = it / nbf, rem = it % nbf;
-    const int j = rem % s, b = rem / s;
-    double2* base = z + pp * N + b * span + j;
-    double2 x[R];
-    x[0] = base[0];
-#pragma unroll
-    for (int q = 1; q < R; ++q) x[q] = cmul(base[q * s], twd<-1>(tw, j * q * stw));
-    DFT<R, -1>::run(x);
-#pragma unroll
-    for (int r = 0; r < R; ++r) base[r * s] = x[r];
-  }
-}
-
-__device__ void dif_dispatch(int R, double2* z, int npair, int N, int span, const double2* tw) {
-  switch (R) {
-    case 8: dif_pass<8>(z, npair, N, span, tw); break;
-    case 4: dif_pass<4>(z, npair, N, span, tw); break;
-    case 2: dif_pass<2>(z, npair, N, span, tw); break;
-    case 3: dif_pass<3>(z, npair, N, span, tw); break;
-    default: dif_pass<5>(z, npair, N, span, tw); break;
-  }
-}
-__device__ void dit_dispatch(int R, double2* z, int npair, int N, int span, const double2* tw) {
-  switch (R) {
-    case 8: dit_pass<8>(z, npair, N, span, tw); break;
-    case 4: dit_pass<4>(z, npair, N, span, tw); break;
-    case 2: dit_pass<2>(z, npair, N, span, tw); break;
-    case 3: dit_pass<3>(z, npair, N, span, tw); break;
-    default: dit_pass<5>(z, npair, N, span, tw); break;
-  }
-}
-
-// Complex spectrum of pair pp at frequency k from staged records
-// st[(m*nc + c)*2 + {0: a, 1: b}], m <= L.  z = X_{2pp} + i X_{2pp+1},
-// X_c[m] = (a - i b)/2 for m > 0, X_c[0] = a, X_c[N-m] = conj(X_c[m]).
-// rs: doubles between the records of consecutive orders (staged: 2 nc; in
-// place in rtm: the order stride of the rtm layout)
-__device__ __forceinline__ double2 spec_at(const double* st, int nc, int nv, int pp, int k, int N, int L,
-                                           long long rs) {
-  int m;
-  bool mirror;
-  if (k <= L) { m = k; mirror = false; }
-  else if (k >= N - L) { m = N - k; mirror = true; }
-  else return make_double2(0.0, 0.0);
-  const double* rec = st + m * rs;
-  const double* r0 = rec + rec_off(2 * pp, nv);
-  const double a0 = r0[0], b0 = r0[1];
-  double a1 = 0.0, b1 = 0.0;
-  if (2 * pp + 1 < nc) {
-    const double* r1 = rec + rec_off(2 * pp + 1, nv);
-    a1 = r1[0];
-    b1 = r1[1];
-  }
-  if (m == 0) return make_double2(a0, a1);
-  return mirror ? make_double2(0.5 * a0 - 0.5 * b1, 0.5 * b0 + 0.5 * a1)
-                : make_double2(0.5 * a0 + 0.5 * b1, 0.5 * a1 - 0.5 * b0);
-}
-
-// First DIF pass: input from the spectra (staged records, order stride rs =
-// 2 nc; or the rtm records in place, rs = their order stride), output into z.
-template <int R>
-__device__ void dif_first(const double* st, int nc, int nv, double2* z, int npair, int N, int L,
-                          const double2* __restrict__ tw, long long rs) {
-  const int s = N / R, nbf = N / R;
-  for (int it = threadIdx.x; it < npair * nbf; it += blockDim.x) {
-    const int pp = it / nbf, j = it % nbf;
-    double2 x[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) x[r] = spec_at(st, nc, nv, pp, j + r * s, N, L, rs);
-    DFT<R, +1>::run(x);
-    double2* base = z + pp * N + j;
-    base[0] = x[0];
-#pragma unroll
-    for (int q = 1; q < R; ++q) base[q * s] = cmul(x[q], twd<+1>(tw, j * q));
-  }
-}
-__device__ void dif_first_dispatch(int R, const double* st, int nc, int nv, double2* z, int npair,
-                                   int N, int L, const double2* tw, long long rs = -1) {
-  if (rs < 0) rs = 2LL * nc;
-  switch (R) {
-    case 8: dif_first<8>(st, nc, nv, z, npair, N, L, tw, rs); break;
-    case 4: dif_first<4>(st, nc, nv, z, npair, N, L, tw, rs); break;
-    case 2: dif_first<2>(st, nc, nv, z, npair, N, L, tw, rs); break;
-    case 3: dif_first<3>(st, nc, nv, z, npair, N, L, tw, rs); break;
-    default: dif_first<5>(st, nc, nv, z, npair, N, L, tw, rs); break;
-  }
-}
-
-__device__ void dif_rest(double2* z, int npair, int N, const Plan& P, const double2* tw) {
-  int span = N / P.fac[0];
-  for (int f = 1; f < P.nfac; ++f) {
-    dif_dispatch(P.fac[f], z, npair, N, span, tw);
-    __syncthreads();
-    span /= P.fac[f];
-  }
-}
-
-__device__ void dit_all(double2* z, int npair, int N, const Plan& P, const double2* tw) {
-  int spans[kMaxFftFactors];
-  int span = N;
-  for (int f = 0; f < P.nfac; ++f) {
-    spans[f] = span;
-    span /= P.fac[f];
-  }
-  for (int f = P.nfac - 1; f >= 0; --f) {
-    dit_dispatch(P.fac[f], z, npair, N, spans[f], tw);
-    __syncthreads();
-  }
-}
-
-// Stage the records of line (th, r) for all m into st via cp.async (16 B each).
-__device__ void prefetch_line(double* st, const double* rtm, int nc, const Plan& P, int th, int r) {
-  const long long strideM = (long long)P.nth * P.nr * nc * 2;
-  const double* base = rtm + rtm_off(P, 0, th, r, nc);
-  const int n = (P.L + 1) * nc;
-  for (int it = threadIdx.x; it < n; it += blockDim.x) {
-    const int m = it / nc, c = it % nc;
-    cp_async16(st + (m * nc + c) * 2, base + m * strideM + c * 2);
-  }
-  cp_async_commit();
-}
-
-// Natural-order forward spectra in z -> (a_m, b_m), m <= L, into rtm.
-__device__ void store_line(const double2* z, int npair, const Plan& P, double* rtm, int nc, int nv, int th, int r) {
+// Complex spectrum of pair pp at frequency k from a line's records.  z = x + i y,
+// X[m] = (a - i b)/2 for m > 0, X[0] = a, X[N-m] = conj(X[m]).
+// line: the line's block rows, bs doubles apart (staged: rtm_row; in place in
+// rtm: rtm_row nr nth).
+__device__ __forceinline__ double2 spec_at(const Plan& P, const double* line, long long bs, int nc, int pp, int k) {
+  // no branch around the loads: a butterfly's loads go out together (zero-band
+  // frequencies load order 0)
   const int N = P.nph, L = P.L;
-  const double aN = 1.0 / (double)N;
-  const long long strideM = (long long)P.nth * P.nr * nc * 2;
-  double* base = rtm + rtm_off(P, 0, th, r, nc);
-  for (int it = threadIdx.x; it < (L + 1) * npair; it += blockDim.x) {
-    const int m = it / npair, pp = it % npair;
-    const double2* zp = z + pp * N;
-    const double2 zm = zp[m];
-    double a0, b0, a1, b1;
-    if (m == 0) {
-      a0 = zm.x * aN; a1 = zm.y * aN; b0 = 0.0; b1 = 0.0;
-    } else {
-      const double2 wm = zp[N - m];
-      a0 = (zm.x + wm.x) * aN;
-      b0 = (wm.y - zm.y) * aN;
-      a1 = (zm.y + wm.y) * aN;
-      b1 = (zm.x - wm.x) * aN;
-    }
-    double* rec = base + m * strideM;
-    *reinterpret_cast<double2*>(rec + rec_off(2 * pp, nv)) = make_double2(a0, b0);
-    if (2 * pp + 1 < nc) *reinterpret_cast<double2*>(rec + rec_off(2 * pp + 1, nv)) = make_double2(a1, b1);
-  }
-}
-
-// Vector a of the backward fields, selected without dynamic register indexing.
-template <int MV>
-__device__ __forceinline__ void selvec(const double* in, int a, double& x0, double& x1, double& x2) {
-  x0 = in[0]; x1 = in[1]; x2 = in[2];
-#pragma unroll
-  for (int v = 1; v < MV; ++v)
-    if (a == v) { x0 = in[3 * v]; x1 = in[3 * v + 1]; x2 = in[3 * v + 2]; }
-}
-template <int MS>
-__device__ __forceinline__ double selscl(const double* s, int b) {
-  double x = s[0];
-#pragma unroll
-  for (int q = 1; q < MS; ++q)
-    if (b == q) x = s[q];
-  return x;
-}
-
-// Pointwise products on the digit-reversed grid.  MV*/MS* are compile-time
-// maxima; the plan's counts are <= them (products are ordered vectors first).
-template <int MVB, int MSB, int MVF, int MSF>
-__device__ void products(double2* z, int N, const Plan& P) {
-  constexpr int MCF = 3 * MVF + MSF;
-  const int nvb = P.nvb, nsb = P.nsb, nvf = P.nvf, nsf = P.nsf;
-  for (int pos = threadIdx.x; pos < N; pos += blockDim.x) {
-    double vin[3 * MVB > 0 ? 3 * MVB : 1], sin_[MSB > 0 ? MSB : 1];
-#pragma unroll
-    for (int c = 0; c < 3 * MVB; ++c)
-      if (c < 3 * nvb) {
-        const double2 v = z[(c >> 1) * N + pos];
-        vin[c] = (c & 1) ? v.y : v.x;
-      }
-#pragma unroll
-    for (int q = 0; q < MSB; ++q)
-      if (q < nsb) {
-        const int c = 3 * nvb + q;
-        const double2 v = z[(c >> 1) * N + pos];
-        sin_[q] = (c & 1) ? v.y : v.x;
-      }
-    double out[MCF > 0 ? MCF : 1];
-#pragma unroll
-    for (int i = 0; i < MVF; ++i) {
-      if (i < nvf) {
-        const int kind = P.pkind[i];
-        const double cf = P.pcoef[i];
-        double x0, x1, x2;
-        selvec<MVB>(vin, P.pa[i], x0, x1, x2);
-        if (kind == KMHD_PROD_CROSS) {
-          double y0, y1, y2;
-          selvec<MVB>(vin, P.pb[i], y0, y1, y2);
-          out[3 * i + 0] = (x1 * y2 - x2 * y1) * cf;
-          out[3 * i + 1] = (x2 * y0 - x0 * y2) * cf;
-          out[3 * i + 2] = (x0 * y1 - x1 * y0) * cf;
-        } else {
-          const double s = selscl<MSB>(sin_, P.pb[i]);
-          out[3 * i + 0] = x0 * s * cf;
-          out[3 * i + 1] = x1 * s * cf;
-          out[3 * i + 2] = x2 * s * cf;
-        }
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < MSF; ++j) {
-      if (j < nsf) {
-        const int q = nvf + j;
-        const int kind = P.pkind[q];
-        const double cf = P.pcoef[q];
-        double o;
-        if (kind == KMHD_PROD_DOT) {
-          double x0, x1, x2, y0, y1, y2;
-          selvec<MVB>(vin, P.pa[q], x0, x1, x2);
-          selvec<MVB>(vin, P.pb[q], y0, y1, y2);
-          o = (x0 * y0 + x1 * y1 + x2 * y2) * cf;
-        } else {
-          o = selscl<MSB>(sin_, P.pa[q]) * selscl<MSB>(sin_, P.pb[q]) * cf;
-        }
-        // output component 3*nvf + j: compile-time slot only when nvf == MVF
-        out[3 * MVF + j] = o;
-      }
-    }
-    // dense output order: vectors [0, 3*nvf), then scalars; compile-time slots
-    const int ncf = 3 * nvf + nsf;
-    double dense[MCF > 0 ? MCF : 1];
-#pragma unroll
-    for (int c = 0; c < MCF; ++c) {
-      double v = 0.0;
-      if (c < 3 * MVF) v = out[c < 3 * MVF ? c : 0];
-      if (c >= 3 * nvf) {
-        v = 0.0;
-#pragma unroll
-        for (int j = 0; j < MSF; ++j)
-          if (c == 3 * nvf + j) v = out[3 * MVF + j];
-      }
-      dense[c] = v;
-    }
-#pragma unroll
-    for (int c = 0; c < MCF; c += 2) {
-      if (c < ncf) {
-        const double hi = (c + 1 < MCF && c + 1 < ncf) ? dense[c + 1 < MCF ? c + 1 : c] : 0.0;
-        z[(c >> 1) * N + pos] = make_double2(dense[c], hi);
-      }
-    }
-  }
-}
-
-template <int MVB, int MSB, int MVF, int MSF>
-__global__ void __launch_bounds__(kFftThreads) k_fft_cycle(Plan P, int line0, int nlines) {
-  extern __shared__ double4 smraw[];
-  const int N = P.nph;
-  const int npb = (P.ncb + 1) / 2, npf = (P.ncf + 1) / 2;
-  const int npair = npb > npf ? npb : npf;
-  double2* z = reinterpret_cast<double2*>(smraw);
-  double* st = reinterpret_cast<double*>(z + npair * N);
-  int line = line0 + blockIdx.x;
-  if (line >= nlines) return;
-  prefetch_line(st, P.rtm_b, P.ncb, P, line % P.nth, line / P.nth);
-  while (line < nlines) {
-    const int th = line % P.nth, r = line / P.nth;
-    cp_async_wait<0>();
-    __syncthreads();
-    dif_first_dispatch(P.fac[0], st, P.ncb, P.nvb, z, npb, N, P.L, P.twid);
-    __syncthreads();
-    const int next = line + gridDim.x;
-    if (next < nlines) prefetch_line(st, P.rtm_b, P.ncb, P, next % P.nth, next / P.nth);
-    dif_rest(z, npb, N, P, P.twid);
-    products<MVB, MSB, MVF, MSF>(z, N, P);
-    __syncthreads();
-    dit_all(z, npf, N, P, P.twid);
-    store_line(z, npf, P, P.rtm_f, P.ncf, P.nvf, th, r);
-    __syncthreads();
-    line = next;
-  }
-}
-
-// Lines whose grid fits in shared memory but not together with the staged
-// spectra of the next line (many fields, e.g. 14 + 16 components at
-// Nphi = 1536: 197 KB of grid pairs): the first pass reads the line's spectra
-// in place from the rtm records, everything else as k_fft_cycle.
-template <int MVB, int MSB, int MVF, int MSF>
-__global__ void __launch_bounds__(kFftThreads) k_fft_cycle_direct(Plan P, int line0, int nlines) {
-  extern __shared__ double4 smraw[];
-  const int N = P.nph;
-  const int npb = (P.ncb + 1) / 2, npf = (P.ncf + 1) / 2;
-  double2* z = reinterpret_cast<double2*>(smraw);
-  const long long rs = (long long)P.nth * P.nr * P.ncb * 2;
-  for (int line = line0 + blockIdx.x; line < nlines; line += gridDim.x) {
-    const int th = line % P.nth, r = line / P.nth;
-    dif_first_dispatch(P.fac[0], P.rtm_b + rtm_off(P, 0, th, r, P.ncb), P.ncb, P.nvb, z, npb, N, P.L, P.twid, rs);
-    __syncthreads();
-    dif_rest(z, npb, N, P, P.twid);
-    products<MVB, MSB, MVF, MSF>(z, N, P);
-    __syncthreads();
-    dit_all(z, npf, N, P, P.twid);
-    store_line(z, npf, P, P.rtm_f, P.ncf, P.nvf, th, r);
-    __syncthreads();
-  }
+  const bool mirror = k >= N - L, zero = k > L && !mirror;
+  const int m = mirror ? N - k : zero ? 0 : k;
+  const bool two = 2 * pp + 1 < nc;
+  const double* s = line + (m >> P.mbs) * bs + rtm_pair(P, m, pp, nc);
+  const double2 c0 = *reinterpret_cast<const double2*>(s);
+  double2 c1 = *reinterpret_cast<const double2*>(s + (two ? 2 : 0));
+  const double h = zero ? 0.0 : m == 0 ? 1.0 : 0.5;
+  const double h1 = two ? h : 0.0, hs = m == 0 ? 0.0 : mirror ? -h : h, hs1 = m == 0 ? 0.0 : mirror ? -h1 : h1;
+  // m = 0: (a_x, a_y); else x / 2 -+ i y / 2 of the two components
+  return m == 0 ? make_double2(h * c0.x, h1 * c1.x) : make_double2(h * c0.x + hs1 * c1.y, h1 * c1.x - hs * c0.y);
 }
 
 // ---------------------------------------------------------------------------
-// Wide lines (one line of every component does not fit in shared memory, e.g.
-// Nphi = 3072 with 10 components): the pairs go through shared memory one at a
-// time.  The cycle keeps the line's grid in a per-CTA global scratch
-// (pairs x N x 16 bytes, L2-resident), forms the products there and runs the
-// forward transforms pair by pair from it.
-
-// First inverse pass of pair pp only: spectra from the staged records, output z[0 .. N).
-template <int R>
-__device__ void dif_first_one(const double* st, int nc, int nv, int pp, double2* z, int N, int L,
-                              const double2* __restrict__ tw, long long rs) {
-  const int s = N / R;
-  for (int j = threadIdx.x; j < s; j += blockDim.x) {
-    double2 x[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) x[r] = spec_at(st, nc, nv, pp, j + r * s, N, L, rs);
-    DFT<R, +1>::run(x);
-    z[j] = x[0];
-#pragma unroll
-    for (int q = 1; q < R; ++q) z[j + q * s] = cmul(x[q], twd<+1>(tw, j * q));
-  }
-}
-__device__ void dif_first_one_dispatch(int R, const double* st, int nc, int nv, int pp, double2* z, int N, int L,
-                                       const double2* tw, long long rs) {
-  switch (R) {
-    case 8: dif_first_one<8>(st, nc, nv, pp, z, N, L, tw, rs); break;
-    case 4: dif_first_one<4>(st, nc, nv, pp, z, N, L, tw, rs); break;
-    case 2: dif_first_one<2>(st, nc, nv, pp, z, N, L, tw, rs); break;
-    case 3: dif_first_one<3>(st, nc, nv, pp, z, N, L, tw, rs); break;
-    default: dif_first_one<5>(st, nc, nv, pp, z, N, L, tw, rs); break;
-  }
-}
-// Natural-order forward spectrum of pair q in z -> (a_m, b_m), m <= L, into rtm.
-__device__ void store_one(const double2* z, int q, const Plan& P, double* rtm, int nc, int nv, int th, int r) {
-  const int N = P.nph, L = P.L;
-  const double aN = 1.0 / (double)N;
-  const long long strideM = (long long)P.nth * P.nr * nc * 2;
-  double* base = rtm + rtm_off(P, 0, th, r, nc);
-  for (int m = threadIdx.x; m <= L; m += blockDim.x) {
-    const double2 zm = z[m];
-    double a0, b0, a1, b1;
-    if (m == 0) {
-      a0 = zm.x * aN; a1 = zm.y * aN; b0 = 0.0; b1 = 0.0;
-    } else {
-      const double2 wm = z[N - m];
-      a0 = (zm.x + wm.x) * aN;
-      b0 = (wm.y - zm.y) * aN;
-      a1 = (zm.y + wm.y) * aN;
-      b1 = (zm.x - wm.x) * aN;
-    }
-    double* rec = base + m * strideM;
-    *reinterpret_cast<double2*>(rec + rec_off(2 * q, nv)) = make_double2(a0, b0);
-    if (2 * q + 1 < nc) *reinterpret_cast<double2*>(rec + rec_off(2 * q + 1, nv)) = make_double2(a1, b1);
-  }
-}
-
-template <int MVB, int MSB, int MVF, int MSF>
-__global__ void __launch_bounds__(kFftThreads) k_fft_cycle_wide(Plan P, int line0, int nlines) {
-  extern __shared__ double4 smraw[];
-  const int N = P.nph;
-  const int npb = (P.ncb + 1) / 2, npf = (P.ncf + 1) / 2;
-  const int npm = npb > npf ? npb : npf;
-  double2* z = reinterpret_cast<double2*>(smraw);
-  double2* sc = P.fft_scratch + (long long)blockIdx.x * npm * N;
-  // the first pass reads the line's spectra in place (rtm records, order
-  // stride rs): one line of a wide grid is too large to stage, and a small
-  // CTA keeps several resident per SM
-  const long long rs = (long long)P.nth * P.nr * P.ncb * 2;
-  for (int line = line0 + blockIdx.x; line < nlines; line += gridDim.x) {
-    const int th = line % P.nth, r = line / P.nth;
-    const double* st = P.rtm_b + rtm_off(P, 0, th, r, P.ncb);
-    for (int pp = 0; pp < npb; ++pp) {
-      dif_first_one_dispatch(P.fac[0], st, P.ncb, P.nvb, pp, z, N, P.L, P.twid, rs);
-      __syncthreads();
-      dif_rest(z, 1, N, P, P.twid);
-      for (int i = threadIdx.x; i < N; i += blockDim.x) sc[(long long)pp * N + i] = z[i];
-      __syncthreads();
-    }
-    products<MVB, MSB, MVF, MSF>(sc, N, P);
-    __syncthreads();
-    for (int q = 0; q < npf; ++q) {
-      for (int i = threadIdx.x; i < N; i += blockDim.x) z[i] = sc[(long long)q * N + i];
-      __syncthreads();
-      dit_all(z, 1, N, P, P.twid);
-      store_one(z, q, P, P.rtm_f, P.ncf, P.nvf, th, r);
-      __syncthreads();
-    }
-  }
-}
-
-// Separable backward for wide lines: one pair at a time straight to the grid.
-__global__ void __launch_bounds__(kFftThreads) k_fft_bwd_grid_wide(Plan P, double* __restrict__ fld) {
-  extern __shared__ double4 smraw[];
-  const int N = P.nph;
-  const int npb = (P.ncb + 1) / 2;
-  double2* z = reinterpret_cast<double2*>(smraw);
-  const int line = blockIdx.x;
-  const int r = line % P.nr, th = line / P.nr;
-  const long long nnod = (long long)P.nr * P.nth * N;
-  const double* st = P.rtm_b + rtm_off(P, 0, th, r, P.ncb);  // spectra read in place
-  const long long rs = (long long)P.nth * P.nr * P.ncb * 2;
-  for (int pp = 0; pp < npb; ++pp) {
-    dif_first_one_dispatch(P.fac[0], st, P.ncb, P.nvb, pp, z, N, P.L, P.twid, rs);
-    __syncthreads();
-    dif_rest(z, 1, N, P, P.twid);
-    const int nc2 = 2 * pp + 1 < P.ncb ? 2 : 1;
-    for (int it = threadIdx.x; it < N * nc2; it += blockDim.x) {
-      const int c = it / N, pos = it % N;
-      const int phi = P.digrev[pos];
-      const double2 v = z[pos];
-      fld[(long long)r + (long long)P.nr * (th + (long long)P.nth * phi) + nnod * (2 * pp + c)] = c ? v.y : v.x;
-    }
-    __syncthreads();
-  }
-}
-
-// Separable forward for wide lines: one pair at a time from the grid.
-__global__ void __launch_bounds__(kFftThreads) k_fft_fwd_grid_wide(Plan P, const double* __restrict__ frc) {
-  extern __shared__ double4 smraw[];
-  const int N = P.nph;
-  const int npf = (P.ncf + 1) / 2;
-  double2* z = reinterpret_cast<double2*>(smraw);
-  const int line = blockIdx.x;
-  const int r = line % P.nr, th = line / P.nr;
-  const long long nnod = (long long)P.nr * P.nth * N;
-  for (int q = 0; q < npf; ++q) {
-    for (int pos = threadIdx.x; pos < N; pos += blockDim.x) {
-      const int phi = P.digrev[pos];
-      const long long node = (long long)r + (long long)P.nr * (th + (long long)P.nth * phi);
-      const double lo = frc[node + nnod * (2 * q)];
-      const double hi = (2 * q + 1 < P.ncf) ? frc[node + nnod * (2 * q + 1)] : 0.0;
-      z[pos] = make_double2(lo, hi);
-    }
-    __syncthreads();
-    dit_all(z, 1, N, P, P.twid);
-    store_one(z, q, P, P.rtm_f, P.ncf, P.nvf, th, r);
-    __syncthreads();
-  }
-}
-
-// Separable backward: spectra -> grid fld[node + nnod*c], node = r + nr*(th + nth*phi).
-__global__ void __launch_bounds__(kFftThreads) k_fft_bwd_grid(Plan P, double* __restrict__ fld) {
-  extern __shared__ double4 smraw[];
-  const int N = P.nph;
-  const int npb = (P.ncb + 1) / 2;
-  double2* z = reinterpret_cast<double2*>(smraw);
-  double* st = reinterpret_cast<double*>(z + npb * N);
-  const int line = blockIdx.x;
-  const int r = line % P.nr, th = line / P.nr;
-  prefetch_line(st, P.rtm_b, P.ncb, P, th, r);
-  cp_async_wait<0>();
-  __syncthreads();
-  dif_first_dispatch(P.fac[0], st, P.ncb, P.nvb, z, npb, N, P.L, P.twid);
-  __syncthreads();
-  dif_rest(z, npb, N, P, P.twid);
-  const long long nnod = (long long)P.nr * P.nth * N;
-  for (int it = threadIdx.x; it < N * P.ncb; it += blockDim.x) {
-    const int c = it / N, pos = it % N;
-    const int phi = P.digrev[pos];
-    const double2 v = z[(c >> 1) * N + pos];
-    fld[(long long)r + (long long)P.nr * (th + (long long)P.nth * phi) + nnod * c] = (c & 1) ? v.y : v.x;
-  }
-}
-
-// Separable forward: grid frc -> spectra rtm_f.
-__global__ void __launch_bounds__(kFftThreads) k_fft_fwd_grid(Plan P, const double* __restrict__ frc) {
-  extern __shared__ double4 smraw[];
-  const int N = P.nph;
-  const int npf = (P.ncf + 1) / 2;
-  double2* z = reinterpret_cast<double2*>(smraw);
-  const int line = blockIdx.x;
-  const int r = line % P.nr, th = line / P.nr;
-  const long long nnod = (long long)P.nr * P.nth * N;
-  for (int it = threadIdx.x; it < N * npf; it += blockDim.x) {
-    const int q = it / N, pos = it % N;
-    const int phi = P.digrev[pos];
-    const long long node = (long long)r + (long long)P.nr * (th + (long long)P.nth * phi);
-    const double lo = frc[node + nnod * (2 * q)];
-    const double hi = (2 * q + 1 < P.ncf) ? frc[node + nnod * (2 * q + 1)] : 0.0;
-    z[q * N + pos] = make_double2(lo, hi);
-  }
-  __syncthreads();
-  dit_all(z, npf, N, P, P.twid);
-  store_line(z, npf, P, P.rtm_f, P.ncf, P.nvf, th, r);
-}
-
-// ---------------------------------------------------------------------------
-// staged records of one line: [m][ncs pairs], ncs = nc rounded up to odd
-__device__ __forceinline__ int ncs_of(int nc) { return nc | 1; }
-
-// Stages the spectra of one line (NC components, all orders) into shared
-// memory with cp.async: thread t copies the 16-byte pieces of component t % NC of orders t / NC, t / NC + T / NC, ...
-// (T = the largest multiple of NC not above the thread count), with pointer
-// increments instead of divisions.
-template <int NC>
-__device__ void prefetch_line_c(double* st, const double* rtm, const Plan& P, int th, int r) {
-  constexpr int NCS = NC | 1;
-  const int per = blockDim.x / NC;  // orders per sweep
-  if ((int)threadIdx.x < per * NC) {
-    const int c = threadIdx.x % NC;
-    int m = threadIdx.x / NC;
-    const long long strideM = (long long)P.nth * P.nr * NC * 2;
-    const double* src = rtm + rtm_off(P, m, th, r, NC) + 2 * c;
-    double* dst = st + (m * NCS + c) * 2;
-    const long long sstep = strideM * per;
-    for (; m <= P.L; m += per, src += sstep, dst += 2 * NCS * per) cp_async16(dst, src);
-  }
-  cp_async_commit();
-}
-
-__device__ __forceinline__ double2 spec_at_t(const double* st, int nc, int nv, int pp, int k, int N, int L) {
-  int m;
-  bool mirror;
-  if (k <= L) { m = k; mirror = false; }
-  else if (k >= N - L) { m = N - k; mirror = true; }
-  else return make_double2(0.0, 0.0);
-  const double* rec = st + m * ncs_of(nc) * 2;
-  const double* r0 = rec + rec_off(2 * pp, nv);
-  const double a0 = r0[0], b0 = r0[1];
-  double a1 = 0.0, b1 = 0.0;
-  if (2 * pp + 1 < nc) {
-    const double* r1 = rec + rec_off(2 * pp + 1, nv);
-    a1 = r1[0];
-    b1 = r1[1];
-  }
-  if (m == 0) return make_double2(a0, a1);
-  return mirror ? make_double2(0.5 * a0 - 0.5 * b1, 0.5 * b0 + 0.5 * a1)
-                : make_double2(0.5 * a0 + 0.5 * b1, 0.5 * a1 - 0.5 * b0);
-}
-
-size_t smem_cycle_f(const Plan& p) {
-  const int npair = ((p.ncb > p.ncf ? p.ncb : p.ncf) + 1) / 2;
-  // grid pairs, alignment of the staging to 128 bytes, staged spectra, mbarrier
-  return sizeof(double2) * ((size_t)npair * (p.nph + 1)) + 128 + sizeof(double) * 2 * (size_t)(p.L + 1) * (p.ncb | 1) + 16;
-}
-
-// cuTensorMapEncodeTiled, resolved through the runtime (no link-time
-// dependency on the driver library, so the library also loads on hosts
-// without a GPU driver); null when unavailable.
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static EncodeTiledFn encode_tiled() {
-  static const EncodeTiledFn fn = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      return static_cast<EncodeTiledFn>(nullptr);
-    return reinterpret_cast<EncodeTiledFn>(p);
-  }();
-  return fn;
-}
-
-// Tensor map of rtm_b for the TMA staging of k_fft_cycle_f: [m][r][theta][record]
-// doubles, box (2 (ncb | 1), 1, 1, mbox).  False when the orders do not split
-// into whole boxes or the driver refuses the map (the kernel then uses cp.async).
-bool make_rtm_map(const Plan& p, CUtensorMap* map, int* mbox) {
-  const int nc = p.ncb, ncs2 = 2 * (nc | 1);
-  const int mb = p.L + 1 < 256 ? p.L + 1 : 256;
-  *mbox = mb;
-  if ((p.L + 1) % mb != 0 || !p.rtm_b || (reinterpret_cast<uintptr_t>(p.rtm_b) & 15)) return false;
-  const cuuint64_t dims[4] = {(cuuint64_t)(2 * nc), (cuuint64_t)p.nth, (cuuint64_t)p.nr, (cuuint64_t)(p.L + 1)};
-  const cuuint64_t strides[3] = {16ull * nc, 16ull * nc * p.nth, 16ull * nc * p.nth * p.nr};
-  const cuuint32_t box[4] = {(cuuint32_t)ncs2, 1, 1, (cuuint32_t)mb};
-  const cuuint32_t es[4] = {1, 1, 1, 1};
-  const EncodeTiledFn enc = encode_tiled();
-  if (!enc) return false;
-  return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, const_cast<double*>(p.rtm_b), dims, strides, box, es,
-             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-// ---------------------------------------------------------------------------
-// Fused-pass variant for N = F0 * M * 4 (F0 in {3, 6, 12, 24}, M in {4, 16}):
-// inverse passes radix F0 (reading the staged spectra), radix M, radix 4; the
-// last inverse radix-4 pass, the grid products and the first forward radix-4
-// pass share one item (4 grid points of every component in registers), so a
-// line takes five sweeps over shared memory instead of nine.  The radix-4
-// passes of span 4 carry no twiddles.  Swizzle i -> i ^ (((i >> 3) ^ (i >> 6))
-// & 7) inside each pair sequence (pairs N + 1 entries apart) keeps every
-// quarter warp on 8 distinct 16-byte bank groups in all passes at N = 1536.
-constexpr int kFftThreadsF = 384;
-
-// Threads of one staged CTA.  Every variant fills the register file
-// (168 registers x 384 threads per SM): at N = 1536 one line takes the whole
-// shared memory, so one CTA has them all; the shorter lines leave room for
-// several CTAs per SM, whose barriers and record stores then overlap, and a
-// pass of theirs has fewer items than 384 threads could take (N / F0 or N / M
-// per pair).  FFT ms at 384 threads -> here: L = 255, Nr = 129 (N = 768)
-// 2.64 -> 2.42 (160 threads 2.53); L = 127, Nr = 65 (N = 384) 0.390 -> 0.292
-// (128 threads 0.296); L = 63, Nr = 65 (N = 192) 0.153 -> 0.081 (96 threads
-// 0.085); L = 31, Nr = 33 (N = 96) 0.034 -> 0.016 (64 threads 0.018).
-__host__ __device__ constexpr int ff_threads(int n) { return n == 768 ? 192 : n == 384 ? 96 : n == 192 ? 64 : n == 96 ? 32 : kFftThreadsF; }
-
-__host__ __device__ constexpr int ff_mid(int n) { return (n % 64 == 0 && (n / 64 == 3 || n / 64 == 6 || n / 64 == 12 || n / 64 == 24)) ? 16 : 4; }
-__host__ __device__ constexpr int ff_first(int n) { return n / (4 * ff_mid(n)); }
-__device__ __forceinline__ int swf(int i) { return i ^ (((i >> 3) ^ (i >> 6)) & 7); }
-// 32-byte global store; p 32-byte aligned
-__device__ __forceinline__ void st_v4(double* p, double a, double b, double c, double d) {
-  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};\n" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
-}
-
-// e^{2 pi i k / 48}: cos and sin of the first quadrant, k = 0..11
+// Composite radices.  e^{2 pi i k / 48}: cos and sin of the first quadrant, k = 0..11
 __host__ __device__ constexpr double c48q(int k) {
   constexpr double c[12] = {1.0, 0.9914448613738104, 0.9659258262890683, 0.9238795325112867,
                             0.8660254037844386, 0.7933533402912352, 0.7071067811865476, 0.6087614290087207,
                             0.5, 0.3826834323650898, 0.25881904510252074, 0.1305261922200516};
   return c[k];
 }
-// x * e^{SIGN 2 pi i e / R}, e and R compile-time, R | 48
+// cos and sin of 2 pi k / R for the radices that do not divide 48
+__host__ __device__ constexpr double cos9(int k) {
+  constexpr double c[9] = {1.0, 0.76604444311897803520, 0.17364817766693034885, -0.5, -0.93969262078590838405,
+                           -0.93969262078590838405, -0.5, 0.17364817766693034885, 0.76604444311897803520};
+  return c[k];
+}
+__host__ __device__ constexpr double sin9(int k) {
+  constexpr double c[9] = {0.0, 0.64278760968653932632, 0.98480775301220805936, 0.86602540378443864676,
+                           0.34202014332566873304, -0.34202014332566873304, -0.86602540378443864676,
+                           -0.98480775301220805936, -0.64278760968653932632};
+  return c[k];
+}
+// multiples of 12 degrees, k = 0 .. 29 (R = 15: 2 e, R = 10: 3 e)
+__host__ __device__ constexpr double cos30(int k) {
+  constexpr double c[8] = {1.0, 0.97814760073380563793, 0.91354545764260089550, 0.80901699437494742410,
+                           0.66913060635885821383, 0.5, 0.30901699437494742410, 0.10452846326765347140};
+  k = k % 30;
+  if (k > 15) k = 30 - k;
+  return k <= 7 ? c[k] : -c[15 - k];
+}
+__host__ __device__ constexpr double sin30(int k) {
+  constexpr double c[8] = {0.0, 0.20791169081775933710, 0.40673664307580020775, 0.58778525229247312917,
+                           0.74314482547739423501, 0.86602540378443864676, 0.95105651629515357212,
+                           0.99452189536827333692};
+  k = k % 30;
+  if (k > 15) return -sin30(30 - k);
+  return k <= 7 ? c[k] : c[15 - k];
+}
+// x * e^{SIGN 2 pi i e / R}, e and R compile-time, R | 48 or R = 9, 10, 15
 template <int R, int E, int SIGN>
 __device__ __forceinline__ double2 rot(double2 x) {
+  if constexpr (48 % R != 0) {
+    if constexpr (E % R == 0) return x;
+    constexpr double c = R == 9 ? cos9(E % 9) : cos30(E % R * (30 / (R == 9 ? 10 : R)));
+    constexpr double sn = (R == 9 ? sin9(E % 9) : sin30(E % R * (30 / (R == 9 ? 10 : R)))) * (double)SIGN;
+    return make_double2(x.x * c - x.y * sn, x.x * sn + x.y * c);
+  } else {
   constexpr int k = (E * (48 / R)) % 48;
   constexpr int q = k / 12, k0 = k % 12;
   if constexpr (k0 == 0) {
@@ -813,6 +250,7 @@ __device__ __forceinline__ double2 rot(double2 x) {
     constexpr double c = q == 0 ? c0 : q == 1 ? -s0 : q == 2 ? -c0 : s0;
     constexpr double sn = (q == 0 ? s0 : q == 1 ? c0 : q == 2 ? -s0 : -c0) * (double)SIGN;
     return make_double2(x.x * c - x.y * sn, x.x * sn + x.y * c);
+  }
   }
 }
 
@@ -851,10 +289,520 @@ struct DFT2F {
   }
 };
 template <int SIGN> struct DFT<6, SIGN> { __device__ static void run(double2* x) { DFT2F<3, 2, SIGN>::run(x); } };
+template <int SIGN> struct DFT<9, SIGN> { __device__ static void run(double2* x) { DFT2F<3, 3, SIGN>::run(x); } };
+template <int SIGN> struct DFT<10, SIGN> { __device__ static void run(double2* x) { DFT2F<5, 2, SIGN>::run(x); } };
+template <int SIGN> struct DFT<15, SIGN> { __device__ static void run(double2* x) { DFT2F<5, 3, SIGN>::run(x); } };
 template <int SIGN> struct DFT<12, SIGN> { __device__ static void run(double2* x) { DFT2F<3, 4, SIGN>::run(x); } };
 template <int SIGN> struct DFT<16, SIGN> { __device__ static void run(double2* x) { DFT2F<4, 4, SIGN>::run(x); } };
 template <int SIGN> struct DFT<24, SIGN> { __device__ static void run(double2* x) { DFT2F<3, 8, SIGN>::run(x); } };
 template <int SIGN> struct DFT<1, SIGN> { __device__ static void run(double2*) {} };
+
+#define KMHD_RADIX_SWITCH(R, CALL) \
+  switch (R) {                     \
+    case 2: CALL(2); break;        \
+    case 3: CALL(3); break;        \
+    case 4: CALL(4); break;        \
+    case 5: CALL(5); break;        \
+    case 6: CALL(6); break;        \
+    case 8: CALL(8); break;        \
+    case 9: CALL(9); break;        \
+    case 10: CALL(10); break;      \
+    case 12: CALL(12); break;      \
+    case 15: CALL(15); break;      \
+    default: CALL(16); break;      \
+  }
+
+// First inverse pass: sequence i is pair q0 + i dq of the line at line + i ls
+// (block rows bs doubles apart, see spec_at).
+template <int R>
+__device__ __forceinline__ void dif_first(const Seqs Z, const Plan& P, const double* line, long long ls, long long bs,
+                                          int nc, int q0, int dq) {
+  const int N = Z.N, s = N / R;
+  for (int it = threadIdx.x; it < Z.n * s; it += blockDim.x) {
+    const int pp = it / s, j = it - pp * s;
+    double2 x[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) x[r] = spec_at(P, line + pp * ls, bs, nc, q0 + pp * dq, j + r * s);
+    DFT<R, +1>::run(x);
+    double2* base = Z.z + pp * Z.zs;
+    TwiddleRun<+1> tr(P.twid, j);
+#pragma unroll
+    for (int q = 0; q < R; ++q) base[Z.ix(j + q * s)] = q == 0 ? x[0] : cmul(x[q], tr.next(q));
+  }
+}
+__device__ __noinline__ void dif_first_dispatch(const Seqs Z, const Plan& P, const double* line, long long ls,
+                                                long long bs, int nc, int q0, int dq) {
+#define KMHD_CALL(R) dif_first<R>(Z, P, line, ls, bs, nc, q0, dq)
+  KMHD_RADIX_SWITCH(P.fac[0], KMHD_CALL)
+#undef KMHD_CALL
+}
+
+// One in-place DIF (SIGN > 0: butterfly, then twiddle) or DIT (SIGN < 0, its
+// transpose) pass of radix R over blocks of span entries.
+template <int R, int SIGN>
+__device__ __forceinline__ void mid_pass(const Seqs Z, int span, const double2* __restrict__ tw) {
+  const int N = Z.N, s = span / R, nbf = N / R, stw = N / span;
+  for (int it = threadIdx.x; it < Z.n * nbf; it += blockDim.x) {
+    const int pp = it / nbf, rem = it - pp * nbf;
+    const int b = rem / s, j = rem - b * s;
+    double2* base = Z.z + pp * Z.zs;
+    const int i0 = b * span + j;
+    double2 x[R];
+    if (s == 1) {  // one butterfly per block: every twiddle is 1
+#pragma unroll
+      for (int r = 0; r < R; ++r) x[r] = base[Z.ix(i0 + r)];
+      DFT<R, SIGN>::run(x);
+#pragma unroll
+      for (int q = 0; q < R; ++q) base[Z.ix(i0 + q)] = x[q];
+      continue;
+    }
+    TwiddleRun<SIGN> tr(tw, j * stw);
+    if constexpr (SIGN > 0) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) x[r] = base[Z.ix(i0 + r * s)];
+      DFT<R, +1>::run(x);
+#pragma unroll
+      for (int q = 0; q < R; ++q) base[Z.ix(i0 + q * s)] = q == 0 ? x[0] : cmul(x[q], tr.next(q));
+    } else {
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const double2 v = base[Z.ix(i0 + r * s)];
+        x[r] = r == 0 ? v : cmul(v, tr.next(r));
+      }
+      DFT<R, -1>::run(x);
+#pragma unroll
+      for (int q = 0; q < R; ++q) base[Z.ix(i0 + q * s)] = x[q];
+    }
+  }
+}
+__device__ __noinline__ void dif_dispatch(const Seqs Z, int R, int span, const double2* tw) {
+#define KMHD_CALL(R) mid_pass<R, +1>(Z, span, tw)
+  KMHD_RADIX_SWITCH(R, KMHD_CALL)
+#undef KMHD_CALL
+}
+__device__ __noinline__ void dit_dispatch(const Seqs Z, int R, int span, const double2* tw) {
+#define KMHD_CALL(R) mid_pass<R, -1>(Z, span, tw)
+  KMHD_RADIX_SWITCH(R, KMHD_CALL)
+#undef KMHD_CALL
+}
+
+// The inverse passes after the first, and every forward pass.
+__device__ void dif_rest(const Seqs& Z, const Plan& P) {
+  int span = Z.N / P.fac[0];
+  for (int f = 1; f < P.nfac; ++f) {
+    dif_dispatch(Z, P.fac[f], span, P.twid);
+    __syncthreads();
+    span /= P.fac[f];
+  }
+}
+__device__ void dit_all(const Seqs& Z, const Plan& P) {
+  int span = 1;
+  for (int f = P.nfac - 1; f >= 0; --f) {
+    span *= P.fac[f];
+    dit_dispatch(Z, P.fac[f], span, P.twid);
+    __syncthreads();
+  }
+}
+
+// Stage the records of line (th, r) into st via cp.async (16 B each).
+__device__ void prefetch_line(double* st, const double* rtm, int nc, const Plan& P, int th, int r) {
+  const int row = rtm_row(P, nc);
+  const long long bs = (long long)P.nth * P.nr * row;
+  const double* base = rtm + rtm_off(P, 0, th, r, nc);
+  const int per = row / 2, n = rtm_blocks(P) * per;
+  for (int it = threadIdx.x; it < n; it += blockDim.x) {
+    const int b = it / per, c = it - b * per;
+    cp_async16(st + 2 * it, base + b * bs + 2 * c);
+  }
+  cp_async_commit();
+}
+
+// Record sector of order m from the natural-order forward spectrum of one pair:
+// zm = z[m], wm = z[N - m].
+__device__ __forceinline__ void store_pair(double* base, long long bs, const Plan& P, int m, int pp, int nc, bool al,
+                                           double2 zm, double2 wm) {
+  const double aN = 1.0 / (double)P.nph;
+  double a0, b0, a1, b1;
+  if (m == 0) {
+    a0 = zm.x * aN; a1 = zm.y * aN; b0 = 0.0; b1 = 0.0;
+  } else {
+    a0 = (zm.x + wm.x) * aN;
+    b0 = (wm.y - zm.y) * aN;
+    a1 = (zm.y + wm.y) * aN;
+    b1 = (zm.x - wm.x) * aN;
+  }
+  double* d = base + (m >> P.mbs) * bs + rtm_pair(P, m, pp, nc);
+  if (2 * pp + 1 < nc) st_sector(d, al, a0, b0, a1, b1);
+  else *reinterpret_cast<double2*>(d) = make_double2(a0, b0);
+}
+
+// Natural-order forward spectra of the sequences -> records: sequence i is pair
+// q0 + i dq of the line that starts at base + i ls.  Lanes take consecutive
+// orders of one sequence: eight lanes write 256 contiguous bytes.
+__device__ __forceinline__ void store_seqs(const Seqs& Z, const Plan& P, double* base, long long ls, int nc, int q0,
+                                           int dq) {
+  const int N = P.nph, L = P.L;
+  const long long bs = (long long)P.nth * P.nr * rtm_row(P, nc);
+  const bool al = rtm_aligned(P, nc);
+  auto ix = [&](int i) { return Z.ix(i); };
+  int m = threadIdx.x, pp = 0;
+  for (int it = threadIdx.x; it < (L + 1) * Z.n; it += blockDim.x, m += blockDim.x) {
+    while (m > L) { m -= L + 1; ++pp; }
+    const double2* zp = Z.z + pp * Z.zs;
+    store_pair(base + pp * ls, bs, P, m, q0 + pp * dq, nc, al, zp[ix(m)],
+               m == 0 ? make_double2(0.0, 0.0) : zp[ix(N - m)]);
+  }
+}
+// x[a], selected without dynamic register indexing.
+template <int M>
+__device__ __forceinline__ double selv(const double* x, int a) {
+  double v = x[0];
+#pragma unroll
+  for (int q = 1; q < M; ++q)
+    if (a == q) v = x[q];
+  return v;
+}
+
+// Grid products of one point.  Backward vector v is (rr, th, ph)[v], scalar s
+// is sc[s]; forward vector i goes to (orr, oth, oph)[i], scalar j to os[j].  MV*
+// / MS* are compile-time maxima, the plan's counts (EX: equal to them) are <= them.
+template <int MVB, int MSB, int MVF, int MSF, bool EX>
+__device__ __forceinline__ void point_products(const double* rr, const double* th, const double* ph, const double* sc,
+                                               const Plan& P, double* orr, double* oth, double* oph, double* os) {
+  const int nvf = EX ? MVF : P.nvf, nsf = EX ? MSF : P.nsf;
+#pragma unroll
+  for (int i = 0; i < MVF; ++i) {
+    if (i < nvf) {
+      const double cf = P.pcoef[i];
+      const int a = P.pa[i], b = P.pb[i];
+      const double x0 = selv<MVB>(rr, a), x1 = selv<MVB>(th, a), x2 = selv<MVB>(ph, a);
+      if (P.pkind[i] == KMHD_PROD_CROSS) {
+        const double y0 = selv<MVB>(rr, b), y1 = selv<MVB>(th, b), y2 = selv<MVB>(ph, b);
+        orr[i] = (x1 * y2 - x2 * y1) * cf;
+        oth[i] = (x2 * y0 - x0 * y2) * cf;
+        oph[i] = (x0 * y1 - x1 * y0) * cf;
+      } else {
+        const double s = selv<MSB>(sc, b);
+        orr[i] = x0 * s * cf;
+        oth[i] = x1 * s * cf;
+        oph[i] = x2 * s * cf;
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < MSF; ++j) {
+    if (j < nsf) {
+      const int q = nvf + j;
+      const double cf = P.pcoef[q];
+      const int a = P.pa[q], b = P.pb[q];
+      if (P.pkind[q] == KMHD_PROD_DOT) {
+        os[j] = (selv<MVB>(rr, a) * selv<MVB>(rr, b) + selv<MVB>(th, a) * selv<MVB>(th, b) +
+                 selv<MVB>(ph, a) * selv<MVB>(ph, b)) * cf;
+      } else {
+        os[j] = selv<MSB>(sc, a) * selv<MSB>(sc, b) * cf;
+      }
+    }
+  }
+}
+
+// Product lists known at compile time (vector-valued products first): the
+// field sets of the reference's MHD, convection and heat runs.  PK = 0: the
+// plan's list, read at run time.
+constexpr int kX = KMHD_PROD_CROSS, kVS = KMHD_PROD_VEC_SCALAR, kDot = KMHD_PROD_DOT;
+struct ProdList {
+  int nvb, nsb, nvf, nsf, n;
+  int kind[6], a[6], b[6];
+};
+constexpr ProdList kProdLists[6] = {
+    {},
+    // u, omega, B + T -> omega x u, u x B, u T + u . omega
+    {3, 1, 3, 1, 4, {kX, kX, kVS, kDot}, {1, 0, 0, 0}, {0, 2, 0, 1}},
+    // u, omega, B, J + T -> omega x u, J x B, u x B, u T
+    {4, 1, 4, 0, 4, {kX, kX, kX, kVS}, {1, 3, 0, 0}, {0, 2, 2, 0}},
+    // u, omega, B, J + T, C -> omega x u, J x B, u x B, u T, u C + u . omega
+    {4, 2, 5, 1, 6, {kX, kX, kX, kVS, kVS, kDot}, {1, 3, 0, 0, 0, 0}, {0, 2, 2, 0, 1, 1}},
+    // u, omega + T -> omega x u, u T + u . omega
+    {2, 1, 2, 1, 3, {kX, kVS, kDot}, {1, 0, 0}, {0, 0, 1}},
+    // u + T -> u T
+    {1, 1, 1, 0, 1, {kVS}, {0}, {0}}};
+
+// the entry of kProdLists that is the plan's list, or 0
+inline int prod_list(const Plan& p) {
+  for (int k = 1; k < 6; ++k) {
+    const ProdList& q = kProdLists[k];
+    if (p.nvb != q.nvb || p.nsb != q.nsb || p.nvf != q.nvf || p.nsf != q.nsf || p.nprod != q.n) continue;
+    bool same = true;
+    for (int i = 0; i < q.n; ++i) same = same && p.pkind[i] == q.kind[i] && p.pa[i] == q.a[i] && p.pb[i] == q.b[i];
+    if (same) return k;
+  }
+  return 0;
+}
+
+// point_products for list PK > 0.
+template <int PK, int I = 0>
+__device__ __forceinline__ void point_products_k(const double* rr, const double* th, const double* ph, const double* sc,
+                                                 const Plan& P, double* orr, double* oth, double* oph, double* os) {
+  constexpr ProdList q = kProdLists[PK];
+  if constexpr (I < q.n) {
+    constexpr int a = q.a[I], b = q.b[I];
+    const double cf = P.pcoef[I];
+    if constexpr (q.kind[I] == kX) {
+      orr[I] = (th[a] * ph[b] - ph[a] * th[b]) * cf;
+      oth[I] = (ph[a] * rr[b] - rr[a] * ph[b]) * cf;
+      oph[I] = (rr[a] * th[b] - th[a] * rr[b]) * cf;
+    } else if constexpr (q.kind[I] == kVS) {
+      orr[I] = rr[a] * sc[b] * cf;
+      oth[I] = th[a] * sc[b] * cf;
+      oph[I] = ph[a] * sc[b] * cf;
+    } else {
+      os[I - q.nvf] = (rr[a] * rr[b] + th[a] * th[b] + ph[a] * ph[b]) * cf;
+    }
+    point_products_k<PK, I + 1>(rr, th, ph, sc, P, orr, oth, oph, os);
+  }
+}
+
+// Pointwise products on the digit-reversed grid (sequence zs entries apart),
+// backward pairs in, forward pairs out (pair and list order: see rtm_off); PK: the
+// product list (0: the plan's).
+template <int PK>
+__device__ __forceinline__ void products(double2* z, int zs, int N, const Plan& P) {
+  constexpr ProdList q = kProdLists[PK];
+  constexpr int MVB = PK ? q.nvb : kMaxVec, MSB = PK ? q.nsb : kMaxScl, MVF = PK ? q.nvf : kMaxVec,
+                MSF = PK ? q.nsf : kMaxScl;
+  const int nvb = PK ? MVB : P.nvb, nsb = PK ? MSB : P.nsb, nvf = PK ? MVF : P.nvf, nsf = PK ? MSF : P.nsf;
+  for (int pos = threadIdx.x; pos < N; pos += blockDim.x) {
+    constexpr int VB = MVB > 0 ? MVB : 1, SB = MSB > 0 ? MSB : 1, VF = MVF > 0 ? MVF : 1, SF = MSF > 0 ? MSF : 1;
+    double rr[VB] = {}, th[VB] = {}, ph[VB] = {}, sc[SB] = {};
+    double orr[VF] = {}, oth[VF] = {}, oph[VF] = {}, os[SF] = {};
+    // list entry f of the pairs that start at pair nv
+    auto entry = [&](int nv, int f) { return reinterpret_cast<double*>(z + (nv + (f >> 1)) * zs + pos) + (f & 1); };
+#pragma unroll
+    for (int v = 0; v < MVB; ++v)
+      if (v < nvb) {
+        const double2 w = z[v * zs + pos];
+        rr[v] = *entry(nvb, v);
+        th[v] = w.x;
+        ph[v] = w.y;
+      }
+#pragma unroll
+    for (int k = 0; k < MSB; ++k)
+      if (k < nsb) sc[k] = *entry(nvb, nvb + k);
+    if constexpr (PK > 0) point_products_k<PK>(rr, th, ph, sc, P, orr, oth, oph, os);
+    else point_products<MVB, MSB, MVF, MSF, false>(rr, th, ph, sc, P, orr, oth, oph, os);
+#pragma unroll
+    for (int v = 0; v < MVF; ++v)
+      if (v < nvf) {
+        z[v * zs + pos] = make_double2(oth[v], oph[v]);
+        *entry(nvf, v) = orr[v];
+      }
+#pragma unroll
+    for (int k = 0; k < MSF; ++k)
+      if (k < nsf) *entry(nvf, nvf + k) = os[k];
+    if ((nvf + nsf) & 1) *entry(nvf, nvf + nsf) = 0.0;
+  }
+}
+
+template <int PK>
+__global__ void __launch_bounds__(kFftThreads) k_fft_cycle(const __grid_constant__ Plan P, int line0, int nlines) {
+  extern __shared__ double4 smraw[];
+  const int N = P.nph;
+  const int npb = (P.ncb + 1) / 2, npf = (P.ncf + 1) / 2;
+  const int npair = npb > npf ? npb : npf;
+  double2* z = reinterpret_cast<double2*>(smraw);
+  double* st = reinterpret_cast<double*>(z + npair * N);
+  const Seqs ZB(z, npb, N, N), ZF(z, npf, N, N);
+  int line = line0 + blockIdx.x;
+  if (line >= nlines) return;
+  prefetch_line(st, P.rtm_b, P.ncb, P, line % P.nth, line / P.nth);
+  while (line < nlines) {
+    const int th = line % P.nth, r = line / P.nth;
+    cp_async_wait<0>();
+    __syncthreads();
+    dif_first_dispatch(ZB, P, st, 0, rtm_row(P, P.ncb), P.ncb, 0, 1);
+    __syncthreads();
+    const int next = line + gridDim.x;
+    if (next < nlines) prefetch_line(st, P.rtm_b, P.ncb, P, next % P.nth, next / P.nth);
+    dif_rest(ZB, P);
+    products<PK>(z, N, N, P);
+    __syncthreads();
+    dit_all(ZF, P);
+    store_seqs(ZF, P, P.rtm_f + rtm_off(P, 0, th, r, P.ncf), 0, P.ncf, 0, 1);
+    __syncthreads();
+    line = next;
+  }
+}
+
+// Lines whose grid fits in shared memory but not together with the staged
+// spectra of the next line (many fields, e.g. 14 + 16 components at
+// Nphi = 1536: 197 KB of grid pairs): the first pass reads the line's spectra
+// in place from the rtm records, everything else as k_fft_cycle.
+template <int PK>
+__global__ void __launch_bounds__(kFftThreads) k_fft_cycle_direct(const __grid_constant__ Plan P, int line0, int nlines) {
+  extern __shared__ double4 smraw[];
+  const int N = P.nph;
+  double2* z = reinterpret_cast<double2*>(smraw);
+  const Seqs ZB(z, (P.ncb + 1) / 2, N, N), ZF(z, (P.ncf + 1) / 2, N, N);
+  const long long bs = (long long)P.nth * P.nr * rtm_row(P, P.ncb);
+  for (int line = line0 + blockIdx.x; line < nlines; line += gridDim.x) {
+    const int th = line % P.nth, r = line / P.nth;
+    dif_first_dispatch(ZB, P, P.rtm_b + rtm_off(P, 0, th, r, P.ncb), 0, bs, P.ncb, 0, 1);
+    __syncthreads();
+    dif_rest(ZB, P);
+    products<PK>(z, N, N, P);
+    __syncthreads();
+    dit_all(ZF, P);
+    store_seqs(ZF, P, P.rtm_f + rtm_off(P, 0, th, r, P.ncf), 0, P.ncf, 0, 1);
+    __syncthreads();
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Wide lines (one line of every component does not fit in shared memory, e.g.
+// Nphi = 3072 with 10 components): the pairs go through shared memory one at a
+// time.  The cycle keeps the line's grid in a per-CTA global scratch
+// (pairs x N x 16 bytes, L2-resident), forms the products there and runs the
+// forward transforms pair by pair from it.
+template <int PK>
+__global__ void __launch_bounds__(kFftThreads) k_fft_cycle_wide(const __grid_constant__ Plan P, int line0, int nlines) {
+  extern __shared__ double4 smraw[];
+  const int N = P.nph;
+  const int npb = (P.ncb + 1) / 2, npf = (P.ncf + 1) / 2;
+  const int npm = npb > npf ? npb : npf;
+  double2* z = reinterpret_cast<double2*>(smraw);
+  double2* sc = P.fft_scratch + (long long)blockIdx.x * npm * N;
+  const Seqs Z(z, 1, N, N);
+  // the first pass reads the line's spectra in place (rtm records, block rows
+  // bs apart): one line of a wide grid is too large to stage, and a small
+  // CTA keeps several resident per SM
+  const long long bs = (long long)P.nth * P.nr * rtm_row(P, P.ncb);
+  for (int line = line0 + blockIdx.x; line < nlines; line += gridDim.x) {
+    const int th = line % P.nth, r = line / P.nth;
+    const double* st = P.rtm_b + rtm_off(P, 0, th, r, P.ncb);
+    for (int pp = 0; pp < npb; ++pp) {
+      dif_first_dispatch(Z, P, st, 0, bs, P.ncb, pp, 0);
+      __syncthreads();
+      dif_rest(Z, P);
+      for (int i = threadIdx.x; i < N; i += blockDim.x) sc[(long long)pp * N + i] = z[i];
+      __syncthreads();
+    }
+    products<PK>(sc, N, N, P);
+    __syncthreads();
+    for (int q = 0; q < npf; ++q) {
+      for (int i = threadIdx.x; i < N; i += blockDim.x) z[i] = sc[(long long)q * N + i];
+      __syncthreads();
+      dit_all(Z, P);
+      store_seqs(Z, P, P.rtm_f + rtm_off(P, 0, th, r, P.ncf), 0, P.ncf, q, 0);
+      __syncthreads();
+    }
+  }
+}
+
+constexpr int kGridThreads = 256;  // separable kernels: at most, at 128 registers
+
+// Component of part c (0, 1) of pair pp (the inverse of comp_pair).
+__device__ __forceinline__ int pair_comp(int pp, int c, int nv) {
+  if (pp < nv) return 3 * pp + 1 + c;
+  const int f = 2 * (pp - nv) + c;
+  return f < nv ? 3 * f : 2 * nv + f;
+}
+
+// Separable transforms between the spectra and the grid field[node + nnod c],
+// node = r + nr (th + nth phi).  No product couples the components, so one CTA
+// takes one pair of rad neighbouring radii of one latitude: its grid accesses
+// are rad contiguous doubles (with one radius per CTA every lane of a grid
+// access was a sector of its own: at L = 127, Nr = 65 the inverse took 0.65 ms
+// and the forward 0.52 ms; see grid_radii for the present ones).  Sequences lie
+// N + 1 entries apart, so the radii of one point are in different banks.
+// Block order: pair fastest, then radial block, then latitude.
+__global__ void __launch_bounds__(kGridThreads, 2)
+    k_fft_bwd_grid(const __grid_constant__ Plan P, double* __restrict__ fld, int lrad) {
+  const int rad = 1 << lrad;
+  extern __shared__ double4 smraw[];
+  const int N = P.nph, npb = (P.ncb + 1) / 2, nrb = (P.nr + rad - 1) / rad;
+  const int q = blockIdx.x % npb, rest = blockIdx.x / npb;
+  const int r0 = (rest % nrb) * rad, th = rest / nrb;
+  const int nrad = min(rad, P.nr - r0);
+  const Seqs Z(reinterpret_cast<double2*>(smraw), nrad, N + 1, N);
+  const long long ls = (long long)P.nth * rtm_row(P, P.ncb);
+  dif_first_dispatch(Z, P, P.rtm_b + rtm_off(P, 0, th, r0, P.ncb), ls, ls * P.nr, P.ncb, q, 0);
+  __syncthreads();
+  dif_rest(Z, P);
+  const long long nnod = (long long)P.nr * P.nth * N;
+  const bool two = 2 * q + 1 < P.ncb;
+  double* f0 = fld + nnod * pair_comp(q, 0, P.nvb) + r0 + (long long)P.nr * th;
+  double* f1 = two ? fld + nnod * pair_comp(q, 1, P.nvb) + r0 + (long long)P.nr * th : nullptr;
+  const long long ps = (long long)P.nr * P.nth;
+#pragma unroll 4
+  for (int it = threadIdx.x; it < N << lrad; it += blockDim.x) {
+    const int r = it & (rad - 1), pos = it >> lrad;
+    if (r >= nrad) continue;
+    const long long o = ps * __ldg(P.digrev + pos) + r;
+    const double2 v = Z.z[r * Z.zs + Z.ix(pos)];
+    f0[o] = v.x;
+    if (two) f1[o] = v.y;
+  }
+}
+__global__ void __launch_bounds__(kGridThreads, 2)
+    k_fft_fwd_grid(const __grid_constant__ Plan P, const double* __restrict__ frc, int lrad) {
+  const int rad = 1 << lrad;
+  extern __shared__ double4 smraw[];
+  const int N = P.nph, npf = (P.ncf + 1) / 2, nrb = (P.nr + rad - 1) / rad;
+  const int q = blockIdx.x % npf, rest = blockIdx.x / npf;
+  const int r0 = (rest % nrb) * rad, th = rest / nrb;
+  const int nrad = min(rad, P.nr - r0);
+  const Seqs Z(reinterpret_cast<double2*>(smraw), nrad, N + 1, N);
+  const long long nnod = (long long)P.nr * P.nth * N;
+  const bool two = 2 * q + 1 < P.ncf;
+  const double* __restrict__ f0 = frc + nnod * pair_comp(q, 0, P.nvf) + r0 + (long long)P.nr * th;
+  const double* __restrict__ f1 = two ? frc + nnod * pair_comp(q, 1, P.nvf) + r0 + (long long)P.nr * th : nullptr;
+  const long long ps = (long long)P.nr * P.nth;
+#pragma unroll 4
+  for (int it = threadIdx.x; it < N << lrad; it += blockDim.x) {
+    const int r = it & (rad - 1), pos = it >> lrad;
+    if (r >= nrad) continue;
+    const long long o = ps * __ldg(P.digrev + pos) + r;
+    Z.z[r * Z.zs + Z.ix(pos)] = make_double2(__ldg(f0 + o), two ? __ldg(f1 + o) : 0.0);
+  }
+  __syncthreads();
+  dit_all(Z, P);
+  store_seqs(Z, P, P.rtm_f + rtm_off(P, 0, th, r0, P.ncf), (long long)P.nth * rtm_row(P, P.ncf), P.ncf, q, 0);
+}
+
+// ---------------------------------------------------------------------------
+// bytes of one staged line
+size_t staged_bytes(const Plan& p) { return sizeof(double) * (size_t)rtm_blocks(p) * rtm_row(p, p.ncb); }
+
+size_t smem_cycle_f(const Plan& p) {
+  const int npair = ((p.ncb > p.ncf ? p.ncb : p.ncf) + 1) / 2;
+  // grid pairs, alignment of the staging to 128 bytes, staged spectra, mbarrier
+  return sizeof(double2) * ((size_t)npair * (p.nph + 1)) + 128 + staged_bytes(p) + 16;
+}
+
+// ---------------------------------------------------------------------------
+// Fused-pass variant for N = F0 * M * 4 (F0 in {3, 6, 12, 24}, M in {4, 16}):
+// inverse passes radix F0 (reading the staged spectra), radix M, radix 4; the
+// last inverse radix-4 pass, the grid products and the first forward radix-4
+// pass share one item (4 grid points of every component in registers), so a
+// line takes five sweeps over shared memory instead of nine.  The radix-4
+// passes of span 4 carry no twiddles.  Swizzle i -> i ^ (((i >> 3) ^ (i >> 6))
+// & 7) inside each pair sequence (pairs N + 1 entries apart) keeps every
+// quarter warp on 8 distinct 16-byte bank groups in all passes at N = 1536.
+constexpr int kFftThreadsF = 384;
+
+// Threads of one staged CTA.  Every variant fills the register file
+// (168 registers x 384 threads per SM): at N = 1536 one line takes the whole
+// shared memory, so one CTA has them all; the shorter lines leave room for
+// several CTAs per SM, whose barriers and record stores then overlap, and a
+// pass of theirs has fewer items than 384 threads could take (N / F0 or N / M
+// per pair).  FFT ms at 384 threads -> here: L = 255, Nr = 129 (N = 768)
+// 2.64 -> 2.42 (160 threads 2.53); L = 127, Nr = 65 (N = 384) 0.390 -> 0.292
+// (128 threads 0.296); L = 63, Nr = 65 (N = 192) 0.153 -> 0.081 (96 threads
+// 0.085); L = 31, Nr = 33 (N = 96) 0.034 -> 0.016 (64 threads 0.018).
+__host__ __device__ constexpr int ff_threads(int n) { return n == 768 ? 192 : n == 384 ? 96 : n == 192 ? 64 : n == 96 ? 32 : kFftThreadsF; }
+
+__host__ __device__ constexpr int ff_mid(int n) { return (n % 64 == 0 && (n / 64 == 3 || n / 64 == 6 || n / 64 == 12 || n / 64 == 24)) ? 16 : 4; }
+__host__ __device__ constexpr int ff_first(int n) { return n / (4 * ff_mid(n)); }
+__device__ __forceinline__ int swf(int i) { return i ^ (((i >> 3) ^ (i >> 6)) & 7); }
 
 // DFT of length 3B whose middle third of inputs (n = B .. 2B-1) is zero: the
 // first-stage length-3 transforms see (x0, 0, x2).
@@ -902,11 +850,10 @@ struct DFT2F_ZM<3, B, SIGN> {
 // inputs from the staged spectra.  Twiddles w^(j q) are read straight from the
 // table (j q < N here).  When N = 3 (L + 1) (PR), the middle third of the
 // inputs (L < k < N - L) is zero and the outer thirds need no range checks.
-// st: the line's records, staged (order stride 2 ncs) or, with INPLACE, the
-// rtm records themselves (order stride rsg doubles)
+// line / bs: the line's block rows, staged or in place (see spec_at).
 template <int N, bool PR, bool INPLACE = false>
-__device__ __forceinline__ void ff_dif_first(const double* st, int nc, int nv, double2* z, int npair, int L,
-                                             const double2* __restrict__ tw, long long rsg = 0) {
+__device__ __forceinline__ void ff_dif_first(const Plan& P, const double* line, long long bs, int nc, double2* z,
+                                             int npair, const double2* __restrict__ tw) {
   constexpr int R = ff_first(N), S1 = N / R, NP = N + 1, T3 = R / 3;
   for (int it = threadIdx.x; it < npair * S1; it += blockDim.x) {
     const int pp = it / S1, j = it - pp * S1;
@@ -914,10 +861,17 @@ __device__ __forceinline__ void ff_dif_first(const double* st, int nc, int nv, d
     if constexpr (PR) {
       // N = 3 (L + 1), S1 = (L + 1) / T3: input r < T3 is order m = j + r S1
       // (m = 0 only at j = r = 0); input r >= 2 T3 is the mirror of order
-      // m = N - j - r S1 (m = L + 1, a zero, only at j = 0, r = 2 T3); the
-      // pair's two components sit at record offsets o0, o1 (o1 < 0: none)
-      const int o0 = rec_off(2 * pp, nv), o1 = 2 * pp + 1 < nc ? rec_off(2 * pp + 1, nv) : -1;
-      const int rs = 2 * ncs_of(nc);
+      // m = N - j - r S1 (m = L + 1, a zero, only at j = 0, r = 2 T3).  S1 and
+      // N are multiples of the block's orders, so the inputs of one thread are
+      // whole block rows apart.
+      static_assert(S1 % kRtmOrders == 0, "orders per rtm block");
+      const bool two = 2 * pp + 1 < nc;  // the pair holds two components
+      const int per = two ? 4 : 2;
+      const double* up = line + (j >> kRtmShift) * bs + pp * 4 * kRtmOrders + (j & (kRtmOrders - 1)) * per;
+      const double* dn = line + ((-j) >> kRtmShift) * bs + pp * 4 * kRtmOrders + ((-j) & (kRtmOrders - 1)) * per;
+      // staged sectors lie 32 bytes apart: lanes 4..7 of each eight read the
+      // second half first, so a quarter warp covers all banks
+      const int hu = !INPLACE && two ? (j >> 1) & 2 : 0, hd = !INPLACE && two ? ((-j) >> 1) & 2 : 0;
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         if (r >= T3 && r < 2 * T3) {
@@ -925,22 +879,30 @@ __device__ __forceinline__ void ff_dif_first(const double* st, int nc, int nv, d
           continue;
         }
         const bool mir = r >= 2 * T3;
-        const int m = mir ? N - j - r * S1 : j + r * S1;
-        const double* rec = INPLACE ? st + (long long)(m <= L ? m : 0) * rsg : st + (m <= L ? m : 0) * rs;
-        const double2 c0 = *reinterpret_cast<const double2*>(rec + o0);
-        const double2 c1 = o1 >= 0 ? *reinterpret_cast<const double2*>(rec + o1) : make_double2(0.0, 0.0);
+        if (mir && r == 2 * T3 && j == 0) {  // order L + 1
+          x[r] = make_double2(0.0, 0.0);
+          continue;
+        }
+        const double* s = mir ? dn + ((N - r * S1) / kRtmOrders) * bs : up + ((r * S1) / kRtmOrders) * bs;
+        const int h = mir ? hd : hu;
+        double2 c0 = *reinterpret_cast<const double2*>(s + h);
+        double2 c1 = two ? *reinterpret_cast<const double2*>(s + (2 - h)) : make_double2(0.0, 0.0);
+        if (!INPLACE && h) {
+          const double2 t = c0;
+          c0 = c1;
+          c1 = t;
+        }
         if (mir) {
-          x[r] = m <= L ? make_double2(0.5 * c0.x - 0.5 * c1.y, 0.5 * c0.y + 0.5 * c1.x) : make_double2(0.0, 0.0);
+          x[r] = make_double2(0.5 * c0.x - 0.5 * c1.y, 0.5 * c0.y + 0.5 * c1.x);
         } else {
-          x[r] = (r == 0 && m == 0) ? make_double2(c0.x, c1.x)
+          x[r] = (r == 0 && j == 0) ? make_double2(c0.x, c1.x)
                                     : make_double2(0.5 * c0.x + 0.5 * c1.y, 0.5 * c1.x - 0.5 * c0.y);
         }
       }
       DFT2F_ZM<3, T3, +1>::run(x);
     } else {
 #pragma unroll
-      for (int r = 0; r < R; ++r)
-        x[r] = INPLACE ? spec_at(st, nc, nv, pp, j + r * S1, N, L, rsg) : spec_at_t(st, nc, nv, pp, j + r * S1, N, L);
+      for (int r = 0; r < R; ++r) x[r] = spec_at(P, line, bs, nc, pp, j + r * S1);
       DFT<R, +1>::run(x);
     }
     double2* zp = z + pp * NP;
@@ -959,38 +921,66 @@ __device__ __forceinline__ void ff_dif_first(const double* st, int nc, int nv, d
   }
 }
 
-// Last forward pass (transpose of ff_dif_first): radix F0 over the whole line,
-// natural-order output.  With PR only the outer thirds of the output (the
-// orders 0..L and their mirrors) are stored.
+// Last forward pass (transpose of ff_dif_first, radix F0 over the whole line)
+// and the record stores.  Butterfly j holds the frequencies j + q S1; order m =
+// j + q S1 needs them and N - m = (S1 - j) + (F0 - 1 - q) S1, which butterfly
+// S1 - j holds: the lanes are arranged so that j and S1 - j share a warp and
+// the mirrors come by shuffles.  The outputs never return to shared memory
+// (separate passes for the butterflies and the stores took 4.0k + 3.5k of a
+// line's 28k cycles at N = 1536), and eight lanes store 256 contiguous bytes.
+// With PR (N = 3 (L + 1)) only the outer thirds of the output are orders or
+// mirrors.
 template <int N, bool PR>
-__device__ __forceinline__ void ff_dit_last(double2* z, int npair, const double2* __restrict__ tw) {
-  constexpr int R = ff_first(N), S1 = N / R, NP = N + 1, T3 = R / 3;
-  for (int it = threadIdx.x; it < npair * S1; it += blockDim.x) {
-    const int pp = it / S1, j = it - pp * S1;
-    double2* zp = z + pp * NP;
+__device__ __forceinline__ void ff_dit_store(const double2* z, int npair, const Plan& P, double* base, long long bs,
+                                             int nc, const double2* __restrict__ tw) {
+  constexpr int R = ff_first(N), S1 = N / R, NP = N + 1;
+  constexpr int QM = PR ? R / 3 : (R + 1) / 2;  // orders j + q S1 <= L < N / 2 have q < QM
+  static_assert(S1 == 64 || S1 == 16, "lane arrangement");
+  const int lane = threadIdx.x & 31, L = P.L;
+  for (int w0 = threadIdx.x - lane; w0 < npair * S1; w0 += blockDim.x) {
+    int pp, j, mate;  // mate: the lane of butterfly S1 - j (itself for j = 0, S1 / 2)
+    if constexpr (S1 == 64) {
+      pp = w0 / S1;
+      if ((w0 & 32) == 0) {  // 0 .. 15, 63 .. 49, 32
+        j = lane < 16 ? lane : lane == 31 ? 32 : 79 - lane;
+        mate = lane == 0 || lane == 31 ? lane : lane < 16 ? lane + 15 : lane - 15;
+      } else {  // 16 .. 31, 48 .. 33
+        j = lane < 16 ? 16 + lane : 64 - lane;
+        mate = lane ^ 16;
+      }
+    } else {
+      pp = (w0 + lane) / S1;
+      j = lane & 15;
+      mate = (lane & 16) | ((16 - j) & 15);
+    }
+    const bool ok = pp < npair;
+    const double2* zp = z + (ok ? pp : 0) * NP;
     double2 x[R];
     TwiddleRun<-1> tr(tw, j);
-    if constexpr (S1 % 64 == 0) {
-      const int jj = j ^ ((j >> 3) & 7);
+    const int jj = j ^ ((j >> 3) & 7);
 #pragma unroll
-      for (int q = 0; q < R; ++q) {
-        const double2 v = zp[(jj ^ (((q * S1) >> 6) & 7)) + q * S1];
-        x[q] = q == 0 ? v : cmul(v, tr.next(q));
-      }
-      DFT<R, -1>::run(x);
+    for (int q = 0; q < R; ++q) {
+      const double2 v = S1 % 64 == 0 ? zp[(jj ^ (((q * S1) >> 6) & 7)) + q * S1] : zp[swf(j + q * S1)];
+      x[q] = q == 0 ? v : cmul(v, tr.next(q));
+    }
+    DFT<R, -1>::run(x);
+    const bool two = 2 * pp + 1 < nc;
+    double* d = base + (j >> kRtmShift) * bs + pp * 4 * kRtmOrders + (j & (kRtmOrders - 1)) * (two ? 4 : 2);
+    const double aN = 1.0 / (double)N;
 #pragma unroll
-      for (int q = 0; q < R; ++q)
-        if (!PR || q < T3 || q >= 2 * T3) zp[(jj ^ (((q * S1) >> 6) & 7)) + q * S1] = x[q];
-    } else {
-#pragma unroll
-      for (int q = 0; q < R; ++q) {
-        const double2 v = zp[swf(j + q * S1)];
-        x[q] = q == 0 ? v : cmul(v, tr.next(q));
-      }
-      DFT<R, -1>::run(x);
-#pragma unroll
-      for (int q = 0; q < R; ++q)
-        if (!PR || q < T3 || q >= 2 * T3) zp[swf(j + q * S1)] = x[q];
+    for (int q = 0; q < QM; ++q) {
+      double2 wm;
+      wm.x = __shfl_sync(0xffffffffu, x[R - 1 - q].x, mate);
+      wm.y = __shfl_sync(0xffffffffu, x[R - 1 - q].y, mate);
+      if (q > 0 && j == 0) wm = x[R - q];
+      const double2 zm = x[q];
+      const bool m0 = q == 0 && j == 0;
+      if (!ok || (!PR && j + q * S1 > L)) continue;
+      double* dq = d + (q * S1 / kRtmOrders) * bs;
+      const double a0 = m0 ? zm.x * aN : (zm.x + wm.x) * aN, b0 = m0 ? 0.0 : (wm.y - zm.y) * aN;
+      const double a1 = m0 ? zm.y * aN : (zm.y + wm.y) * aN, b1 = m0 ? 0.0 : (zm.x - wm.x) * aN;
+      if (two) st_global_v4(dq, a0, b0, a1, b1);
+      else *reinterpret_cast<double2*>(dq) = make_double2(a0, b0);
     }
   }
 }
@@ -998,9 +988,9 @@ __device__ __forceinline__ void ff_dit_last(double2* z, int npair, const double2
 // Middle pass of radix M over span SP = N/F0 (stride SP/M = 4): butterfly
 // block b fastest across threads.  For SP = 64 the swizzle of element r is
 // ((j + 4r) ^ (r/2) ^ (b % 8)) within the block, j < 4.
-template <int N, int SIGN>
+template <int N, int SIGN, int TS = 1>
 __device__ __forceinline__ void ff_mid_pass(double2* z, int npair, const double2* __restrict__ tw) {
-  constexpr int R = ff_mid(N), SP = N / ff_first(N), s = SP / R, nbf = N / R, NB = N / SP, stw = N / SP;
+  constexpr int R = ff_mid(N), SP = N / ff_first(N), s = SP / R, nbf = N / R, NB = N / SP, stw = TS * (N / SP);  // TS: entries of tw per w_N
   constexpr int NP = N + 1;
   for (int it = threadIdx.x; it < npair * nbf; it += blockDim.x) {
     const int pp = it / nbf, rem = it - pp * nbf;
@@ -1051,305 +1041,397 @@ __device__ __forceinline__ void ff_mid_pass(double2* z, int npair, const double2
   }
 }
 
-// Grid products of one grid point: vin = backward components (3 MVB vector
-// components, then MSB scalars, as laid out in the pairs), out = forward
-// components in pair order.
-template <int MVB, int MSB, int MVF, int MSF>
-__device__ __forceinline__ void point_products(const double* vin_all, const Plan& P, double* dense) {
-  constexpr int MCF = 3 * MVF + MSF;
-  const int nvb = P.nvb, nvf = P.nvf, nsf = P.nsf;
-  double vin[3 * MVB > 0 ? 3 * MVB : 1], sin_[MSB > 0 ? MSB : 1];
-#pragma unroll
-  for (int c = 0; c < 3 * MVB; ++c) vin[c] = vin_all[c];
-#pragma unroll
-  for (int q = 0; q < MSB; ++q) sin_[q] = vin_all[3 * nvb + q < 3 * MVB + MSB ? 3 * nvb + q : 0];
-  double out[MCF > 0 ? MCF : 1];
-#pragma unroll
-  for (int i = 0; i < MVF; ++i) {
-    if (i < nvf) {
-      const double cf = P.pcoef[i];
-      double x0, x1, x2;
-      selvec<MVB>(vin, P.pa[i], x0, x1, x2);
-      if (P.pkind[i] == KMHD_PROD_CROSS) {
-        double y0, y1, y2;
-        selvec<MVB>(vin, P.pb[i], y0, y1, y2);
-        out[3 * i + 0] = (x1 * y2 - x2 * y1) * cf;
-        out[3 * i + 1] = (x2 * y0 - x0 * y2) * cf;
-        out[3 * i + 2] = (x0 * y1 - x1 * y0) * cf;
-      } else {
-        const double sv = selscl<MSB>(sin_, P.pb[i]);
-        out[3 * i + 0] = x0 * sv * cf;
-        out[3 * i + 1] = x1 * sv * cf;
-        out[3 * i + 2] = x2 * sv * cf;
-      }
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < MSF; ++j) {
-    if (j < nsf) {
-      const int q = nvf + j;
-      const double cf = P.pcoef[q];
-      double o;
-      if (P.pkind[q] == KMHD_PROD_DOT) {
-        double x0, x1, x2, y0, y1, y2;
-        selvec<MVB>(vin, P.pa[q], x0, x1, x2);
-        selvec<MVB>(vin, P.pb[q], y0, y1, y2);
-        o = (x0 * y0 + x1 * y1 + x2 * y2) * cf;
-      } else {
-        o = selscl<MSB>(sin_, P.pa[q]) * selscl<MSB>(sin_, P.pb[q]) * cf;
-      }
-      out[3 * MVF + j] = o;
-    }
-  }
-#pragma unroll
-  for (int c = 0; c < MCF; ++c) {
-    double v = 0.0;
-    if (c < 3 * MVF) v = out[c < 3 * MVF ? c : 0];
-    if (c >= 3 * nvf) {
-      v = 0.0;
-#pragma unroll
-      for (int j = 0; j < MSF; ++j)
-        if (c == 3 * nvf + j) v = out[3 * MVF + j];
-    }
-    dense[c] = v;
-  }
-}
-
-// Products of the standard MHD set at one grid point: backward (u, omega, B; T),
-// forward (omega x u, u x B, u T; u . omega), coefficients from the plan.
-__device__ __forceinline__ void point_products_mhd(const double* v, const Plan& P, double* o) {
-  const double u0 = v[0], u1 = v[1], u2 = v[2], w0 = v[3], w1 = v[4], w2 = v[5];
-  const double b0 = v[6], b1 = v[7], b2 = v[8], t = v[9];
-  const double c0 = P.pcoef[0], c1 = P.pcoef[1], c2 = P.pcoef[2], c3 = P.pcoef[3];
-  o[0] = (w1 * u2 - w2 * u1) * c0;
-  o[1] = (w2 * u0 - w0 * u2) * c0;
-  o[2] = (w0 * u1 - w1 * u0) * c0;
-  o[3] = (u1 * b2 - u2 * b1) * c1;
-  o[4] = (u2 * b0 - u0 * b2) * c1;
-  o[5] = (u0 * b1 - u1 * b0) * c1;
-  o[6] = u0 * t * c2;
-  o[7] = u1 * t * c2;
-  o[8] = u2 * t * c2;
-  o[9] = (u0 * w0 + u1 * w1 + u2 * w2) * c3;
-}
-
 // Last inverse radix-4 pass + products + first forward radix-4 pass, for the
-// grid points 4b .. 4b+3 of every pair.
-template <int N, int MVB, int MSB, int MVF, int MSF, int PK>
+// grid points 4b .. 4b+3 of every pair.  Register slots: pair v < MV is slot
+// v, list pair k is slot MV + k (at pair nv + k of z).  EX: the plan's counts
+// equal the template's.
+template <int N, int MVB, int MSB, int MVF, int MSF, bool EX, int PK>
 __device__ __forceinline__ void ff_fused(double2* z, const Plan& P) {
   constexpr int NP = N + 1;
-  constexpr int MCB = 3 * MVB + MSB, MCF = 3 * MVF + MSF;
-  constexpr int NPB = (MCB + 1) / 2, NPF = (MCF + 1) / 2;
+  constexpr int VB = MVB > 0 ? MVB : 1, SB = MSB > 0 ? MSB : 1, VF = MVF > 0 ? MVF : 1, SF = MSF > 0 ? MSF : 1;
+  constexpr int FB = MVB + MSB, FF = MVF + MSF;                     // list entries
+  constexpr int NPB = MVB + (FB + 1) / 2, NPF = MVF + (FF + 1) / 2;  // register slots
   constexpr int NPM = NPB > NPF ? NPB : NPF;
-  const int npb = (P.ncb + 1) / 2, npf = (P.ncf + 1) / 2, ncb = P.ncb, ncf = P.ncf;
+  const int nvb = EX ? MVB : P.nvb, nvf = EX ? MVF : P.nvf;
+  const int nlb = EX ? (FB + 1) / 2 : (P.nvb + P.nsb + 1) / 2, nlf = EX ? (FF + 1) / 2 : (P.nvf + P.nsf + 1) / 2;
+  const int nff = EX ? FF : P.nvf + P.nsf;
   for (int b = threadIdx.x; b < N / 4; b += blockDim.x) {
     const int e0 = (4 * b) ^ (((b >> 1) ^ (b >> 4)) & 7);  // swf(4b + r) = e0 ^ r
     double2 v[NPM][4];
 #pragma unroll
-    for (int pp = 0; pp < NPB; ++pp) {
-      if (pp < npb) {
+    for (int s = 0; s < NPB; ++s) {
+      if (s < MVB ? s < nvb : s - MVB < nlb) {
+        const double2* zp = z + (s < MVB ? s : nvb + s - MVB) * NP;
 #pragma unroll
-        for (int r = 0; r < 4; ++r) v[pp][r] = z[pp * NP + (e0 ^ r)];
-        DFT<4, +1>::run(v[pp]);
+        for (int r = 0; r < 4; ++r) v[s][r] = zp[e0 ^ r];
+        DFT<4, +1>::run(v[s]);
+      } else {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) v[s][r] = make_double2(0.0, 0.0);
       }
     }
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      double vin[MCB > 0 ? MCB : 1], dense[MCF > 0 ? MCF : 1];
+      double rr[VB] = {}, th[VB] = {}, ph[VB] = {}, sc[SB] = {};
+      double orr[VF] = {}, oth[VF] = {}, oph[VF] = {}, os[SF] = {};
+      auto lst = [&](int f) { return (f & 1) ? v[MVB + f / 2][r].y : v[MVB + f / 2][r].x; };
 #pragma unroll
-      for (int c = 0; c < MCB; ++c) vin[c] = (c < ncb) ? ((c & 1) ? v[c >> 1][r].y : v[c >> 1][r].x) : 0.0;
-      if constexpr (PK == 1) point_products_mhd(vin, P, dense);
-      else point_products<MVB, MSB, MVF, MSF>(vin, P, dense);
+      for (int q = 0; q < MVB; ++q) {
+        rr[q] = lst(q);
+        th[q] = v[q][r].x;
+        ph[q] = v[q][r].y;
+      }
 #pragma unroll
-      for (int q = 0; q < NPF; ++q)
-        v[q][r] = make_double2(2 * q < ncf ? dense[2 * q] : 0.0, 2 * q + 1 < ncf ? dense[2 * q + 1 < MCF ? 2 * q + 1 : 0] : 0.0);
+      for (int q = 0; q < MSB; ++q) {
+        if constexpr (EX) {
+          sc[q] = lst(MVB + q);
+        } else {
+#pragma unroll
+          for (int f = 0; f < FB; ++f)
+            if (f == nvb + q) sc[q] = lst(f);
+        }
+      }
+      if constexpr (PK > 0) point_products_k<PK>(rr, th, ph, sc, P, orr, oth, oph, os);
+      else point_products<MVB, MSB, MVF, MSF, EX>(rr, th, ph, sc, P, orr, oth, oph, os);
+      // forward list entry f: r of a vector, scalar or (odd count) zero
+      auto out = [&](int f) {
+        if (EX) return f < MVF ? orr[f < MVF ? f : 0] : f < FF ? os[f < MVF ? 0 : (f < FF ? f - MVF : 0)] : 0.0;
+        double x = f < nvf && f < MVF ? orr[f < MVF ? f : 0] : 0.0;
+#pragma unroll
+        for (int q = 0; q < MSF; ++q)
+          if (f == nvf + q && f < nff) x = os[q];
+        return x;
+      };
+#pragma unroll
+      for (int q = 0; q < MVF; ++q) v[q][r] = make_double2(oth[q], oph[q]);
+#pragma unroll
+      for (int k = 0; k < (FF + 1) / 2; ++k) v[MVF + k][r] = make_double2(out(2 * k), out(2 * k + 1));
     }
 #pragma unroll
-    for (int q = 0; q < NPF; ++q) {
-      if (q < npf) {
-        DFT<4, -1>::run(v[q]);
+    for (int s = 0; s < NPF; ++s) {
+      if (s < MVF ? s < nvf : s - MVF < nlf) {
+        DFT<4, -1>::run(v[s]);
+        double2* zp = z + (s < MVF ? s : nvf + s - MVF) * NP;
 #pragma unroll
-        for (int r = 0; r < 4; ++r) z[q * NP + (e0 ^ r)] = v[q][r];
+        for (int r = 0; r < 4; ++r) zp[e0 ^ r] = v[s][r];
       }
     }
   }
 }
 
-template <int N>
-__device__ void ff_store_line(const double2* z, int npair, const Plan& P, double* rtm, int nc, int nv, int th, int r) {
-  constexpr int NP = N + 1;
-  const int L = P.L;
-  const double aN = 1.0 / (double)N;
-  const long long strideM = (long long)P.nth * P.nr * nc * 2;
-  double* base = rtm + rtm_off(P, 0, th, r, nc);
-  for (int it = threadIdx.x; it < (L + 1) * npair; it += blockDim.x) {
-    const int pp = it / (L + 1), m = it - pp * (L + 1);
-    const double2* zp = z + pp * NP;
-    const double2 zm = zp[swf(m)];
-    double a0, b0, a1, b1;
-    if (m == 0) {
-      a0 = zm.x * aN; a1 = zm.y * aN; b0 = 0.0; b1 = 0.0;
-    } else {
-      const double2 wm = zp[swf(N - m)];
-      a0 = (zm.x + wm.x) * aN;
-      b0 = (wm.y - zm.y) * aN;
-      a1 = (zm.y + wm.y) * aN;
-      b1 = (zm.x - wm.x) * aN;
-    }
-    double* rec = base + m * strideM;
-    *reinterpret_cast<double2*>(rec + rec_off(2 * pp, nv)) = make_double2(a0, b0);
-    if (2 * pp + 1 < nc) *reinterpret_cast<double2*>(rec + rec_off(2 * pp + 1, nv)) = make_double2(a1, b1);
-  }
+// shared memory of half a line
+size_t smem_half(const Plan& p) {
+  const int npair = ((p.ncb > p.ncf ? p.ncb : p.ncf) + 1) / 2;
+  return sizeof(double2) * (size_t)npair * (p.nph / 2 + 1);
 }
 
-// Store of the line's forward spectra, one thread per order m writing the
-// whole rtm record (every component's (cos, sin) pair, assembled in registers)
-// as 32-byte stores: each record sector is written once, by one store.  The
-// record holds NC = 3 MVF + MSF pairs (NC even: 16 NC bytes, a multiple of 32).
-template <int N, int MVF, int MSF>
-__device__ void ff_store_records(const double2* z, const Plan& P, double* rtm, int th, int r) {
-  constexpr int NP = N + 1;
-  constexpr int NC = 3 * MVF + MSF, NPF = (NC + 1) / 2;
-  static_assert(NC % 2 == 0, "32-byte record stores need an even component count");
-  const int L = P.L;
-  const double aN = 1.0 / (double)N;
-  const long long strideM = (long long)P.nth * P.nr * NC * 2;
-  double* base = rtm + rtm_off(P, 0, th, r, NC);
-  for (int m = threadIdx.x; m <= L; m += blockDim.x) {
-    double rec[2 * NC];
-    const int im = swf(m), iw = swf(N - m);
-#pragma unroll
-    for (int pp = 0; pp < NPF; ++pp) {
-      const double2* zp = z + pp * NP;
-      const double2 zm = zp[im];
-      double a0, b0, a1, b1;
-      if (m == 0) {
-        a0 = zm.x * aN; a1 = zm.y * aN; b0 = 0.0; b1 = 0.0;
-      } else {
-        const double2 wm = zp[iw];
-        a0 = (zm.x + wm.x) * aN;
-        b0 = (wm.y - zm.y) * aN;
-        a1 = (zm.y + wm.y) * aN;
-        b1 = (zm.x - wm.x) * aN;
-      }
-      rec[rec_off(2 * pp, MVF)] = a0;
-      rec[rec_off(2 * pp, MVF) + 1] = b0;
-      rec[rec_off(2 * pp + 1, MVF)] = a1;
-      rec[rec_off(2 * pp + 1, MVF) + 1] = b1;
-    }
-    double* dst = base + m * strideM;
-#pragma unroll
-    for (int q = 0; q < 2 * NC; q += 4) st_v4(dst + q, rec[q], rec[q + 1], rec[q + 2], rec[q + 3]);
-  }
+// cuTensorMapEncodeTiled, resolved through the runtime (no link-time
+// dependency on the driver library, so the library also loads on hosts
+// without a GPU driver); null when unavailable.
+using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+static EncodeTiledFn encode_tiled() {
+  static const EncodeTiledFn fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      return static_cast<EncodeTiledFn>(nullptr);
+    return reinterpret_cast<EncodeTiledFn>(p);
+  }();
+  return fn;
 }
 
-// Staging of the next line's spectra: with a tensor map (tma != 0) thread 0
-// issues one TMA tensor load per mbox orders: the map views rtm_b as
-// [m][r][theta][record] doubles with a box of (2 ncs, 1, 1, mbox), the two
-// doubles past each record zero-filled, which lands the records at the
-// conflict-free stride 2 ncs that the first pass reads; completion on an
-// mbarrier with a bounded wait.  Otherwise 16-byte cp.async pieces.
+// Tensor map of rtm_b for the staging of k_fft_cycle_f: [block][r][theta][block
+// row], box (block row, 1, 1, all blocks) = one line.  False when a line is not
+// one box (the caller then takes a kernel that does not stage by TMA).
+bool make_rtm_map(const Plan& p, CUtensorMap* map) {
+  const int row = rtm_row(p, p.ncb), nblk = rtm_blocks(p);
+  if (row > 256 || nblk > 256 || !p.rtm_b) return false;
+  const cuuint64_t dims[4] = {(cuuint64_t)row, (cuuint64_t)p.nth, (cuuint64_t)p.nr, (cuuint64_t)nblk};
+  const cuuint64_t strides[3] = {8ull * row, 8ull * row * p.nth, 8ull * row * p.nth * p.nr};
+  const cuuint32_t box[4] = {(cuuint32_t)row, 1, 1, (cuuint32_t)nblk};
+  const cuuint32_t es[4] = {1, 1, 1, 1};
+  const EncodeTiledFn enc = encode_tiled();
+  if (!enc) return false;
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, const_cast<double*>(p.rtm_b), dims, strides, box, es,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// fn(integral_constant<int, I>) for every I of the sequence
+template <typename F, int... I>
+__device__ __forceinline__ void for_constants(F& fn, std::integer_sequence<int, I...>) {
+  (fn(std::integral_constant<int, I>()), ...);
+}
+
+// One line per pass of the loop.  STG: the next line's spectra arrive during
+// the current line by one TMA tensor load (thread 0; one bulk copy per block
+// row, issued by the lanes of warp 0, held that warp up for 5.2k of a line's
+// 28k cycles), completion on an mbarrier with a bounded wait.  Without STG
+// only the grid fits in shared memory: the first pass reads the line's records
+// in place, after an L2 prefetch issued one line ahead.
 // NT threads: fewer threads leave more registers to each for the fused
-// products of many fields (the unstaged variants)
-template <int N, int MVB, int MSB, int MVF, int MSF, bool PR, int PK, bool STG = true, int NT = kFftThreadsF>
+// products of many fields (the unstaged variants).
+template <int N, int MVB, int MSB, int MVF, int MSF, bool EX, bool PR, int PK, bool STG = true, int NT = kFftThreadsF>
 __global__ void __launch_bounds__(NT, kFftThreadsF / NT)
-    k_fft_cycle_f(Plan P, int line0, int nlines, const __grid_constant__ CUtensorMap tmap, int tma, int mbox) {
+    k_fft_cycle_f(const __grid_constant__ Plan P, int line0, int nlines, const __grid_constant__ CUtensorMap tmap) {
   extern __shared__ double4 smraw[];
   constexpr int NP = N + 1;
-  constexpr int NCB = 3 * MVB + MSB, NCS2 = 2 * (NCB | 1);
-  const int npb = (P.ncb + 1) / 2, npf = (P.ncf + 1) / 2;
+  // eight orders per rtm block
+  const int ncb = EX ? 3 * MVB + MSB : P.ncb, ncf = EX ? 3 * MVF + MSF : P.ncf;
+  const int npb = (ncb + 1) / 2, npf = (ncf + 1) / 2;
   const int npair = npb > npf ? npb : npf;
   double2* z = reinterpret_cast<double2*>(smraw);
-  // staged spectra, 128-byte aligned (TMA destination), then the mbarrier
+  // staged spectra, 128-byte aligned, then the mbarrier
   double* st = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(z + npair * NP) + 127) & ~static_cast<uintptr_t>(127));
-  unsigned long long* bar = reinterpret_cast<unsigned long long*>(st + (P.L + 1) * NCS2);
+  const int row = 2 * kRtmOrders * ncb, nblk = (P.L + kRtmOrders) >> kRtmShift;
+  unsigned long long* bar = reinterpret_cast<unsigned long long*>(st + nblk * row);
   int line = line0 + blockIdx.x;
   if (line >= nlines) return;
+  auto rest = [&](int th, int r) {
+    ff_mid_pass<N, +1>(z, npb, P.twid);
+    __syncthreads();
+    ff_fused<N, MVB, MSB, MVF, MSF, EX, PK>(z, P);
+    __syncthreads();
+    ff_mid_pass<N, -1>(z, npf, P.twid);
+    __syncthreads();
+    ff_dit_store<N, PR>(z, npf, P, P.rtm_f + rtm_off(P, 0, th, r, ncf), (long long)P.nth * P.nr * (2 * kRtmOrders) * ncf, ncf, P.twid);
+    __syncthreads();
+  };
   if constexpr (!STG) {
-    // only the grid fits in shared memory: the first pass reads the line's
-    // records in place (order stride nth nr ncb 2)
-    const long long rsg = (long long)P.nth * P.nr * P.ncb * 2;
     for (; line < nlines; line += gridDim.x) {
-      const int th = line % P.nth, r = line / P.nth;
-      ff_dif_first<N, PR, true>(P.rtm_b + rtm_off(P, 0, th, r, P.ncb), P.ncb, P.nvb, z, npb, P.L, P.twid, rsg);
+      const int th = line % P.nth, r = line / P.nth, next = line + gridDim.x;
+      if (threadIdx.x == 0 && next < nlines)
+        asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];\n" ::"l"(
+                         reinterpret_cast<uint64_t>(&tmap)),
+                     "r"(0), "r"(next % P.nth), "r"(next / P.nth), "r"(0)
+                     : "memory");
+      ff_dif_first<N, PR, true>(P, P.rtm_b + rtm_off(P, 0, th, r, ncb), (long long)P.nth * P.nr * row, ncb, z, npb,
+                                P.twid);
       __syncthreads();
-      ff_mid_pass<N, +1>(z, npb, P.twid);
-      __syncthreads();
-      ff_fused<N, MVB, MSB, MVF, MSF, PK>(z, P);
-      __syncthreads();
-      ff_mid_pass<N, -1>(z, npf, P.twid);
-      __syncthreads();
-      ff_dit_last<N, PR>(z, npf, P.twid);
-      __syncthreads();
-      if constexpr ((3 * MVF + MSF) % 2 == 0) ff_store_records<N, MVF, MSF>(z, P, P.rtm_f, th, r);
-      else ff_store_line<N>(z, npf, P, P.rtm_f, P.ncf, P.nvf, th, r);
-      __syncthreads();
+      rest(th, r);
     }
     return;
   }
-  if (tma && threadIdx.x == 0) {
+  if (threadIdx.x == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(ssa(bar)));
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   auto stage = [&](int ln) {
-    const int sth = ln % P.nth, sr = ln / P.nth;
-    if (!tma) {
-      prefetch_line_c<NCB>(st, P.rtm_b, P, sth, sr);
-    } else if (threadIdx.x == 0) {
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(ssa(bar)),
-                   "r"((unsigned)((P.L + 1) * NCS2 * 8)));
-      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // the first pass's reads of st
-      for (int m0 = 0; m0 <= P.L; m0 += mbox)
-        asm volatile(
-            "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
-            "[%6];\n" ::"r"(ssa(st + m0 * NCS2)),
-            "l"(reinterpret_cast<uint64_t>(&tmap)), "r"(0), "r"(sth), "r"(sr), "r"(m0), "r"(ssa(bar))
-            : "memory");
-    }
+    if (threadIdx.x != 0) return;
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(ssa(bar)),
+                 "r"((unsigned)(nblk * row * 8)) : "memory");
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // the first pass's reads of st
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
+        "[%6];\n" ::"r"(ssa(st)),
+        "l"(reinterpret_cast<uint64_t>(&tmap)), "r"(0), "r"(ln % P.nth), "r"(ln / P.nth), "r"(0), "r"(ssa(bar))
+        : "memory");
   };
   __syncthreads();
-  // lines theta fastest: concurrent CTAs touch neighbouring records of one (m, r)
+  // lines theta fastest: concurrent CTAs touch neighbouring rows of one (m block, r)
   stage(line);
   unsigned phase = 0;
   while (line < nlines) {
     const int th = line % P.nth, r = line / P.nth;
-    if (tma) {
-      const bool late = !fbar_wait(bar, phase);
-      phase ^= 1u;
-      if (__syncthreads_or(late)) {
-        // the staging did not complete in time: report it, let the copy land, stop
-        if (threadIdx.x == 0) {
-          if (P.err) atomicExch(P.err, KMHD_ERR_TIMEOUT);
-          (void)fbar_wait(bar, phase ^ 1u);
-        }
-        return;
+    const bool late = !fbar_wait(bar, phase);
+    phase ^= 1u;
+    if (__syncthreads_or(late)) {
+      // the staging did not complete in time: report it, let the copy land, stop
+      if (threadIdx.x == 0) {
+        if (P.err) atomicExch(P.err, KMHD_ERR_TIMEOUT);
+        (void)fbar_wait(bar, phase ^ 1u);
       }
-    } else {
-      cp_async_wait<0>();
-      __syncthreads();
+      return;
     }
-    ff_dif_first<N, PR>(st, P.ncb, P.nvb, z, npb, P.L, P.twid);
+    ff_dif_first<N, PR>(P, st, row, ncb, z, npb, P.twid);
     __syncthreads();
     const int next = line + gridDim.x;
     if (next < nlines) stage(next);
-    ff_mid_pass<N, +1>(z, npb, P.twid);
-    __syncthreads();
-    ff_fused<N, MVB, MSB, MVF, MSF, PK>(z, P);
-    __syncthreads();
-    ff_mid_pass<N, -1>(z, npf, P.twid);
-    __syncthreads();
-    ff_dit_last<N, PR>(z, npf, P.twid);
-    __syncthreads();
-    if constexpr ((3 * MVF + MSF) % 2 == 0) ff_store_records<N, MVF, MSF>(z, P, P.rtm_f, th, r);
-    else ff_store_line<N>(z, npf, P, P.rtm_f, P.ncf, P.nvf, th, r);
-    __syncthreads();
+    rest(th, r);
     line = next;
   }
 }
 
-template <int N, int MVB, int MSB, int MVF, int MSF, bool PR, int PK, bool STG = true, int NT = ff_threads(N)>
-cudaError_t run_cycle_fk(const Plan& p, cudaStream_t s) {
-  auto kern = k_fft_cycle_f<N, MVB, MSB, MVF, MSF, PR, PK, STG, NT>;
+// ---------------------------------------------------------------------------
+// Lines of N = 2 NH longitudes whose NH-point halves fit the specialised passes
+// (N = 3072, NH = 1536).  A radix-2 step splits the line into the grid points of
+// even and odd j: half h is the NH-point inverse transform of
+//   x_h[k] = (X[k] + (-1)^h X[k + NH]) w_N^(h k),
+// it goes through the products and back to its spectrum A_h on its own, and
+//   X[k] = A_0[k] + w_N^-k A_1[k],  X[k + NH] = A_0[k] - w_N^-k A_1[k].
+// So every component of half a line is in shared memory at once; only A_0 waits
+// in the CTA's global scratch (L2), written and read back by the same thread.
+// Going pair by pair with the whole line in the scratch instead took 17.1 ms at
+// L = 1023, Nr = 17.  w_N^(h (j + r S1)) = w_N^(h j) w_48^r: the first factor is
+// common to a butterfly and goes into the twiddles, the second is compile-time.
+template <int NH, int H, bool PR>
+__device__ __forceinline__ void ff_half_first(const Plan& P, const double* line, long long bs, int nc, double2* z,
+                                              int npair) {
+  constexpr int R = ff_first(NH), S1 = NH / R, NP = NH + 1;
+  static_assert(R == 24 && S1 == 64, "w_48 rotations, whole block rows");
+  const int L = P.L;
+  const double2* __restrict__ tw = P.twid;
+  for (int it = threadIdx.x; it < npair * S1; it += blockDim.x) {
+    const int pp = it / S1, j = it - pp * S1;
+    const bool two = 2 * pp + 1 < nc;
+    const int per = two ? 4 : 2;
+    const double* up = line + (j >> kRtmShift) * bs + pp * 4 * kRtmOrders + (j & (kRtmOrders - 1)) * per;
+    const double* dn = line + ((-j) >> kRtmShift) * bs + pp * 4 * kRtmOrders + ((-j) & (kRtmOrders - 1)) * per;
+    const double2 zero = make_double2(0.0, 0.0);
+    double2 x[R];
+    auto input = [&](auto rc) {
+      constexpr int r = decltype(rc)::value;
+      // k = j + r S1 is order k if k <= L; k + NH mirrors order NH - k if that is <= L
+      const int k = j + r * S1;
+      double2 u = zero, d = zero;
+      if ((!PR || r < 2 * R / 3) && (PR || k <= L)) {
+        const double* s = up + (r * S1 / kRtmOrders) * bs;
+        const double2 c0 = *reinterpret_cast<const double2*>(s);
+        const double2 c1 = two ? *reinterpret_cast<const double2*>(s + 2) : zero;
+        u = r == 0 && j == 0 ? make_double2(c0.x, c1.x)
+                             : make_double2(0.5 * c0.x + 0.5 * c1.y, 0.5 * c1.x - 0.5 * c0.y);
+      }
+      if (PR ? r >= R / 3 && (r > R / 3 || j > 0) : NH - k <= L) {
+        const double* s = dn + ((NH - r * S1) / kRtmOrders) * bs;
+        const double2 c0 = *reinterpret_cast<const double2*>(s);
+        const double2 c1 = two ? *reinterpret_cast<const double2*>(s + 2) : zero;
+        d = make_double2(0.5 * c0.x - 0.5 * c1.y, 0.5 * c0.y + 0.5 * c1.x);
+      }
+      x[r] = H == 0 ? cadd(u, d) : rot<48, r, +1>(csub(u, d));
+    };
+    for_constants(input, std::make_integer_sequence<int, R>{});
+    DFT<R, +1>::run(x);
+    double2* zp = z + pp * NP;
+    // w_N^(j (2 q + H)): running product, restarted from the table every eighth q
+    const double2 w1 = twd<+1>(tw, 2 * j);
+    double2 cur = make_double2(1.0, 0.0);
+    const int jj = j ^ ((j >> 3) & 7);
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      cur = (q & 7) == 0 ? (H == 0 && q == 0 ? cur : twd<+1>(tw, j * (2 * q + H))) : cmul(cur, w1);
+      zp[(jj ^ (((q * S1) >> 6) & 7)) + q * S1] = H == 0 && q == 0 ? x[0] : cmul(x[q], cur);
+    }
+  }
+}
+
+// Last forward pass of half H: H = 0 leaves A_0 in the scratch, H = 1 forms the
+// line's spectrum and stores the records (lane arrangement of ff_dit_store:
+// order m = j + q S1 takes X[N - m] from butterfly S1 - j, entry R - 1 - q).
+template <int NH, int H, bool PR>
+__device__ __forceinline__ void ff_half_store(const double2* z, int npair, const Plan& P, double2* __restrict__ sc,
+                                              double* base, long long bs, int nc) {
+  constexpr int R = ff_first(NH), S1 = NH / R, NP = NH + 1;
+  constexpr int QM = PR ? 2 * R / 3 : R;  // orders j + q S1 <= L < NH
+  const double2* __restrict__ tw = P.twid;
+  const int lane = threadIdx.x & 31, L = P.L;
+  for (int w0 = threadIdx.x - lane; w0 < npair * S1; w0 += blockDim.x) {
+    const int pp = w0 / S1, hi = w0 & 32;
+    const int j = hi ? (lane < 16 ? 16 + lane : 64 - lane) : (lane < 16 ? lane : lane == 31 ? 32 : 79 - lane);
+    const int mate = hi ? lane ^ 16 : (lane == 0 || lane == 31 ? lane : lane < 16 ? lane + 15 : lane - 15);
+    const double2* zp = z + pp * NP;
+    double2 x[R];
+    const double2 w1 = twd<-1>(tw, 2 * j);
+    double2 cur = make_double2(1.0, 0.0);
+    const int jj = j ^ ((j >> 3) & 7);
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      cur = q == 0 ? cur : (q & 7) == 0 ? twd<-1>(tw, 2 * j * q) : cmul(cur, w1);
+      const double2 v = zp[(jj ^ (((q * S1) >> 6) & 7)) + q * S1];
+      x[q] = q == 0 ? v : cmul(v, cur);
+    }
+    DFT<R, -1>::run(x);
+    double2* a0 = sc + pp * NH + hi + lane;  // entry q at a0[q S1]
+    if constexpr (H == 0) {
+#pragma unroll
+      for (int q = 0; q < R; ++q) a0[q * S1] = x[q];
+    } else {
+      const double2 wj = twd<-1>(tw, j);
+      auto turn = [&](auto qc) {
+        constexpr int q = decltype(qc)::value;
+        x[q] = rot<48, q, -1>(cmul(x[q], wj));  // w_N^-k A_1[k]
+      };
+      for_constants(turn, std::make_integer_sequence<int, R>{});
+      const bool two = 2 * pp + 1 < nc;
+      double* d = base + (j >> kRtmShift) * bs + pp * 4 * kRtmOrders + (j & (kRtmOrders - 1)) * (two ? 4 : 2);
+      const double aN = 1.0 / (double)(2 * NH);
+      auto put = [&](int q, double2 zm, double2 wm) {
+        if (!PR && j + q * S1 > L) return;
+        const bool m0 = q == 0 && j == 0;
+        double* dq = d + (q * S1 / kRtmOrders) * bs;
+        const double c0 = m0 ? zm.x * aN : (zm.x + wm.x) * aN, s0 = m0 ? 0.0 : (wm.y - zm.y) * aN;
+        const double c1 = m0 ? zm.y * aN : (zm.y + wm.y) * aN, s1 = m0 ? 0.0 : (zm.x - wm.x) * aN;
+        if (two) st_global_v4(dq, c0, s0, c1, s1);
+        else *reinterpret_cast<double2*>(dq) = make_double2(c0, s0);
+      };
+      auto from_mate = [&](double2 v) {
+        return make_double2(__shfl_sync(0xffffffffu, v.x, mate), __shfl_sync(0xffffffffu, v.y, mate));
+      };
+#pragma unroll
+      for (int q = 0; q < R / 2; ++q) {
+        const int p = R - 1 - q;
+        const double2 aq = a0[q * S1], ap = a0[p * S1];
+        // entries q and p of the line: X[k] = a + x, X[k + NH] = a - x
+        double2 wq = from_mate(csub(ap, x[p])), wp = from_mate(csub(aq, x[q]));
+        if (j == 0) {  // mirrors of its own: entry R - q
+          if (q > 0) wq = csub(a0[(R - q) * S1], x[R - q]);
+          wp = csub(a0[(R - p) * S1], x[R - p]);
+        }
+        put(q, cadd(aq, x[q]), wq);
+        if (p < QM) put(p, cadd(ap, x[p]), wp);
+      }
+    }
+  }
+}
+
+template <int NH, int MVB, int MSB, int MVF, int MSF, bool EX, bool PR, int PK>
+__global__ void __launch_bounds__(kFftThreadsF, 1)
+    k_fft_cycle_half(const __grid_constant__ Plan P, int line0, int nlines, const __grid_constant__ CUtensorMap tmap) {
+  extern __shared__ double4 smraw[];
+  constexpr int NP = NH + 1;
+  const int ncb = EX ? 3 * MVB + MSB : P.ncb, ncf = EX ? 3 * MVF + MSF : P.ncf;
+  const int npb = (ncb + 1) / 2, npf = (ncf + 1) / 2;
+  double2* z = reinterpret_cast<double2*>(smraw);
+  double2* sc = P.fft_scratch + (long long)blockIdx.x * (npb > npf ? npb : npf) * P.nph;
+  const long long bsb = (long long)P.nth * P.nr * (2 * kRtmOrders) * ncb, bsf = (long long)P.nth * P.nr * (2 * kRtmOrders) * ncf;
+  for (int line = line0 + blockIdx.x; line < nlines; line += gridDim.x) {
+    const int th = line % P.nth, r = line / P.nth, next = line + gridDim.x;
+    if (threadIdx.x == 0 && next < nlines)
+      asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];\n" ::"l"(
+                       reinterpret_cast<uint64_t>(&tmap)),
+                   "r"(0), "r"(next % P.nth), "r"(next / P.nth), "r"(0)
+                   : "memory");
+    const double* src = P.rtm_b + rtm_off(P, 0, th, r, ncb);
+    double* dst = P.rtm_f + rtm_off(P, 0, th, r, ncf);
+    auto half = [&](auto hc) {
+      constexpr int H = decltype(hc)::value;
+      ff_half_first<NH, H, PR>(P, src, bsb, ncb, z, npb);
+      __syncthreads();
+      ff_mid_pass<NH, +1, 2>(z, npb, P.twid);
+      __syncthreads();
+      ff_fused<NH, MVB, MSB, MVF, MSF, EX, PK>(z, P);
+      __syncthreads();
+      ff_mid_pass<NH, -1, 2>(z, npf, P.twid);
+      __syncthreads();
+      ff_half_store<NH, H, PR>(z, npf, P, sc, dst, bsf, ncf);
+      __syncthreads();
+    };
+    half(std::integral_constant<int, 0>());
+    half(std::integral_constant<int, 1>());
+  }
+}
+
+// the specialised kernels' conditions besides shared memory
+bool ff_usable(const Plan& p, CUtensorMap* map) {
+  std::memset(map, 0, sizeof(*map));
+  return p.mbs == kRtmShift && make_rtm_map(p, map);
+}
+
+template <int N, int MVB, int MSB, int MVF, int MSF, bool EX, bool PR, int PK, bool STG = true, int NT = ff_threads(N)>
+cudaError_t run_cycle_fk(const Plan& p, const CUtensorMap& map, cudaStream_t s) {
+  auto kern = k_fft_cycle_f<N, MVB, MSB, MVF, MSF, EX, PR, PK, STG, NT>;
   const int npair = ((p.ncb > p.ncf ? p.ncb : p.ncf) + 1) / 2;
   const size_t smem = STG ? smem_cycle_f(p) : sizeof(double2) * (size_t)npair * (N + 1);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1364,54 +1446,57 @@ cudaError_t run_cycle_fk(const Plan& p, cudaStream_t s) {
   int grid = nsm * occ;
   if (grid > nlines - line0) grid = nlines - line0;
   if (grid <= 0) return cudaSuccess;
-  CUtensorMap map;
-  std::memset(&map, 0, sizeof(map));
-  int mbox = 1;
-  const int tma = STG && make_rtm_map(p, &map, &mbox) ? 1 : 0;
-  kern<<<grid, NT, smem, s>>>(p, line0, nlines, map, tma, mbox);
+  kern<<<grid, NT, smem, s>>>(p, line0, nlines, map);
   return cudaGetLastError();
 }
 
-// The specialised passes without staging (the first pass reads the records in
-// place), for lines whose grid fits in shared memory but not with the staged
-// spectra; generic products.
-template <int N, int MVB, int MSB, int MVF, int MSF, int NT = kFftThreadsF>
-cudaError_t run_cycle_fu(const Plan& p, cudaStream_t s) {
+// N = 3072 by halves; the standard set at compile time, any other at run time
+template <int MVB, int MSB, int MVF, int MSF, bool EX, bool PR, int PK>
+cudaError_t run_cycle_half(const Plan& p, const CUtensorMap& map, cudaStream_t s) {
+  auto kern = k_fft_cycle_half<1536, MVB, MSB, MVF, MSF, EX, PR, PK>;
+  const size_t smem = smem_half(p);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  int dev = 0, nsm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  const int line0 = p.r_lo * p.nth, nlines = p.r_hi * p.nth;
+  const int grid = std::min(std::min(nsm, p.fft_scratch_ctas), nlines - line0);
+  if (grid <= 0) return cudaSuccess;
+  kern<<<grid, kFftThreadsF, smem, s>>>(p, line0, nlines, map);
+  return cudaGetLastError();
+}
+cudaError_t run_cycle_half(const Plan& p, const CUtensorMap& map, cudaStream_t s) {
   const bool pr = p.nph == 3 * (p.L + 1);
-  return pr ? run_cycle_fk<N, MVB, MSB, MVF, MSF, true, 0, false, NT>(p, s)
-            : run_cycle_fk<N, MVB, MSB, MVF, MSF, false, 0, false, NT>(p, s);
+  if (prod_list(p) == 1)
+    return pr ? run_cycle_half<3, 1, 3, 1, true, true, 1>(p, map, s) : run_cycle_half<3, 1, 3, 1, true, false, 1>(p, map, s);
+  return pr ? run_cycle_half<kMaxVec, kMaxScl, kMaxVec, kMaxScl, false, true, 0>(p, map, s)
+            : run_cycle_half<kMaxVec, kMaxScl, kMaxVec, kMaxScl, false, false, 0>(p, map, s);
 }
 
-// the standard MHD product list, after the vectors-first reordering
-inline bool is_mhd_products(const Plan& p) {
-  if (p.nvb != 3 || p.nsb != 1 || p.nvf != 3 || p.nsf != 1 || p.nprod != 4) return false;
-  const int k[4] = {KMHD_PROD_CROSS, KMHD_PROD_CROSS, KMHD_PROD_VEC_SCALAR, KMHD_PROD_DOT};
-  const int a[4] = {1, 0, 0, 0}, b[4] = {0, 2, 0, 1};
-  for (int i = 0; i < 4; ++i)
-    if (p.pkind[i] != k[i] || p.pa[i] != a[i] || p.pb[i] != b[i]) return false;
-  return true;
-}
-
-template <int N, int MVB, int MSB, int MVF, int MSF>
-cudaError_t run_cycle_f(const Plan& p, cudaStream_t s) {
+// by N = 3 (L + 1) and the product list
+template <int N, int MVB, int MSB, int MVF, int MSF, bool EX, int PK, bool STG, int NT>
+cudaError_t run_cycle_fp(const Plan& p, const CUtensorMap& map, cudaStream_t s) {
   const bool pr = p.nph == 3 * (p.L + 1);
-  if constexpr (MVB == 3 && MSB == 1 && MVF == 3 && MSF == 1) {
-    if (is_mhd_products(p))
-      return pr ? run_cycle_fk<N, MVB, MSB, MVF, MSF, true, 1>(p, s) : run_cycle_fk<N, MVB, MSB, MVF, MSF, false, 1>(p, s);
-  }
-  return pr ? run_cycle_fk<N, MVB, MSB, MVF, MSF, true, 0>(p, s) : run_cycle_fk<N, MVB, MSB, MVF, MSF, false, 0>(p, s);
+  if (PK > 0 && prod_list(p) == PK)
+    return pr ? run_cycle_fk<N, MVB, MSB, MVF, MSF, EX, true, PK, STG, NT>(p, map, s)
+              : run_cycle_fk<N, MVB, MSB, MVF, MSF, EX, false, PK, STG, NT>(p, map, s);
+  return pr ? run_cycle_fk<N, MVB, MSB, MVF, MSF, EX, true, 0, STG, NT>(p, map, s)
+            : run_cycle_fk<N, MVB, MSB, MVF, MSF, EX, false, 0, STG, NT>(p, map, s);
 }
 
-template <int MVB, int MSB, int MVF, int MSF>
+// Staged specialised kernel of the plan's N at its own field counts.
+template <int MVB, int MSB, int MVF, int MSF, int PK>
 cudaError_t run_cycle_n(const Plan& p, cudaStream_t s, bool* handled) {
   *handled = true;
-  if (smem_cycle_f(p) <= 227 * 1024) {
+  CUtensorMap map;
+  if (smem_cycle_f(p) <= 227 * 1024 && ff_usable(p, &map)) {
     switch (p.nph) {
-      case 96: return run_cycle_f<96, MVB, MSB, MVF, MSF>(p, s);
-      case 192: return run_cycle_f<192, MVB, MSB, MVF, MSF>(p, s);
-      case 384: return run_cycle_f<384, MVB, MSB, MVF, MSF>(p, s);
-      case 768: return run_cycle_f<768, MVB, MSB, MVF, MSF>(p, s);
-      case 1536: return run_cycle_f<1536, MVB, MSB, MVF, MSF>(p, s);
+      case 96: return run_cycle_fp<96, MVB, MSB, MVF, MSF, true, PK, true, ff_threads(96)>(p, map, s);
+      case 192: return run_cycle_fp<192, MVB, MSB, MVF, MSF, true, PK, true, ff_threads(192)>(p, map, s);
+      case 384: return run_cycle_fp<384, MVB, MSB, MVF, MSF, true, PK, true, ff_threads(384)>(p, map, s);
+      case 768: return run_cycle_fp<768, MVB, MSB, MVF, MSF, true, PK, true, ff_threads(768)>(p, map, s);
+      case 1536: return run_cycle_fp<1536, MVB, MSB, MVF, MSF, true, PK, true, ff_threads(1536)>(p, map, s);
       default: break;
     }
   }
@@ -1421,26 +1506,51 @@ cudaError_t run_cycle_n(const Plan& p, cudaStream_t s, bool* handled) {
 
 size_t smem_cycle(const Plan& p) {
   const int npair = ((p.ncb > p.ncf ? p.ncb : p.ncf) + 1) / 2;
-  return sizeof(double2) * (size_t)npair * p.nph + sizeof(double) * 2 * (size_t)(p.L + 1) * p.ncb;
+  return sizeof(double2) * (size_t)npair * p.nph + staged_bytes(p);
 }
 
-template <int MVB, int MSB, int MVF, int MSF>
-cudaError_t run_cycle(const Plan& p, cudaStream_t s) {
-  auto kern = k_fft_cycle<MVB, MSB, MVF, MSF>;
-  const size_t smem = smem_cycle(p);
+// Threads of the run-time-radix cycle kernels: about two butterflies of a
+// radix-12 pass per thread, so that short lines leave room for several CTAs
+int generic_threads(const Plan& p, int npair) {
+  const int want = (npair * p.nph / 24 + 31) / 32 * 32;
+  return want < 64 ? 64 : want > kFftThreads ? kFftThreads : want;
+}
+
+template <typename K>
+cudaError_t launch_generic(K kern, const Plan& p, size_t smem, int nt, int max_grid, cudaStream_t s) {
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int dev = 0, nsm = 0, occ = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kFftThreads, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, nt, smem);
   if (occ < 1) occ = 1;
   const int line0 = p.r_lo * p.nth, nlines = p.r_hi * p.nth;
-  int grid = nsm * occ;
-  if (grid > nlines - line0) grid = nlines - line0;
+  int grid = std::min(max_grid > 0 ? max_grid : nsm * occ, nlines - line0);
   if (grid <= 0) return cudaSuccess;
-  kern<<<grid, kFftThreads, smem, s>>>(p, line0, nlines);
+  kern<<<grid, nt, smem, s>>>(p, line0, nlines);
   return cudaGetLastError();
+}
+
+template <int PK>
+cudaError_t run_generic(const Plan& p, cudaStream_t s, bool staged) {
+  const int npair = ((p.ncb > p.ncf ? p.ncb : p.ncf) + 1) / 2;
+  const int nt = generic_threads(p, npair);
+  if (staged) return launch_generic(k_fft_cycle<PK>, p, smem_cycle(p), nt, 0, s);
+  const size_t direct = sizeof(double2) * (size_t)npair * p.nph;
+  if (direct <= 227 * 1024) return launch_generic(k_fft_cycle_direct<PK>, p, direct, nt, 0, s);
+  if (!p.fft_scratch) return cudaErrorInvalidValue;
+  return launch_generic(k_fft_cycle_wide<PK>, p, sizeof(double2) * (size_t)p.nph, kFftThreads, p.fft_scratch_ctas, s);
+}
+cudaError_t run_generic(const Plan& p, cudaStream_t s, bool staged) {
+  switch (prod_list(p)) {
+    case 1: return run_generic<1>(p, s, staged);
+    case 2: return run_generic<2>(p, s, staged);
+    case 3: return run_generic<3>(p, s, staged);
+    case 4: return run_generic<4>(p, s, staged);
+    case 5: return run_generic<5>(p, s, staged);
+    default: return run_generic<0>(p, s, staged);
+  }
 }
 
 // Failure-path self-test: the staging wait on an mbarrier that nothing
@@ -1471,114 +1581,64 @@ size_t fft_smem_bytes(const Plan& p, int npair) {
   return smem_cycle(p);
 }
 
-size_t smem_wide(const Plan& p) { return sizeof(double2) * (size_t)p.nph; }
-
 size_t smem_direct(const Plan& p) {
   const int npair = ((p.ncb > p.ncf ? p.ncb : p.ncf) + 1) / 2;
   return sizeof(double2) * (size_t)npair * p.nph;
 }
 
-template <int MVB, int MSB, int MVF, int MSF>
-cudaError_t run_cycle_direct(const Plan& p, cudaStream_t s) {
-  auto kern = k_fft_cycle_direct<MVB, MSB, MVF, MSF>;
-  const size_t smem = smem_direct(p);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  int dev = 0, nsm = 0, occ = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kFftThreads, smem);
-  if (occ < 1) occ = 1;
-  const int line0 = p.r_lo * p.nth, nlines = p.r_hi * p.nth;
-  int grid = nsm * occ;
-  if (grid > nlines - line0) grid = nlines - line0;
-  if (grid <= 0) return cudaSuccess;
-  kern<<<grid, kFftThreads, smem, s>>>(p, line0, nlines);
-  return cudaGetLastError();
-}
-
-template <int MVB, int MSB, int MVF, int MSF>
-cudaError_t run_cycle_wide(const Plan& p, cudaStream_t s) {
-  auto kern = k_fft_cycle_wide<MVB, MSB, MVF, MSF>;
-  const size_t smem = smem_wide(p);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  if (!p.fft_scratch) return cudaErrorInvalidValue;
-  const int line0 = p.r_lo * p.nth, nlines = p.r_hi * p.nth;
-  const int grid = std::min(p.fft_scratch_ctas, nlines - line0);
-  if (grid <= 0) return cudaSuccess;
-  kern<<<grid, kFftThreads, smem, s>>>(p, line0, nlines);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_fft_cycle(const Plan& p, cudaStream_t s) {
   if (smem_cycle(p) > 227 * 1024 && smem_cycle_f(p) > 227 * 1024) {
     // the specialised passes need (N + 1)-strided pairs: at most 16 pairs more
-    if (smem_direct(p) + 16 * 16 <= 227 * 1024) {
+    CUtensorMap map;
+    if (smem_direct(p) + 16 * 16 <= 227 * 1024 && ff_usable(p, &map)) {
       // the reference's full MHD set (u, omega, B, J + T, C -> five vectors + one scalar) at its own counts
       if (p.nph == 1536 && p.nvb == 4 && p.nsb == 2 && p.nvf == 5 && p.nsf == 1)
-        return run_cycle_fu<1536, 4, 2, 5, 1>(p, s);
+        return run_cycle_fp<1536, 4, 2, 5, 1, true, 3, false, kFftThreadsF>(p, map, s);
       // the dynamo benchmark set (u, omega, B, J + T -> omega x u, J x B, u x B, u T)
       if (p.nph == 1536 && p.nvb == 4 && p.nsb == 1 && p.nvf == 4 && p.nsf == 0)
-        return run_cycle_fu<1536, 4, 1, 4, 0, 256>(p, s);  // 256 threads: 71.8 against 78.8 ms at L=511
-      if (p.nph == 1536) return run_cycle_fu<1536, kMaxVec, kMaxScl, kMaxVec, kMaxScl>(p, s);
-      if (p.nph == 768) return run_cycle_fu<768, kMaxVec, kMaxScl, kMaxVec, kMaxScl>(p, s);
+        return run_cycle_fp<1536, 4, 1, 4, 0, true, 2, false, 256>(p, map, s);
+      if (p.nph == 1536) return run_cycle_fp<1536, kMaxVec, kMaxScl, kMaxVec, kMaxScl, false, 0, false, kFftThreadsF>(p, map, s);
+      if (p.nph == 768) return run_cycle_fp<768, kMaxVec, kMaxScl, kMaxVec, kMaxScl, false, 0, false, kFftThreadsF>(p, map, s);
     }
-    if (smem_direct(p) <= 227 * 1024) return run_cycle_direct<kMaxVec, kMaxScl, kMaxVec, kMaxScl>(p, s);
-    if (p.nvb == 3 && p.nsb == 1 && p.nvf == 3 && p.nsf == 1) return run_cycle_wide<3, 1, 3, 1>(p, s);
-    return run_cycle_wide<kMaxVec, kMaxScl, kMaxVec, kMaxScl>(p, s);
+    if (p.nph == 3072 && p.fft_scratch && smem_half(p) <= 227 * 1024 && ff_usable(p, &map)) return run_cycle_half(p, map, s);
+    return run_generic(p, s, false);
   }
-  if (p.nvb == 3 && p.nsb == 1 && p.nvf == 3 && p.nsf == 1) {
-    bool handled = false;
-    const cudaError_t e = run_cycle_n<3, 1, 3, 1>(p, s, &handled);
-    if (handled) return e;
-    return run_cycle<3, 1, 3, 1>(p, s);
-  }
-  if (p.nvb == 2 && p.nsb == 1 && p.nvf == 2 && p.nsf == 1) {
-    bool handled = false;
-    const cudaError_t e = run_cycle_n<2, 1, 2, 1>(p, s, &handled);
-    if (handled) return e;
-    return run_cycle<2, 1, 2, 1>(p, s);
-  }
-  if (p.nvb == 1 && p.nsb == 1 && p.nvf == 1 && p.nsf == 0) {
-    bool handled = false;
-    const cudaError_t e = run_cycle_n<1, 1, 1, 0>(p, s, &handled);
-    if (handled) return e;
-    return run_cycle<1, 1, 1, 0>(p, s);
-  }
-  return run_cycle<kMaxVec, kMaxScl, kMaxVec, kMaxScl>(p, s);
+  bool handled = false;
+  cudaError_t e = cudaSuccess;
+  if (p.nvb == 3 && p.nsb == 1 && p.nvf == 3 && p.nsf == 1) e = run_cycle_n<3, 1, 3, 1, 1>(p, s, &handled);
+  else if (p.nvb == 2 && p.nsb == 1 && p.nvf == 2 && p.nsf == 1) e = run_cycle_n<2, 1, 2, 1, 4>(p, s, &handled);
+  else if (p.nvb == 1 && p.nsb == 1 && p.nvf == 1 && p.nsf == 0) e = run_cycle_n<1, 1, 1, 0, 5>(p, s, &handled);
+  if (handled) return e;
+  return run_generic(p, s, smem_cycle(p) <= 227 * 1024);
+}
+
+// Radii per CTA (log2) of the separable transforms: eight (64-byte grid accesses)
+// while two CTAs fit on an SM, four or fewer for longer lines; a shell of
+// fewer radii takes what it has.
+static int grid_lrad(const Plan& p) {
+  int l = 3;
+  while (l > 0 && ((sizeof(double2) * (size_t)(p.nph + 1) << l) > (l > 2 ? 110 : 227) * 1024 || (1 << (l - 1)) >= p.nr)) --l;
+  return l;
+}
+
+template <typename K, typename T>
+static cudaError_t launch_grid(K kern, const Plan& p, int npair, T field, cudaStream_t s) {
+  const int l = grid_lrad(p);
+  const size_t smem = sizeof(double2) * (size_t)(p.nph + 1) << l;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  // 16 warps per SM: four CTAs of 128 threads while their lines fit, else two of 256
+  const int nt = 4 * smem <= 226 * 1024 ? kGridThreads / 2 : kGridThreads;
+  kern<<<npair * ((p.nr + (1 << l) - 1) >> l) * p.nth, nt, smem, s>>>(p, field, l);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_fft_bwd_grid(const Plan& p, double* fld, cudaStream_t s) {
-  const int npb = (p.ncb + 1) / 2;
-  const size_t smem = sizeof(double2) * (size_t)npb * p.nph + sizeof(double) * 2 * (size_t)(p.L + 1) * p.ncb;
-  if (smem > 227 * 1024) {
-    const size_t sw = smem_wide(p);
-    cudaError_t e = cudaFuncSetAttribute(k_fft_bwd_grid_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sw);
-    if (e != cudaSuccess) return e;
-    k_fft_bwd_grid_wide<<<p.nr * p.nth, kFftThreads, sw, s>>>(p, fld);
-    return cudaGetLastError();
-  }
-  cudaError_t e = cudaFuncSetAttribute(k_fft_bwd_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  k_fft_bwd_grid<<<p.nr * p.nth, kFftThreads, smem, s>>>(p, fld);
-  return cudaGetLastError();
+  return launch_grid(k_fft_bwd_grid, p, (p.ncb + 1) / 2, fld, s);
 }
 
 cudaError_t launch_fft_fwd_grid(const Plan& p, const double* frc, cudaStream_t s) {
-  const int npf = (p.ncf + 1) / 2;
-  const size_t smem = sizeof(double2) * (size_t)npf * p.nph;
-  if (smem > 227 * 1024) {
-    const size_t sw = sizeof(double2) * (size_t)p.nph;
-    cudaError_t e = cudaFuncSetAttribute(k_fft_fwd_grid_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sw);
-    if (e != cudaSuccess) return e;
-    k_fft_fwd_grid_wide<<<p.nr * p.nth, kFftThreads, sw, s>>>(p, frc);
-    return cudaGetLastError();
-  }
-  cudaError_t e = cudaFuncSetAttribute(k_fft_fwd_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  k_fft_fwd_grid<<<p.nr * p.nth, kFftThreads, smem, s>>>(p, frc);
-  return cudaGetLastError();
+  return launch_grid(k_fft_fwd_grid, p, (p.ncf + 1) / 2, frc, s);
 }
 
 }  // namespace kmhd

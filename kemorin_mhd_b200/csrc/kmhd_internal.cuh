@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 #include "../../include/kmhd_sph.h"
 
 namespace kmhd {
@@ -19,6 +21,7 @@ constexpr int kMaxVec = 5;    // vectors per field group
 constexpr int kMaxScl = 2;    // scalars per field group
 constexpr int kMaxProd = 16;
 constexpr int kMaxFftFactors = 16;
+constexpr int kRtmShift = 3;  // orders per rtm block, log2 (see rtm_off)
 constexpr int kSeedL = 32;    // degrees between on-the-fly recurrence seeds
 constexpr int kWideCtasPerSm = 2;  // resident CTAs per SM of the wide-line FFT cycle (one grid scratch each)
 constexpr long long kSelfTestSpinCap = 1ll << 16;  // bounded-wait rounds of the failure self-test
@@ -26,6 +29,7 @@ constexpr long long kSelfTestSpinCap = 1ll << 16;  // bounded-wait rounds of the
 // Plan of one transform instance (device pointers + sizes).
 struct Plan {
   int L, nth, nph, nr, nh, nh_pad, nr4, nrb;
+  int mbs;  // orders per rtm block, log2 (see rtm_off)
   // radial window [r_lo, r_hi) of the cycle launches (0, nr: every radius);
   // r_lo is a multiple of 16, so the window covers whole radial blocks and
   // whole split-GEMM column tiles
@@ -56,8 +60,8 @@ struct Plan {
   // work buffers
   double* SB;             // packed backward spectra [m][p][kpad][nrb*ncolb_blk]
   const long long* sboff; // [(L+1)*2]
-  double* rtm_b;          // [m][r][th][record of ncb (cos, sin) pairs, see rec_off, rtm_off]
-  double* rtm_f;          // [m][r][th][record of ncf pairs]
+  double* rtm_b;          // backward spectra on the latitudes, ncb (cos, sin) pairs per record (see rtm_off)
+  double* rtm_f;          // forward spectra, ncf pairs per record
   // FFT
   int nfac;
   int fac[kMaxFftFactors];
@@ -78,6 +82,13 @@ __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b)
                : "d"(a), "d"(b));
 }
 
+// 16 x 8 x 4: one B fragment for 16 rows (rows g and g + 8 of lane 4 g + t)
+__device__ __forceinline__ void dmma16(double (&c)[4], double a0, double a1, double b) {
+  asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};\n"
+               : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+               : "d"(a0), "d"(a1), "d"(b));
+}
+
 __device__ __forceinline__ unsigned smem_u32(const void* p) {
   return (unsigned)__cvta_generic_to_shared(p);
 }
@@ -91,23 +102,73 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
 
-// Offset (in doubles) of component c's (cos, sin) pair inside an rtm record of
-// one (m, theta, r): [theta/phi pairs of every vector: (th c, th s, ph c, ph s)]
-// [r pairs of every vector] [scalar pairs].  The theta/phi block of a vector is
-// one 32-byte sector, so tensor-core epilogues write whole sectors.
-__host__ __device__ __forceinline__ int rec_off(int c, int nv) {
-  if (c < 3 * nv) {
-    const int v = c / 3, q = c % 3;
-    return q == 0 ? 4 * nv + 2 * v : 4 * v + 2 * (q - 1);
-  }
-  return 6 * nv + 2 * (c - 3 * nv);
-}
-
-// Offset (in doubles) of the rtm record of (m, theta, r) holding nc (cos, sin)
-// pairs: layout [m][r][theta][record], so the records of one (m, r) are
-// contiguous over theta.
+// rtm records.  The nc components of one (m, theta, r) are taken in pairs, the
+// two real sequences that one complex longitudinal FFT carries: pair v < nv is
+// (theta, phi) of vector v; pair nv + k is entries 2k, 2k + 1 of the list (r of
+// every vector, scalars).  One pair of one order is one 32-byte sector
+// (a_x, b_x, a_y, b_y) (cos, sin); with an odd component count the last pair is
+// (a_x, b_x) alone.  2^mbs = 8 orders form a block, pair-major:
+//   [m / 8][r][theta][pair][m % 8][sector]
+// so a line (r, theta) of the FFT reads and writes contiguous 128 nc bytes per
+// eight orders, 256 bytes per pair (lanes = orders), while the Legendre
+// kernels still move whole sectors (lanes = theta).  With one order per block
+// ([m][r][theta][record]) every lane of the FFT's stores had its own 128-byte
+// line: at L = 511 the store phase took 7.3k of a line's 31k cycles, its
+// scattered sectors a quarter of all L1 data-pipe wavefronts.
+__host__ __device__ __forceinline__ int rtm_blocks(const Plan& P) { return (P.L + (1 << P.mbs)) >> P.mbs; }
+// doubles of one block row (one r, theta)
+__host__ __device__ __forceinline__ int rtm_row(const Plan& P, int nc) { return (2 * nc) << P.mbs; }
+// start of the block row of (m, theta, r)
 __host__ __device__ __forceinline__ long long rtm_off(const Plan& P, int m, int th, int r, int nc) {
-  return (((long long)m * P.nr + r) * P.nth + th) * (2LL * nc);
+  return ((((long long)(m >> P.mbs) * P.nr + r) * P.nth + th) * nc) << (P.mbs + 1);
+}
+// offset of order m's pair q inside its block row
+__host__ __device__ __forceinline__ int rtm_pair(const Plan& P, int m, int q, int nc) {
+  return (q << (P.mbs + 2)) + (m & ((1 << P.mbs) - 1)) * (2 * q + 1 < nc ? 4 : 2);
+}
+// doubles of all records of one direction
+__host__ __device__ __forceinline__ size_t rtm_size(const Plan& P, int nc) {
+  return (size_t)rtm_blocks(P) * P.nr * P.nth * rtm_row(P, nc);
+}
+// pair and part (0: x, 1: y) of component c (three per vector, then scalars)
+__host__ __device__ __forceinline__ int comp_pair(int c, int nv, int* part) {
+  if (c < 3 * nv) {
+    const int v = c / 3, q = c - 3 * v;
+    *part = q == 0 ? (v & 1) : q - 1;
+    return q == 0 ? nv + (v >> 1) : v;
+  }
+  const int f = c - 2 * nv;  // list entry nv + (c - 3 nv)
+  *part = f & 1;
+  return nv + (f >> 1);
+}
+// 32-byte sectors are aligned unless one-order blocks hold an odd count
+__host__ __device__ __forceinline__ bool rtm_aligned(const Plan& P, int nc) { return ((nc << P.mbs) & 1) == 0; }
+
+// 32-byte record loads (256-bit, read-only path), p 32-byte aligned, and the
+// 16-byte halves.  Every lane's sector is the only one of its 128-byte line that
+// this CTA reads, so the lines are kept out of L1: allocating them held the
+// forward slicer at 3.52 ms against 3.24 ms (L = 511, Nr = 65).
+__device__ __forceinline__ void ld_global_v4(const double* p, double& a, double& b, double& c, double& d) {
+  asm volatile("ld.global.nc.L1::no_allocate.v4.f64 {%0, %1, %2, %3}, [%4];\n"
+               : "=d"(a), "=d"(b), "=d"(c), "=d"(d) : "l"(p));
+}
+__device__ __forceinline__ double2 ld_global_v2(const double* p) {
+  double2 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];\n" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  return v;
+}
+// 32-byte record store, p 32-byte aligned; no L1 line either (backward split
+// GEMM 3.51 -> 3.36 ms, FP64 1.61 -> 1.55 ms at L = 255, Nr = 65)
+__device__ __forceinline__ void st_global_v4(double* p, double a, double b, double c, double d) {
+  asm volatile("st.global.L1::no_allocate.v4.f64 [%0], {%1, %2, %3, %4};\n" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
+}
+__device__ __forceinline__ void st_sector(double* p, bool aligned, double a, double b, double c, double d) {
+  if (aligned) {
+    st_global_v4(p, a, b, c, d);
+  } else {
+    reinterpret_cast<double2*>(p)[0] = make_double2(a, b);
+    reinterpret_cast<double2*>(p)[1] = make_double2(c, d);
+  }
 }
 
 // One step of the Schmidt recurrence of order mo at hemisphere latitude th:
@@ -199,6 +260,48 @@ __host__ __device__ __forceinline__ double g6_of(int l, int m) {
 __host__ __device__ __forceinline__ double g3_of(int l) {
   // g(j,3) = l(l+1), overridden to 1/2 at l = 0 (schmidt_poly_on_rtm_grid.f90:109)
   return l == 0 ? 0.5 : (double)(l * (l + 1));
+}
+
+// Radices of the longitudinal FFT, first inverse pass first: the fewest of
+// {2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16} whose product is n, the smallest sum of
+// them, descending but an odd one last where there is one (its unit-stride
+// butterflies then step through the shared-memory banks).  Every pass is one
+// sweep over shared memory: N = 324 takes three (6, 6, 9) where radices 8, 4,
+// 2, 3, 5 took five (FFT at L = 106, Nr = 47: 0.45 -> 0.22 ms).  False unless n is 2^a 3^b 5^c.
+inline bool fft_factors(int n, std::vector<int>& f) {
+  static const int set[] = {16, 15, 12, 10, 9, 8, 6, 5, 4, 3, 2};
+  std::vector<int> cur, best;
+  int best_sum = 0;
+  struct Rec {
+    static void go(int r, int from, int sum, std::vector<int>& cur, std::vector<int>& best, int& best_sum) {
+      if (r == 1) {
+        if (best.empty() || cur.size() < best.size() || (cur.size() == best.size() && sum < best_sum)) {
+          best = cur;
+          best_sum = sum;
+        }
+        return;
+      }
+      if (!best.empty() && cur.size() + 1 > best.size()) return;
+      for (int i = from; i < 11; ++i)
+        if (r % set[i] == 0) {
+          cur.push_back(set[i]);
+          go(r / set[i], i, sum + set[i], cur, best, best_sum);
+          cur.pop_back();
+        }
+    }
+  };
+  f.clear();
+  if (n < 2) return false;
+  Rec::go(n, 0, 0, cur, best, best_sum);
+  if (best.empty() || (int)best.size() > kMaxFftFactors) return false;
+  for (int i = (int)best.size() - 1; i >= 0; --i)
+    if (best[i] % 2) {
+      best.push_back(best[i]);
+      best.erase(best.begin() + i);
+      break;
+    }
+  f = best;
+  return true;
 }
 
 // Launchers (defined in the .cu files).

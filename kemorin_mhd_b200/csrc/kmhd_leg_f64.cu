@@ -308,54 +308,50 @@ __global__ void __launch_bounds__(kThreads + (OTF ? kGenThreadsB : 0), 1) k_leg_
   const int nc = p.ncb;
   double* outN = p.rtm_b + rtm_off(p, m, i, r, nc);
   double* outS = p.rtm_b + rtm_off(p, m, p.nth - 1 - i, r, nc);
+  const bool al = rtm_aligned(p, nc);
+  // (sym, asym) cos and sin of one component -> north and south values
+  auto put = [&](int q, const double (&sy)[4], const double (&as)[4]) {
+    const int o = rtm_pair(p, m, q, nc);
+    if (pair) {
+      st_sector(outN + o, al, sy[0] + as[0], sy[1] + as[1], sy[2] + as[2], sy[3] + as[3]);
+      st_sector(outS + o, al, sy[0] - as[0], sy[1] - as[1], sy[2] - as[2], sy[3] - as[3]);
+    } else {
+      st_sector(outN + o, al, sy[0], sy[1], sy[2], sy[3]);
+    }
+  };
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
-    double sym[6], asym[6];  // r cos, r sin, th cos, th sin, ph cos, ph sin
-    // r component
-    sym[0] = acc[v][4][0][0];
-    asym[0] = acc[v][4][1][0];
-    sym[1] = acc[v][4][0][1];
-    asym[1] = acc[v][4][1][1];
-    // theta: own slot dP*b, mirror slot -/+ m/sin * P*c
-    sym[2] = acc[v][1][1][0] + ms * acc[v][2][0][1];
-    asym[2] = acc[v][1][0][0] + ms * acc[v][2][1][1];
-    sym[3] = acc[v][1][1][1] - ms * acc[v][2][0][0];
-    asym[3] = acc[v][1][0][1] - ms * acc[v][2][1][0];
+    // theta: own slot dP*b, mirror slot -/+ m/sin * P*c;
     // phi: own slot -dP*c, mirror slot +/- m/sin * P*b
-    sym[4] = -acc[v][3][1][0] + ms * acc[v][0][0][1];
-    asym[4] = -acc[v][3][0][0] + ms * acc[v][0][1][1];
-    sym[5] = -acc[v][3][1][1] - ms * acc[v][0][0][0];
-    asym[5] = -acc[v][3][0][1] - ms * acc[v][0][1][0];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      double2 n, s;
-      if (pair) {
-        n.x = sym[2 * c] + asym[2 * c];
-        n.y = sym[2 * c + 1] + asym[2 * c + 1];
-        s.x = sym[2 * c] - asym[2 * c];
-        s.y = sym[2 * c + 1] - asym[2 * c + 1];
-        *reinterpret_cast<double2*>(outS + rec_off(3 * v + c, NV)) = s;
-      } else {
-        n.x = sym[2 * c];
-        n.y = sym[2 * c + 1];
-      }
-      *reinterpret_cast<double2*>(outN + rec_off(3 * v + c, NV)) = n;
-    }
+    const double sy[4] = {acc[v][1][1][0] + ms * acc[v][2][0][1], acc[v][1][1][1] - ms * acc[v][2][0][0],
+                          -acc[v][3][1][0] + ms * acc[v][0][0][1], -acc[v][3][1][1] - ms * acc[v][0][0][0]};
+    const double as[4] = {acc[v][1][0][0] + ms * acc[v][2][1][1], acc[v][1][0][1] - ms * acc[v][2][1][0],
+                          -acc[v][3][0][0] + ms * acc[v][0][1][1], -acc[v][3][0][1] - ms * acc[v][0][1][0]};
+    put(v, sy, as);
   }
+  // radial components and scalars, two list entries per pair
+  constexpr int NF = NV + NS;
 #pragma unroll
-  for (int s2 = 0; s2 < NS; ++s2) {
-    const double sc = accS[s2][0][0], ss = accS[s2][0][1];
-    const double ac = accS[s2][1][0], as = accS[s2][1][1];
-    double2 n, s;
-    const int c = 3 * NV + s2;
-    if (pair) {
-      n.x = sc + ac; n.y = ss + as;
-      s.x = sc - ac; s.y = ss - as;
-      *reinterpret_cast<double2*>(outS + rec_off(c, NV)) = s;
-    } else {
-      n.x = sc; n.y = ss;
+  for (int f = 0; f < NF; f += 2) {
+    double sy[4] = {0.0, 0.0, 0.0, 0.0}, as[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int ff = f + e;
+      if (ff >= NF) break;
+      const double(&c)[2][2] = ff < NV ? acc[ff < NV ? ff : 0][4] : accS[ff < NV ? 0 : ff - NV];
+      sy[2 * e] = c[0][0];
+      sy[2 * e + 1] = c[0][1];
+      as[2 * e] = c[1][0];
+      as[2 * e + 1] = c[1][1];
     }
-    *reinterpret_cast<double2*>(outN + rec_off(c, NV)) = n;
+    if (f + 1 < NF) {
+      put(NV + f / 2, sy, as);
+    } else {  // odd count: the last pair holds one component
+      const int o = rtm_pair(p, m, NV + f / 2, nc);
+      *reinterpret_cast<double2*>(outN + o) =
+          pair ? make_double2(sy[0] + as[0], sy[1] + as[1]) : make_double2(sy[0], sy[1]);
+      if (pair) *reinterpret_cast<double2*>(outS + o) = make_double2(sy[0] - as[0], sy[1] - as[1]);
+    }
   }
 }
 
@@ -410,15 +406,16 @@ k_leg_fwd_f64(Plan p, double* __restrict__ d_rj, long long ld, const int* __rest
   constexpr int kItems = (kKC * kRB * (3 * NV + NS) + kThreads - 1) / kThreads;
   double2 pfN[kItems], pfS[kItems];
   // item it = tid + q kThreads of a chunk is (latitude row, radius u, component
-  // c), the same in every chunk: decomposed once (nc is not a compile-time
-  // constant, so the divisions stay out of the chunk loop), packed as
-  // c | u << 8 | row << 12, or -1 past the chunk's items
+  // in record order e), the same in every chunk: decomposed once, packed as
+  // e | u << 8 | row << 12, or -1 past the chunk's items; neighbouring threads
+  // read the two halves of one record sector
+  constexpr int NC = 3 * NV + NS;
   int item[kItems];
 #pragma unroll
   for (int q = 0; q < kItems; ++q) {
     const int it = tid + q * kThreads;
-    const int rest = it / nc;
-    item[q] = it < kKC * kRB * nc ? (it - rest * nc) | (rest % kRB) << 8 | (rest / kRB) << 12 : -1;
+    const int rest = it / NC;
+    item[q] = it < kKC * kRB * NC ? (it - rest * NC) | (rest % kRB) << 8 | (rest / kRB) << 12 : -1;
   }
   // global loads of one chunk's rtm_f values into registers (overlaps the MMAs)
   auto prefetch = [&](int ch) {
@@ -430,10 +427,11 @@ k_leg_fwd_f64(Plan p, double* __restrict__ d_rj, long long ld, const int* __rest
       if (item[q] >= 0) {
         const int i = th0 + (item[q] >> 12), r = kRB * rb + ((item[q] >> 8) & 15);
         if (i < p.nh && r < p.nr) {
-          const int ro = rec_off(item[q] & 255, NV);
-          pfN[q] = *reinterpret_cast<const double2*>(p.rtm_f + rtm_off(p, m, i, r, nc) + ro);
+          const int e = item[q] & 255;
+          const int ro = rtm_pair(p, m, e >> 1, nc) + 2 * (e & 1);
+          pfN[q] = ld_global_v2(p.rtm_f + rtm_off(p, m, i, r, nc) + ro);
           if (i < p.nth / 2)
-            pfS[q] = *reinterpret_cast<const double2*>(p.rtm_f + rtm_off(p, m, p.nth - 1 - i, r, nc) + ro);
+            pfS[q] = ld_global_v2(p.rtm_f + rtm_off(p, m, p.nth - 1 - i, r, nc) + ro);
         }
       }
     }
@@ -542,13 +540,10 @@ k_leg_fwd_f64(Plan p, double* __restrict__ d_rj, long long ld, const int* __rest
       }
       double* b0 = sB + row * G::CFp;               // parity 0
       double* b1 = sB + G::B_TILE + row * G::CFp;   // parity 1
-      if (c < 3 * NV) {
-        const int v = c / 3, qq = c % 3;
+      if (c < 2 * NV) {
+        const int v = c >> 1;
         const int base = 40 * v + 2 * u;
-        if (qq == 0) {            // r: Zr tile (P)
-          *reinterpret_cast<double2*>(b0 + base + 0) = sy;
-          *reinterpret_cast<double2*>(b1 + base + 0) = as;
-        } else if (qq == 1) {     // theta: U' tile (P, /sin), W tile (dP)
+        if ((c & 1) == 0) {       // theta: U' tile (P, /sin), W tile (dP)
           *reinterpret_cast<double2*>(b0 + base + 16) = syn;
           *reinterpret_cast<double2*>(b1 + base + 16) = asn;
           *reinterpret_cast<double2*>(b0 + base + 24) = as;
@@ -559,9 +554,9 @@ k_leg_fwd_f64(Plan p, double* __restrict__ d_rj, long long ld, const int* __rest
           *reinterpret_cast<double2*>(b0 + base + 32) = as;
           *reinterpret_cast<double2*>(b1 + base + 32) = sy;
         }
-      } else {
-        const int sc = c - 3 * NV;
-        const int base = 40 * NV + 8 * sc + 2 * u;
+      } else {                    // list entry f: r of a vector (Zr tile, P) or a scalar
+        const int f = c - 2 * NV;
+        const int base = (f < NV ? 40 * f : 40 * NV + 8 * (f - NV)) + 2 * u;
         *reinterpret_cast<double2*>(b0 + base) = sy;
         *reinterpret_cast<double2*>(b1 + base) = as;
       }
@@ -626,6 +621,472 @@ k_leg_fwd_f64(Plan p, double* __restrict__ d_rj, long long ld, const int* __rest
     o[jp] = accS[s][0] * g6;
     if (jn >= 0) o[jn] = accS[s][1] * g6;
   }
+}
+
+// ---------------------------------------------------------------------------
+// Forward kernel of the stored tables.  CTA = (m, 64 degrees per parity, 4 radii,
+// field group); 8 warps = (parity, 16 degrees).  Each warp's m16n8k4 DMMAs use a
+// B fragment for 16 degrees (the 8-degree kernel above reads one per 8: its
+// shared-memory reads alone took 62% of the L1 data pipe at 45% DMMA), each
+// staged B chunk serves 64 degrees instead of 32, and both operands are double
+// buffered, so a chunk costs one barrier and its staging runs beside the other
+// warps' DMMAs.  A field group holds at most three vectors (16 accumulator tiles
+// of four doubles per lane; more would spill): groups share nothing but the A
+// operand, so larger sets run group by group.
+constexpr int kLB16 = 64;  // degrees per parity of a CTA
+
+template <int NV, int NS>
+struct Fwd16Geo {
+  static constexpr int CF = 40 * NV + 8 * NS;
+  static constexpr int CFp = CF + ((4 - CF % 16) + 16) % 16;
+  static constexpr int AS = kKC + 4;
+  static constexpr int A_TILE = kLB16 * AS;
+  static constexpr int B_TILE = kKC * CFp;
+  static constexpr size_t SMEM = sizeof(double) * 2 * (4 * A_TILE + 2 * B_TILE);
+};
+
+// group: vectors v0 .. v0 + NV - 1 and scalars s0 .. s0 + NS - 1 of the plan's forward fields
+template <int NV, int NS>
+__global__ void __launch_bounds__(kThreads, 1)
+k_leg_fwd16(const __grid_constant__ Plan p, double* __restrict__ d_rj, long long ld, const int* __restrict__ cols, int v0,
+            int s0) {
+  using G = Fwd16Geo<NV, NS>;
+  extern __shared__ double sm[];
+  double* sA = sm;                  // [2][P_e, P_o, dP_e, dP_o][kLB16][AS]
+  double* sB = sm + 8 * G::A_TILE;  // [2][par][kKC][CFp]
+  const int m = blockIdx.y;
+  const int nrbw = win_nrb(p);
+  const int kb = blockIdx.x / nrbw;
+  const int rb = win_rb0(p) + blockIdx.x % nrbw;
+  const int k0 = kb * kLB16;
+  if (k0 >= kcount(p.L, m, 0)) return;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int g = lane >> 2, t = lane & 3;
+  const int par = warp & 1, rgi = warp >> 1;
+  const int nc = p.ncf;
+  const int nchunk = p.nh_pad / kKC;
+  const bool active = k0 + 16 * rgi < kcount(p.L, m, par);  // else no degree of this warp exists
+
+  double acc[NV > 0 ? NV : 1][5][4];
+  double accS[NS > 0 ? NS : 1][4];
+#pragma unroll
+  for (int v = 0; v < (NV > 0 ? NV : 1); ++v)
+#pragma unroll
+    for (int q = 0; q < 5; ++q)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[v][q][e] = 0.0;
+#pragma unroll
+  for (int s = 0; s < (NS > 0 ? NS : 1); ++s)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) accS[s][e] = 0.0;
+
+  // items of a chunk: (latitude row, radius u, component e of the group in
+  // record order), the same in every chunk: record offset and tile column
+  // decomposed once
+  constexpr int NC = 3 * NV + NS;
+  constexpr int kItems = (kKC * kRB * NC + kThreads - 1) / kThreads;
+  double2 pfN[kItems], pfS[kItems];
+  int item[kItems];  // e | u << 8 | row << 12, or -1 past the items
+  int roff[kItems];  // offset of the component inside the record
+#pragma unroll
+  for (int q = 0; q < kItems; ++q) {
+    const int it = tid + q * kThreads;
+    const int rest = it / NC, e = it - rest * NC;
+    item[q] = it < kKC * kRB * NC ? e | (rest % kRB) << 8 | (rest / kRB) << 12 : -1;
+    if (e < 2 * NV) {
+      roff[q] = rtm_pair(p, m, v0 + (e >> 1), nc) + 2 * (e & 1);
+    } else {
+      const int f = e - 2 * NV, li = f < NV ? v0 + f : p.nvf + s0 + f - NV;
+      roff[q] = rtm_pair(p, m, p.nvf + (li >> 1), nc) + 2 * (li & 1);
+    }
+    if (item[q] >= 0 && kRB * rb + ((item[q] >> 8) & 15) >= p.nr) item[q] |= 1 << 30;  // past the last radius: zeros
+  }
+  const long long rowTh = rtm_row(p, nc);
+  const double* recN[kItems];
+#pragma unroll
+  for (int q = 0; q < kItems; ++q)
+    recN[q] = p.rtm_f + rtm_off(p, m, 0, min(kRB * rb + ((item[q] >> 8) & 15), p.nr - 1), nc) + roff[q];
+  auto prefetch = [&](int ch) {
+#pragma unroll
+    for (int q = 0; q < kItems; ++q) {
+      pfN[q] = make_double2(0.0, 0.0);
+      pfS[q] = make_double2(0.0, 0.0);
+      const int i = ch * kKC + ((item[q] >> 12) & 15);
+      if (item[q] >= 0 && item[q] < (1 << 30) && i < p.nh) {
+        pfN[q] = ld_global_v2(recN[q] + i * rowTh);
+        if (i < p.nth / 2) pfS[q] = ld_global_v2(recN[q] + (p.nth - 1 - i) * rowTh);
+      }
+    }
+  };
+  const int rows0 = min(kLB16, p.kpad[2 * m] - k0), rows1 = min(kLB16, p.kpad[2 * m + 1] - k0);
+  auto loadA = [&](int st, int ch) {
+    // P_e, P_o, dP_e, dP_o: the degrees that exist (padded to kKC) x 16 latitudes
+#pragma unroll
+    for (int it = tid; it < 4 * kLB16 * (kKC / 2); it += kThreads) {
+      const int tb = it / (kLB16 * (kKC / 2));
+      const int rem = it % (kLB16 * (kKC / 2));
+      const int row = rem / (kKC / 2), c2 = rem % (kKC / 2);
+      if (row < ((tb & 1) ? rows1 : rows0))
+        cp_async16(sA + (st * 4 + tb) * G::A_TILE + row * G::AS + 2 * c2,
+                   (tb < 2 ? p.P : p.dP) + p.poff[2 * m + (tb & 1)] + (long long)(k0 + row) * p.nh_pad + ch * kKC + 2 * c2);
+    }
+    cp_async_commit();
+  };
+  // sym / asym of the prefetched values with the Gauss weights
+  auto storeB = [&](int st, int ch) {
+#pragma unroll
+    for (int q = 0; q < kItems; ++q) {
+      if (item[q] < 0) continue;
+      const int e = item[q] & 255, u = (item[q] >> 8) & 15, row = (item[q] >> 12) & 15;
+      const int i = ch * kKC + row;
+      const double wp = i < p.nh ? __ldg(p.weight + i) : 0.0;
+      const double2 nv = pfN[q], sv = pfS[q];
+      const bool eq = i >= p.nth / 2;  // equator row: no southern partner
+      const double2 sy = make_double2((nv.x + sv.x) * wp, (nv.y + sv.y) * wp);
+      const double2 as = eq ? make_double2(0.0, 0.0) : make_double2((nv.x - sv.x) * wp, (nv.y - sv.y) * wp);
+      double* b0 = sB + (2 * st) * G::B_TILE + row * G::CFp;      // parity 0
+      double* b1 = sB + (2 * st + 1) * G::B_TILE + row * G::CFp;  // parity 1
+      if (e < 2 * NV) {
+        const double ai = i < p.nh ? __ldg(p.asin_t + i) : 0.0;
+        const double2 syn = make_double2(sy.x * ai, sy.y * ai), asn = make_double2(as.x * ai, as.y * ai);
+        const int base = 40 * (e >> 1) + 2 * u;
+        // theta: U' (P, /sin) and W (dP) tiles; phi: U (P, /sin) and W' (dP) tiles
+        const int c1 = base + ((e & 1) ? 8 : 16), c2 = base + ((e & 1) ? 32 : 24);
+        *reinterpret_cast<double2*>(b0 + c1) = syn;
+        *reinterpret_cast<double2*>(b1 + c1) = asn;
+        *reinterpret_cast<double2*>(b0 + c2) = as;
+        *reinterpret_cast<double2*>(b1 + c2) = sy;
+      } else {  // r of a vector (Zr tile, P) or a scalar
+        const int f = e - 2 * NV;
+        const int base = (f < NV ? 40 * f : 40 * NV + 8 * (f - NV)) + 2 * u;
+        *reinterpret_cast<double2*>(b0 + base) = sy;
+        *reinterpret_cast<double2*>(b1 + base) = as;
+      }
+    }
+  };
+
+  prefetch(0);
+  loadA(0, 0);
+  storeB(0, 0);
+  if (nchunk > 1) prefetch(1);
+  cp_async_wait<0>();
+  __syncthreads();
+  auto stage_next = [&](int ch) {
+    if (ch + 1 < nchunk) {
+      loadA((ch & 1) ^ 1, ch + 1);
+      storeB((ch & 1) ^ 1, ch + 1);
+      if (ch + 2 < nchunk) prefetch(ch + 2);
+    }
+  };
+  auto compute = [&](int ch) {
+    const int st = ch & 1;
+    if (!active) return;
+    const double* aP = sA + (st * 4 + par) * G::A_TILE + (rgi * 16 + g) * G::AS + t;
+    const double* adP = sA + (st * 4 + 2 + par) * G::A_TILE + (rgi * 16 + g) * G::AS + t;
+    const double* bb = sB + (2 * st + par) * G::B_TILE + t * G::CFp + g;
+#pragma unroll
+    for (int kk = 0; kk < kKC / 4; ++kk) {
+      const double a0 = aP[4 * kk], a1 = aP[8 * G::AS + 4 * kk];
+      const double d0 = adP[4 * kk], d1 = adP[8 * G::AS + 4 * kk];
+      const double* brow = bb + 4 * kk * G::CFp;
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        dmma16(acc[v][0], a0, a1, brow[40 * v + 0]);   // Zr
+        dmma16(acc[v][1], a0, a1, brow[40 * v + 8]);   // U
+        dmma16(acc[v][2], a0, a1, brow[40 * v + 16]);  // U'
+        dmma16(acc[v][3], d0, d1, brow[40 * v + 24]);  // W
+        dmma16(acc[v][4], d0, d1, brow[40 * v + 32]);  // W'
+      }
+#pragma unroll
+      for (int s = 0; s < NS; ++s) dmma16(accS[s], a0, a1, brow[40 * NV + 8 * s]);
+    }
+  };
+  // the two warps of a scheduler (warp, warp + 4) take staging and DMMAs in
+  // opposite order, so the tensor pipe works through the staging too
+  for (int ch = 0; ch < nchunk; ++ch) {
+    if (warp < 4) stage_next(ch);
+    compute(ch);
+    if (warp >= 4) stage_next(ch);
+    cp_async_wait<0>();
+    __syncthreads();
+  }
+
+  // ---- epilogue (cal_sp_rlm_vector_sym_matmul / _scalar_)
+  const int r = kRB * rb + t;
+  if (!active || r >= p.nr) return;
+  const double r1 = p.radius[r], r2 = r1 * r1, gm = (double)m;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {  // accumulator rows g, g + 8
+    const int l = m + 2 * (k0 + rgi * 16 + 8 * h + g) + par;
+    if (l > p.L) continue;
+    const double g7 = g7_of(l, m);
+    const long long jp = p.jmap[((long long)m * 2 + 0) * (p.L + 1) + l] + p.J * r;
+    const long long jn = m > 0 ? p.jmap[((long long)m * 2 + 1) * (p.L + 1) + l] + p.J * r : -1;
+    const int e = 2 * h;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      double* o = d_rj + ld * cols[v0 + v];
+      // + slot (cos), gm = +m
+      o[jp] = acc[v][0][e] * r2 * g7;
+      o[jp + ld] = acc[v][3][e] * r1 * g7 - acc[v][1][e + 1] * r1 * g7 * gm;
+      o[jp + 2 * ld] = -(acc[v][2][e + 1] * r1 * g7 * gm) - acc[v][4][e] * r1 * g7;
+      if (jn >= 0) {  // - slot (sin), gm = -m
+        o[jn] = acc[v][0][e + 1] * r2 * g7;
+        o[jn + ld] = acc[v][3][e + 1] * r1 * g7 - acc[v][1][e] * r1 * g7 * (-gm);
+        o[jn + 2 * ld] = -(acc[v][2][e] * r1 * g7 * (-gm)) - acc[v][4][e + 1] * r1 * g7;
+      }
+    }
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      double* o = d_rj + ld * cols[p.nvf + s0 + s];
+      const double g6 = g6_of(l, m);
+      o[jp] = accS[s][e] * g6;
+      if (jn >= 0) o[jn] = accS[s][e + 1] * g6;
+    }
+  }
+}
+
+template <int NV, int NS>
+cudaError_t run_fwd16(const Plan& p, double* d_rj, long long ld, const int* cols, cudaStream_t s, int m_count, int v0,
+                      int s0) {
+  auto kern = k_leg_fwd16<NV, NS>;
+  const size_t smem = Fwd16Geo<NV, NS>::SMEM;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  const int nkb = (kcount(p.L, 0, 0) + kLB16 - 1) / kLB16;
+  if (win_nrb(p) <= 0) return cudaSuccess;
+  kern<<<dim3(nkb * win_nrb(p), m_count), kThreads, smem, s>>>(p, d_rj, ld, cols, v0, s0);
+  return cudaGetLastError();
+}
+// ---------------------------------------------------------------------------
+// Backward kernel of the stored tables.  CTA = (m, 64 latitudes, 8 radii, field
+// group); 8 warps = (16 latitudes, 4 radii).  The +-m cross terms are summed
+// inside the accumulators: m/sin P is a third A operand and the mirror slot's
+// columns are B fragments of the neighbouring column with a sign, so a vector
+// needs six output tiles (sym / asym of r, theta, phi) where separate P and dP
+// products of each parity take ten, and 16 latitudes per warp (m16n8k4) fit the
+// registers: one B fragment serves 16 rows.  Operands come through a ring of
+// four cp.async stages, one barrier per chunk.  A field group holds at most
+// three vectors (see k_leg_fwd16); groups start at even vectors, so no record
+// pair is split between two of them.
+constexpr int kRing16 = 4;
+
+template <int NV, int NS>
+struct Bwd16Geo {
+  static constexpr int CB = 24 * NV + 8 * NS;
+  static constexpr int CBp = CB + ((4 - CB % 16) + 16) % 16;
+  static constexpr int AS = kThBlk + 4;
+  static constexpr int A_STAGE = 2 * kKC * AS;
+  static constexpr int B_STAGE = 2 * kKC * CBp;  // two radial blocks
+  static constexpr size_t SMEM = sizeof(double) * kRing16 * (A_STAGE + B_STAGE);
+};
+
+template <int NV, int NS>
+__global__ void __launch_bounds__(kThreads, 1) k_leg_bwd16(const __grid_constant__ Plan p, int v0, int s0) {
+  using G = Bwd16Geo<NV, NS>;
+  extern __shared__ double sm[];
+  double* sA = sm;                            // [ring][P, dP][kKC][AS]
+  double* sB = sm + kRing16 * G::A_STAGE;     // [ring][2 radial blocks][kKC][CBp]
+  const int nthb = p.nh_pad / kThBlk;
+  const int nrbw = win_nrb(p), nrp = (nrbw + 1) / 2;
+  int b = blockIdx.x;
+  const int rp = b % nrp;
+  b /= nrp;
+  const int th0 = (b % nthb) * kThBlk;
+  const int m = b / nthb;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int g = lane >> 2, t = lane & 3;
+  const int tg = warp & 3, rbi = warp >> 2;
+  const int nrb_here = min(2, nrbw - 2 * rp);  // radial blocks of this CTA
+  const int rb0 = win_rb0(p) + 2 * rp;
+  const int n0 = p.kpad[2 * m] / kKC, n1 = p.kpad[2 * m + 1] / kKC;
+  const int total = n0 + n1;
+  const int CBt = 24 * p.nvb + 8 * p.nsb;     // columns of one radial block in SB
+  const long long rowB = (long long)p.nrb * CBt;
+  const bool active = rbi < nrb_here && th0 + 16 * tg < p.nh;
+
+  auto load = [&](int step) {
+    const int st = step % kRing16;
+    const int par = step < n0 ? 0 : 1;
+    const int ch = step < n0 ? step : step - n0;
+    const long long po = p.poff[2 * m + par] + (long long)(ch * kKC) * p.nh_pad + th0;
+    double* a = sA + st * G::A_STAGE;
+#pragma unroll
+    for (int it = tid; it < 2 * kKC * (kThBlk / 2); it += kThreads) {
+      const int tb = it / (kKC * (kThBlk / 2));
+      const int rem = it % (kKC * (kThBlk / 2));
+      const int row = rem / (kThBlk / 2), c2 = rem % (kThBlk / 2);
+      cp_async16(a + (tb * kKC + row) * G::AS + 2 * c2, (tb ? p.dP : p.P) + po + (long long)row * p.nh_pad + 2 * c2);
+    }
+    const double* Bg = p.SB + p.sboff[2 * m + par] + (long long)(ch * kKC) * rowB + (long long)rb0 * CBt;
+    double* bs = sB + st * G::B_STAGE;
+    constexpr int NV2 = 12 * NV, NP2 = 12 * NV + 4 * NS;  // 16-byte pieces of a row: vectors, all
+    for (int it = tid; it < 2 * kKC * NP2; it += kThreads) {
+      const int rr = it / NP2, c2 = it - rr * NP2;  // rr = radial block * kKC + row
+      const int q = rr / kKC, row = rr % kKC;
+      if (q >= nrb_here) break;
+      const int src = c2 < NV2 ? 24 * v0 + 2 * c2 : 24 * p.nvb + 8 * s0 + 2 * (c2 - NV2);
+      cp_async16(bs + rr * G::CBp + 2 * c2, Bg + row * rowB + q * CBt + src);
+    }
+  };
+
+  // tiles of a vector: [r, theta, phi][sym, asym]; of a scalar: [sym, asym]
+  double acc[NV > 0 ? NV : 1][3][2][4];
+  double accS[NS > 0 ? NS : 1][2][4];
+#pragma unroll
+  for (int v = 0; v < (NV > 0 ? NV : 1); ++v)
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+#pragma unroll
+      for (int s = 0; s < 2; ++s)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[v][q][s][e] = 0.0;
+#pragma unroll
+  for (int v = 0; v < (NS > 0 ? NS : 1); ++v)
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) accS[v][s][e] = 0.0;
+
+  const int i0 = th0 + 16 * tg + g;  // latitudes i0, i0 + 8
+  const double ms0 = i0 < p.nh ? (double)m * p.asin_t[i0] : 0.0;
+  const double ms1 = i0 + 8 < p.nh ? (double)m * p.asin_t[i0 + 8] : 0.0;
+  const double sg = (g & 1) ? -1.0 : 1.0;  // mirror slot: cos takes +sin, sin takes -cos
+
+  // chunk of parity par: P feeds sym (par = 0) or asym r, dP asym or sym, m/sin P sym or asym theta / phi
+  auto compute = [&](int st, auto parc) {
+    constexpr int par = decltype(parc)::value;
+    const double* a = sA + st * G::A_STAGE + t * G::AS + 16 * tg + g;
+    const double* bs = sB + st * G::B_STAGE + (rbi * kKC + t) * G::CBp;
+#pragma unroll
+    for (int kk = 0; kk < kKC / 4; ++kk) {
+      const double p0 = a[4 * kk * G::AS], p1 = a[4 * kk * G::AS + 8];
+      const double d0 = a[(kKC + 4 * kk) * G::AS], d1 = a[(kKC + 4 * kk) * G::AS + 8];
+      const double q0 = ms0 * p0, q1 = ms1 * p1;
+      const double* br = bs + 4 * kk * G::CBp;
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        const double bX = br[24 * v + g], bY = br[24 * v + 8 + g], bZ = br[24 * v + 16 + g];
+        const double mX = sg * br[24 * v + (g ^ 1)], mY = sg * br[24 * v + 8 + (g ^ 1)];
+        dmma16(acc[v][0][par], p0, p1, bZ);
+        dmma16(acc[v][1][1 - par], d0, d1, bX);
+        dmma16(acc[v][1][par], q0, q1, mY);
+        dmma16(acc[v][2][1 - par], d0, d1, -bY);
+        dmma16(acc[v][2][par], q0, q1, mX);
+      }
+#pragma unroll
+      for (int s = 0; s < NS; ++s) dmma16(accS[s][par], p0, p1, br[24 * NV + 8 * s + g]);
+    }
+  };
+
+#pragma unroll
+  for (int q = 0; q < kRing16 - 1; ++q) {
+    if (q < total) load(q);
+    cp_async_commit();
+  }
+  for (int step = 0; step < total; ++step) {
+    cp_async_wait<kRing16 - 2>();
+    __syncthreads();  // stage step has landed; every warp is done with the stage that load() overwrites
+    if (step + kRing16 - 1 < total) load(step + kRing16 - 1);
+    cp_async_commit();
+    if (active) {
+      if (step < n0) compute(step % kRing16, std::integral_constant<int, 0>());
+      else compute(step % kRing16, std::integral_constant<int, 1>());
+    }
+  }
+  cp_async_wait<0>();
+
+  // ---- epilogue: north = sym + asym, south = sym - asym
+  const int r = kRB * (rb0 + rbi) + t;
+  if (!active || r >= p.nr) return;
+  const int nc = p.ncb;
+  const bool al = rtm_aligned(p, nc);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int i = i0 + 8 * h, e = 2 * h;
+    if (i >= p.nh) continue;
+    const bool pair = i < p.nth / 2;
+    double* outN = p.rtm_b + rtm_off(p, m, i, r, nc);
+    double* outS = p.rtm_b + rtm_off(p, m, p.nth - 1 - i, r, nc);
+    // two components x, y: [sym, asym] tiles -> one record sector of each hemisphere
+    auto put = [&](int q, const double(&x)[2][4], const double(&y)[2][4]) {
+      const int o = rtm_pair(p, m, q, nc);
+      if (pair) {
+        st_sector(outN + o, al, x[0][e] + x[1][e], x[0][e + 1] + x[1][e + 1], y[0][e] + y[1][e], y[0][e + 1] + y[1][e + 1]);
+        st_sector(outS + o, al, x[0][e] - x[1][e], x[0][e + 1] - x[1][e + 1], y[0][e] - y[1][e], y[0][e + 1] - y[1][e + 1]);
+      } else {
+        st_sector(outN + o, al, x[0][e], x[0][e + 1], y[0][e], y[0][e + 1]);
+      }
+    };
+#pragma unroll
+    for (int v = 0; v < NV; ++v) put(v0 + v, acc[v][1], acc[v][2]);
+    // radial components and scalars, two list entries per pair (v0 is even; the
+    // scalars follow the last group's vectors)
+    constexpr int NF = NV + NS;
+#pragma unroll
+    for (int f = 0; f < NF; f += 2) {
+      const double(&x)[2][4] = f < NV ? acc[f < NV ? f : 0][0] : accS[f < NV ? 0 : f - NV];
+      if (f + 1 < NF) {
+        const double(&y)[2][4] = f + 1 < NV ? acc[f + 1 < NV ? f + 1 : 0][0] : accS[f + 1 < NV ? 0 : (f + 1 < NF ? f + 1 - NV : 0)];
+        put(p.nvb + (v0 + f) / 2, x, y);
+      } else {  // odd count: the last pair holds one component
+        const int o = rtm_pair(p, m, p.nvb + (v0 + f) / 2, nc);
+        *reinterpret_cast<double2*>(outN + o) =
+            pair ? make_double2(x[0][e] + x[1][e], x[0][e + 1] + x[1][e + 1]) : make_double2(x[0][e], x[0][e + 1]);
+        if (pair) *reinterpret_cast<double2*>(outS + o) = make_double2(x[0][e] - x[1][e], x[0][e + 1] - x[1][e + 1]);
+      }
+    }
+  }
+}
+
+template <int NV, int NS>
+cudaError_t run_bwd16(const Plan& p, cudaStream_t s, int v0, int s0) {
+  auto kern = k_leg_bwd16<NV, NS>;
+  const size_t smem = Bwd16Geo<NV, NS>::SMEM;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  const long long nblk = (long long)(p.L + 1) * (p.nh_pad / kThBlk) * ((win_nrb(p) + 1) / 2);
+  if (nblk <= 0) return cudaSuccess;
+  kern<<<(unsigned)nblk, kThreads, smem, s>>>(p, v0, s0);
+  return cudaGetLastError();
+}
+
+// Field groups of the stored-table kernels: two vectors while more than three
+// are left, then the rest with the scalars; fn(nv, ns, v0) launches one group.
+template <typename F>
+cudaError_t for_groups(int nvec, int nscl, F fn) {
+  cudaError_t e = cudaSuccess;
+  int v0 = 0;
+  do {
+    const int nv = nvec - v0 <= 3 ? nvec - v0 : 2;
+    e = fn(nv, v0 + nv == nvec ? nscl : 0, v0);
+    v0 += nv;
+  } while (e == cudaSuccess && v0 < nvec);
+  return e;
+}
+#define KMHD_GROUP(NVv, NSv, FN, ...)             \
+  switch ((NVv)*3 + (NSv)) {                      \
+    case 1: return FN<0, 1>(__VA_ARGS__);         \
+    case 2: return FN<0, 2>(__VA_ARGS__);         \
+    case 3: return FN<1, 0>(__VA_ARGS__);         \
+    case 4: return FN<1, 1>(__VA_ARGS__);         \
+    case 5: return FN<1, 2>(__VA_ARGS__);         \
+    case 6: return FN<2, 0>(__VA_ARGS__);         \
+    case 7: return FN<2, 1>(__VA_ARGS__);         \
+    case 8: return FN<2, 2>(__VA_ARGS__);         \
+    case 9: return FN<3, 0>(__VA_ARGS__);         \
+    case 10: return FN<3, 1>(__VA_ARGS__);        \
+    case 11: return FN<3, 2>(__VA_ARGS__);        \
+    default: return cudaErrorInvalidValue;        \
+  }
+cudaError_t run_bwd16(const Plan& p, cudaStream_t s) {
+  return for_groups(p.nvb, p.nsb, [&](int nv, int ns, int v0) -> cudaError_t { KMHD_GROUP(nv, ns, run_bwd16, p, s, v0, 0); });
+}
+
+cudaError_t run_fwd16(const Plan& p, double* d_rj, long long ld, const int* cols, cudaStream_t s, int m_count) {
+  return for_groups(p.nvf, p.nsf, [&](int nv, int ns, int v0) -> cudaError_t {
+    KMHD_GROUP(nv, ns, run_fwd16, p, d_rj, ld, cols, s, m_count, v0, 0);
+  });
 }
 
 template <int NV, int NS, bool OTF>
@@ -699,12 +1160,24 @@ cudaError_t launch_pack_b(const Plan& p, int nlc_max, const double* d_rj, long l
 }
 
 cudaError_t launch_leg_bwd_f64(const Plan& p, cudaStream_t s) {
+  // The 16-latitude kernel takes a whole SM per CTA: it wins when there are
+  // enough CTAs and at least two vectors to share a chunk's operands.  ms old ->
+  // new: L = 255, Nr = 129 3.19 -> 2.64; L = 511, Nr = 17 3.24 -> 2.91; L = 127,
+  // Nr = 17 (768 CTAs) 0.109 -> 0.092; but L = 31, Nr = 33 (160) 0.016 -> 0.019,
+  // L = 63, Nr = 9 (128) 0.018 -> 0.020, one vector at L = 255, Nr = 33 0.309 -> 0.322.
+  const long long ctas = (long long)(p.L + 1) * (p.nh_pad / kThBlk) * ((win_nrb(p) + 1) / 2);
+  if (!p.otf && p.nvb >= 2 && ctas >= 2 * 148) return run_bwd16(p, s);
   KMHD_DISPATCH(p.nvb, p.nsb, run_bwd, p, s);
 }
 
 cudaError_t launch_leg_fwd_f64(const Plan& p, double* d_rj, long long ld, const int* cols,
                                cudaStream_t s, int m_count) {
   if (m_count <= 0 || m_count > p.L + 1) m_count = p.L + 1;
+  // 64 degrees per parity and a whole SM per CTA: for truncations that fill them
+  // and launches with several CTAs per SM (not the few orders of the split
+  // tiers' dipole modes).  FWDMEAS
+  const long long ctas = (long long)((kcount(p.L, 0, 0) + kLB16 - 1) / kLB16) * win_nrb(p) * m_count;
+  if (!p.otf && p.L >= 128 && ctas >= 4 * 148) return run_fwd16(p, d_rj, ld, cols, s, m_count);
   KMHD_DISPATCH(p.nvf, p.nsf, run_fwd, p, d_rj, ld, cols, s, m_count);
 }
 

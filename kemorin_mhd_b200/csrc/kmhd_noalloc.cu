@@ -66,17 +66,6 @@ struct Carve {
   }
 };
 
-bool na_factor(int n, std::vector<int>& f) {
-  f.clear();
-  int r = n;
-  while (r % 8 == 0) { f.push_back(8); r /= 8; }
-  while (r % 4 == 0) { f.push_back(4); r /= 4; }
-  while (r % 2 == 0) { f.push_back(2); r /= 2; }
-  while (r % 3 == 0) { f.push_back(3); r /= 3; }
-  while (r % 5 == 0) { f.push_back(5); r /= 5; }
-  return r == 1 && (int)f.size() <= kMaxFftFactors;
-}
-
 // Same acceptance rules as kmhd_sph_create for the FP64 tier.
 int na_validate(const kmhd_sph_desc* d) {
   if (!d) return KMHD_ERR_ARG;
@@ -112,7 +101,7 @@ int na_validate(const kmhd_sph_desc* d) {
   }
   if (nv != d->nvector_f || ns != d->nscalar_f) return KMHD_ERR_ARG;
   std::vector<int> f;
-  if (!na_factor(d->nph, f)) return KMHD_ERR_SIZE;
+  if (!fft_factors(d->nph, f)) return KMHD_ERR_SIZE;
   const int ncb = 3 * d->nvector_b + d->nscalar_b, ncf = 3 * d->nvector_f + d->nscalar_f;
   const int npair = (std::max(ncb, ncf) + 1) / 2;
   if (sizeof(double2) * (size_t)npair * d->nph + sizeof(double) * 2 * (size_t)(d->ltr + 1) * ncb > 227 * 1024)
@@ -167,10 +156,8 @@ int na_plan(const kmhd_sph_desc* d, Plan& p, NaHost& H) {
     }
   H.nP = (size_t)po;
   H.nSB = (size_t)so;
-  H.nrtm_b = (size_t)(L + 1) * p.nth * p.nr * p.ncb * 2;
-  H.nrtm_f = (size_t)(L + 1) * p.nth * p.nr * p.ncf * 2;
   std::vector<int> fac;
-  na_factor(p.nph, fac);
+  fft_factors(p.nph, fac);
   p.nfac = (int)fac.size();
   for (int i = 0; i < p.nfac; ++i) p.fac[i] = fac[i];
   p.nprod = 0;
@@ -241,9 +228,11 @@ struct NaBufs {
   double2* twid;
 };
 
-size_t na_layout(const Plan& p, const NaHost& H, unsigned char* base, NaBufs& b) {
+size_t na_layout(const Plan& p, NaHost& H, unsigned char* base, NaBufs& b) {
   Carve c{base};
   const int L = p.L;
+  H.nrtm_b = rtm_size(p, p.ncb);
+  H.nrtm_f = rtm_size(p, p.ncf);
   b.radius = c.take<double>(p.nr);
   b.colat = c.take<double>(p.nth);
   b.weight = c.take<double>(p.nth);
@@ -282,6 +271,10 @@ extern "C" int kmhd_sph_cycle_noalloc(const kmhd_sph_desc* desc, const double* d
   for (int f = 0; f < p.nvf + p.nsf; ++f)
     if (cols_f[f] < 0) return KMHD_ERR_ARG;
   NaBufs b;
+  // eight orders per rtm block pad the orders to a multiple of eight: where
+  // that does not fit, smaller blocks (one order per block pads nothing)
+  p.mbs = kRtmShift;
+  while (p.mbs > 0 && na_layout(p, H, nullptr, b) > kNoAllocBytes) --p.mbs;
   if (na_layout(p, H, nullptr, b) > kNoAllocBytes) return KMHD_ERR_SIZE;  // work area too small
   if ((st = na_tables(desc, p, H)) != KMHD_OK) return st;
 

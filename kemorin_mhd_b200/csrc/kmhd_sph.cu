@@ -135,17 +135,6 @@ int dalloc(kmhd_sph* h, T** p, size_t n) {
   return KMHD_OK;
 }
 
-bool factor_fft(int n, std::vector<int>& f) {
-  f.clear();
-  int r = n;
-  while (r % 8 == 0 && r / 8 >= 1) { f.push_back(8); r /= 8; }
-  while (r % 4 == 0) { f.push_back(4); r /= 4; }
-  while (r % 2 == 0) { f.push_back(2); r /= 2; }
-  while (r % 3 == 0) { f.push_back(3); r /= 3; }
-  while (r % 5 == 0) { f.push_back(5); r /= 5; }
-  return r == 1 && (int)f.size() <= kMaxFftFactors;
-}
-
 int validate(const kmhd_sph_desc* d) {
   if (!d) return KMHD_ERR_ARG;
   if (d->ltr < 1 || d->nth < 2 || d->nr < 1 || d->nph < 4) return KMHD_ERR_SIZE;
@@ -183,7 +172,7 @@ int validate(const kmhd_sph_desc* d) {
   }
   if (d->nproduct > 0 && (nv != d->nvector_f || ns != d->nscalar_f)) return KMHD_ERR_ARG;
   std::vector<int> f;
-  if (!factor_fft(d->nph, f)) return KMHD_ERR_SIZE;
+  if (!fft_factors(d->nph, f)) return KMHD_ERR_SIZE;
   // one (r, theta) line of one component pair plus the staged spectra of the
   // line must fit in shared memory (wide lines go through the FFT pair by pair)
   const int ncb = 3 * d->nvector_b + d->nscalar_b;
@@ -316,6 +305,7 @@ int kmhd_sph_create(const kmhd_sph_desc* d, kmhd_sph** out) {
   p.nrb = p.nr4 / kRB;
   p.r_lo = 0;
   p.r_hi = p.nr;
+  p.mbs = kRtmShift;
   p.J = (long long)(p.L + 1) * (p.L + 1);
   p.nvb = d->nvector_b;
   p.nsb = d->nscalar_b;
@@ -369,7 +359,7 @@ int kmhd_sph_create(const kmhd_sph_desc* d, kmhd_sph** out) {
   }
   // FFT factors, twiddles e^{+2 pi i k/N}, digit reversal of the DIF output
   std::vector<int> fac;
-  factor_fft(p.nph, fac);
+  fft_factors(p.nph, fac);
   p.nfac = (int)fac.size();
   for (int i = 0; i < p.nfac; ++i) p.fac[i] = fac[i];
   std::vector<double2> tw(p.nph);
@@ -410,8 +400,7 @@ int kmhd_sph_create(const kmhd_sph_desc* d, kmhd_sph** out) {
   // ---- device allocations
   const size_t nP = (size_t)po, nSB = (size_t)so;
   const bool otf = (d->flags & KMHD_FLAG_P_ON_THE_FLY) != 0;
-  const size_t nrtm_b = (size_t)(L + 1) * p.nth * p.nr * p.ncb * 2;
-  const size_t nrtm_f = (size_t)(L + 1) * p.nth * p.nr * std::max(p.ncf, 1) * 2;
+  const size_t nrtm_b = rtm_size(p, p.ncb), nrtm_f = rtm_size(p, std::max(p.ncf, 1));
   const size_t nrj = (size_t)p.J * p.nr;
   const size_t nnod = (size_t)p.nr * p.nth * p.nph;
   if ((st = dalloc(h, &h->radius, p.nr)) || (st = dalloc(h, &h->colat, p.nth)) ||

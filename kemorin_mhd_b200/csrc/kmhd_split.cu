@@ -126,11 +126,6 @@ __device__ __forceinline__ double pow2(int e) {
   return __longlong_as_double((long long)(e + 1023) << 52);
 }
 
-// 32-byte global load (sm_100 256-bit ld.global, read-only path); p must be 32-byte aligned
-__device__ __forceinline__ void ld_global_v4(const double* p, double& a, double& b, double& c, double& d) {
-  asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];\n" : "=d"(a), "=d"(b), "=d"(c), "=d"(d) : "l"(p));
-}
-
 // frexp-style exponent: smallest e with |x| < 2^e (x > 0)
 __device__ __forceinline__ int exp_above(double x) {
   int e;
@@ -338,8 +333,8 @@ __device__ __forceinline__ void digits4(const double (&v)[4], uint32_t (&w)[NS])
 // Slicer: one CTA per (field group z, radius r, order m).  Backward groups:
 // z < nvb is vector z (types 0/1 from its theta/phi components); z = nvb is
 // the radial components and scalars (types 2/3).  Forward groups: z = 0 is the
-// radial components and scalars (types 4/5, record words [4 nvf, rec));
-// z = 1 + v is vector v (types 6/7, record words [4v, 4v + 4)).
+// radial components and scalars (types 4/5, record pairs nvf, nvf + 1, ...);
+// z = 1 + v is vector v (types 6/7, record pair v).
 //
 // Pass 1 builds the group's derived columns X[col][k] = B[k][col] 2^-dexp[k]
 // in shared memory, one thread per theta row (forward) or degree l
@@ -350,8 +345,12 @@ template <bool FWD, int NS>
 __global__ void __launch_bounds__(kSliceThreads) k_slice_mr(Plan P, SliceTabs S, const double* __restrict__ d_rj, long long ld,
                                                    const int* __restrict__ cols) {
   extern __shared__ double X[];
-  const int z = blockIdx.x, r = P.r_lo + blockIdx.y, m = blockIdx.z;
+  // forward, the orders of one rtm block are neighbours in the grid: their CTAs
+  // read the same 256-byte pieces of the records
+  const int z = FWD ? blockIdx.x >> kRtmShift : blockIdx.x, r = P.r_lo + blockIdx.y;
+  const int m = FWD ? (blockIdx.z << kRtmShift) | (blockIdx.x & ((1 << kRtmShift) - 1)) : blockIdx.z;
   const int L = P.L;
+  if (m > L) return;
   const int Kall = L - m + 1;
   const int nv = FWD ? P.nvf : P.nvb;
   const int nF = FWD ? P.nvf + P.nsf : P.nvb + P.nsb;
@@ -379,22 +378,21 @@ __global__ void __launch_bounds__(kSliceThreads) k_slice_mr(Plan P, SliceTabs S,
 
   // ---- pass 1: derived columns
   if (FWD) {
-    const int rec = 2 * P.ncf;
-    const long long strideTh = rec;  // records of one (m, r) are contiguous over theta
-    const double* base = P.rtm_f + rtm_off(P, m, 0, r, P.ncf) + (vgrp ? 4 * v : 4 * nv);
-    // 256-bit loads need 32-byte aligned records (an even forward component count)
-    const bool v4 = ((reinterpret_cast<uintptr_t>(P.rtm_f) | (uintptr_t)(16 * P.ncf)) & 31) == 0;
+    const long long strideTh = rtm_row(P, P.ncf);
+    const double* base = P.rtm_f + rtm_off(P, m, 0, r, P.ncf);
+    if (vgrp) base += rtm_pair(P, m, v, P.ncf);
     double2 nxt = make_double2(0.0, 0.0), sxt = nxt;  // second field of a 256-bit load
     // the thread's second row is loaded (vector groups) or its first sector
     // pair (radial / scalar group: fields 0 and 1) before the first row is
     // processed: twice the loads in flight
     const int th2 = threadIdx.x + blockDim.x;
-    const bool pre = v4 && th2 < P.nh && (vgrp || nF >= 2);
+    const bool pre = th2 < P.nh && (vgrp || nF >= 2);
+    const int o0 = vgrp ? 0 : rtm_pair(P, m, nv, P.ncf);  // the first sector read of a row
     double pn2[4] = {0.0, 0.0, 0.0, 0.0}, ps2[4] = {0.0, 0.0, 0.0, 0.0};
     if (pre) {
-      ld_global_v4(base + th2 * strideTh, pn2[0], pn2[1], pn2[2], pn2[3]);
+      ld_global_v4(base + th2 * strideTh + o0, pn2[0], pn2[1], pn2[2], pn2[3]);
       if (th2 < P.nth / 2)
-        ld_global_v4(base + (long long)(P.nth - 1 - th2) * strideTh, ps2[0], ps2[1], ps2[2], ps2[3]);
+        ld_global_v4(base + (long long)(P.nth - 1 - th2) * strideTh + o0, ps2[0], ps2[1], ps2[2], ps2[3]);
     }
     for (int th = threadIdx.x; th < P.nh; th += blockDim.x) {
       const bool hasS = th < P.nth / 2;
@@ -404,7 +402,7 @@ __global__ void __launch_bounds__(kSliceThreads) k_slice_mr(Plan P, SliceTabs S,
       const double sa = pow2(-__ldg(dxa + th)), sb = pow2(-__ldg(dxb + th));
       if (vgrp) {
         // words (theta slot 0, theta slot 1, phi slot 0, phi slot 1): one
-        // 32-byte sector per row, one 256-bit load when the records are aligned
+        // 32-byte sector per row, one 256-bit load
         double nn[4], ss[4] = {0.0, 0.0, 0.0, 0.0};
         if (pre && th == th2) {
 #pragma unroll
@@ -412,18 +410,9 @@ __global__ void __launch_bounds__(kSliceThreads) k_slice_mr(Plan P, SliceTabs S,
             nn[c] = pn2[c];
             ss[c] = ps2[c];
           }
-        } else if (v4) {
+        } else {
           ld_global_v4(pn, nn[0], nn[1], nn[2], nn[3]);
           if (hasS) ld_global_v4(ps, ss[0], ss[1], ss[2], ss[3]);
-        } else {
-          const double2 n01 = __ldg(reinterpret_cast<const double2*>(pn));
-          const double2 n23 = __ldg(reinterpret_cast<const double2*>(pn + 2));
-          nn[0] = n01.x; nn[1] = n01.y; nn[2] = n23.x; nn[3] = n23.y;
-          if (hasS) {
-            const double2 s01 = __ldg(reinterpret_cast<const double2*>(ps));
-            const double2 s23 = __ldg(reinterpret_cast<const double2*>(ps + 2));
-            ss[0] = s01.x; ss[1] = s01.y; ss[2] = s23.x; ss[3] = s23.y;
-          }
         }
         double sy[4], as[4];
 #pragma unroll
@@ -456,26 +445,28 @@ __global__ void __launch_bounds__(kSliceThreads) k_slice_mr(Plan P, SliceTabs S,
       } else {
         for (int f = 0; f < nF; ++f) {
           double2 nn, ss = make_double2(0.0, 0.0);
-          if (v4 && f + 1 < nF && !(f & 1)) {
-            // fields f, f + 1 in one 32-byte sector
+          if (f & 1) {
+            nn = nxt;
+            ss = sxt;
+          } else if (f + 1 < nF) {
+            // fields f, f + 1 are one record pair, one sector
+            const int o = rtm_pair(P, m, nv + (f >> 1), P.ncf);
             double4 a, b = make_double4(0.0, 0.0, 0.0, 0.0);
             if (pre && th == th2 && f == 0) {
               a = make_double4(pn2[0], pn2[1], pn2[2], pn2[3]);
               b = make_double4(ps2[0], ps2[1], ps2[2], ps2[3]);
             } else {
-              ld_global_v4(pn + 2 * f, a.x, a.y, a.z, a.w);
-              if (hasS) ld_global_v4(ps + 2 * f, b.x, b.y, b.z, b.w);
+              ld_global_v4(pn + o, a.x, a.y, a.z, a.w);
+              if (hasS) ld_global_v4(ps + o, b.x, b.y, b.z, b.w);
             }
             nn = make_double2(a.x, a.y);
             ss = make_double2(b.x, b.y);
             nxt = make_double2(a.z, a.w);
             sxt = make_double2(b.z, b.w);
-          } else if (v4 && (f & 1)) {
-            nn = nxt;
-            ss = sxt;
-          } else {
-            nn = __ldg(reinterpret_cast<const double2*>(pn + 2 * f));
-            if (hasS) ss = __ldg(reinterpret_cast<const double2*>(ps + 2 * f));
+          } else {  // odd count: the last pair holds one field
+            const int o = rtm_pair(P, m, nv + (f >> 1), P.ncf);
+            nn = __ldg(reinterpret_cast<const double2*>(pn + o));
+            if (hasS) ss = __ldg(reinterpret_cast<const double2*>(ps + o));
           }
           X[(4 * f + 0) * kst + th] = (nn.x + ss.x) * w * sa;
           X[(4 * f + 2) * kst + th] = hasS ? (nn.x - ss.x) * w * sb : 0.0;
@@ -730,11 +721,6 @@ constexpr double kBiasD = 6755399441055744.0;  // 1.5 2^52
 template <int NS>
 __host__ __device__ constexpr size_t gemm_stage_bytes() { return (size_t)NS * (kTM + kTN) * kTK; }
 
-// 32-byte global store (sm_100 256-bit st.global); p must be 32-byte aligned
-__device__ __forceinline__ void st_global_v4(double* p, double a, double b, double c, double d) {
-  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};\n" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
-}
-
 // Launch parameters: one instance (a), or a group of instances of one tier
 // whose pair units run in one persistent launch (GROUPED: unit u is pair
 // gunit[u].y of instance gunit[u].x, with that instance's arguments inst[.]).
@@ -902,8 +888,6 @@ __global__ void __launch_bounds__(kGemmWarps * 32, 1) k_split_gemm(const __grid_
       const GemmArgs& A = unit(u, base);
       const Plan& P = A.P;
       const SliceTabs& S = A.S;
-      // 32-byte stores into the rtm records need 32-byte aligned records
-      const bool v4ok = ((reinterpret_cast<uintptr_t>(P.rtm_b) | (uintptr_t)(P.ncb * 16)) & 31) == 0;
       for (int h = 0; h < per; ++h, ++it) {
         const Work w = A.work[base + h];
         const int nk = nk_of(P, w);
@@ -1055,7 +1039,7 @@ __global__ void __launch_bounds__(kGemmWarps * 32, 1) k_split_gemm(const __grid_
           if (th < P.nh && ok) {
             const bool pairrow = th < P.nth / 2;
             const double* sr = stash + row * kXS + cbase;
-            const long long rec = (long long)P.nth * P.ncb * 2;  // radius stride of the rtm records
+            const long long rec = (long long)P.nth * rtm_row(P, P.ncb);  // radius stride of the rtm records
             double* baseN = P.rtm_b + rtm_off(P, w.m, th, 0, P.ncb);
             double* baseS = P.rtm_b + rtm_off(P, w.m, P.nth - 1 - th, 0, P.ncb);
             if (w.t <= 1) {
@@ -1076,23 +1060,13 @@ __global__ void __launch_bounds__(kGemmWarps * 32, 1) k_split_gemm(const __grid_
                   n[q] = pairrow ? a[q] + val[c + q] : a[q];
                   s_[q] = a[q] - val[c + q];
                 }
-                double* dN = baseN + (long long)r * rec + 4 * vv;
-                double* dS = baseS + (long long)r * rec + 4 * vv;
-                if (v4ok) {
-                  st_global_v4(dN, n[0], n[1], n[2], n[3]);
-                  if (pairrow) st_global_v4(dS, s_[0], s_[1], s_[2], s_[3]);
-                } else {
-                  reinterpret_cast<double2*>(dN)[0] = make_double2(n[0], n[1]);
-                  reinterpret_cast<double2*>(dN)[1] = make_double2(n[2], n[3]);
-                  if (pairrow) {
-                    reinterpret_cast<double2*>(dS)[0] = make_double2(s_[0], s_[1]);
-                    reinterpret_cast<double2*>(dS)[1] = make_double2(s_[2], s_[3]);
-                  }
-                }
+                const long long o = (long long)r * rec + rtm_pair(P, w.m, vv, P.ncb);
+                st_global_v4(baseN + o, n[0], n[1], n[2], n[3]);
+                if (pairrow) st_global_v4(baseS + o, s_[0], s_[1], s_[2], s_[3]);
               }
             } else {
               // column c = 8 (block - 8 nt) + 2 (f % 4) + slot, block = (f / 4) nrR + r:
-              // radial components and scalars, record words 4 nvb + 2 f
+              // radial components and scalars, record pair nvb + f / 2
               const int nF = P.nvb + P.nsb;
               // nrR is a multiple of 8, so the tile's 8-column blocks share one field group
               const int rg0 = w.nt * (kTN / 8) + cbase / 8;
@@ -1101,8 +1075,6 @@ __global__ void __launch_bounds__(kGemmWarps * 32, 1) k_split_gemm(const __grid_
               for (int rr = 0; rr < kCols / 8; ++rr) {
                 const int r = r0 + rr;
                 if (r >= P.nr || 4 * fg >= nF) continue;
-                double* dN = baseN + (long long)r * rec + 4 * P.nvb + 8 * fg;
-                double* dS = baseS + (long long)r * rec + 4 * P.nvb + 8 * fg;
                 const int nFg = nF - 4 * fg;  // fields of this group (at most 4 used)
 #pragma unroll
                 for (int fp = 0; fp < 2; ++fp) {
@@ -1117,16 +1089,13 @@ __global__ void __launch_bounds__(kGemmWarps * 32, 1) k_split_gemm(const __grid_
                     n[q] = pairrow ? a[q] + val[c + q] : a[q];
                     s_[q] = a[q] - val[c + q];
                   }
-                  if (v4ok && 2 * fp + 1 < nFg) {
-                    st_global_v4(dN + 4 * fp, n[0], n[1], n[2], n[3]);
-                    if (pairrow) st_global_v4(dS + 4 * fp, s_[0], s_[1], s_[2], s_[3]);
-                  } else {
-                    reinterpret_cast<double2*>(dN + 4 * fp)[0] = make_double2(n[0], n[1]);
-                    if (pairrow) reinterpret_cast<double2*>(dS + 4 * fp)[0] = make_double2(s_[0], s_[1]);
-                    if (2 * fp + 1 < nFg) {
-                      reinterpret_cast<double2*>(dN + 4 * fp)[1] = make_double2(n[2], n[3]);
-                      if (pairrow) reinterpret_cast<double2*>(dS + 4 * fp)[1] = make_double2(s_[2], s_[3]);
-                    }
+                  const long long o = (long long)r * rec + rtm_pair(P, w.m, P.nvb + 2 * fg + fp, P.ncb);
+                  if (2 * fp + 1 < nFg) {
+                    st_global_v4(baseN + o, n[0], n[1], n[2], n[3]);
+                    if (pairrow) st_global_v4(baseS + o, s_[0], s_[1], s_[2], s_[3]);
+                  } else {  // odd count: the last pair holds one field
+                    *reinterpret_cast<double2*>(baseN + o) = make_double2(n[0], n[1]);
+                    if (pairrow) *reinterpret_cast<double2*>(baseS + o) = make_double2(s_[0], s_[1]);
                   }
                 }
               }
@@ -1278,17 +1247,19 @@ int split_create(SplitState** out, const Plan& p, int tier, int nslice, cudaStre
   // are adjacent in the list, start together on neighbouring CTAs and share
   // its chunks in L2.  A forward pair whose odd-parity type has one m-tile
   // fewer keeps that tile as an empty partner (no K chunks).
-  for (int m = 0; m <= L; ++m) {
+  // Backward, the orders of one rtm block alternate inside an n-tile: their
+  // sectors share 256-byte pieces of the records, so their stores meet in L2.
+  for (int m0 = 0; m0 <= L; m0 += 1 << p.mbs)
     for (int tp = 0; tp < 4; tp += 2) {
       if ((tp == 0 && p.nvb == 0)) continue;
-      const TypeGeo g = type_geo(tp, L, m, p.nh);
-      const int nn = S.npadT[tp] / kTN;
-      for (int nt = 0; nt < nn; ++nt)
-        for (int mt = 0; mt < g.rpad / kTM; ++mt) {
-          wb.push_back({m, tp, mt, nt});
-          wb.push_back({m, tp + 1, mt, nt});
-        }
+      for (int nt = 0; nt < S.npadT[tp] / kTN; ++nt)
+        for (int m = m0; m <= std::min(L, m0 + (1 << p.mbs) - 1); ++m)
+          for (int mt = 0; mt < type_geo(tp, L, m, p.nh).rpad / kTM; ++mt) {
+            wb.push_back({m, tp, mt, nt});
+            wb.push_back({m, tp + 1, mt, nt});
+          }
     }
+  for (int m = 0; m <= L; ++m) {
     for (int tp = 4; tp < 8; tp += 2) {
       if (tp == 6 && p.nvf == 0) continue;
       const TypeGeo g = type_geo(tp, L, m, p.nh);  // even parity: at least as many rows as odd
@@ -1449,7 +1420,8 @@ int split_slicer(SplitState* s, const Plan& p, bool fwd, const double* d_rj, lon
       cudaMemsetAsync(S.bnz, 0, 64 * (size_t)s->nbnz, st) != cudaSuccess)
     return KMHD_ERR_CUDA;
   if (p.r_hi > p.r_lo)
-    kern<<<dim3((fwd ? p.nvf : p.nvb) + 1, p.r_hi - p.r_lo, p.L + 1), kSliceThreads, smem, st>>>(p, S, d_rj, ld, cols);
+    kern<<<fwd ? dim3((p.nvf + 1) << kRtmShift, p.r_hi - p.r_lo, rtm_blocks(p)) : dim3(p.nvb + 1, p.r_hi - p.r_lo, p.L + 1),
+           kSliceThreads, smem, st>>>(p, S, d_rj, ld, cols);
   return cudaGetLastError() == cudaSuccess ? KMHD_OK : KMHD_ERR_CUDA;
 }
 
