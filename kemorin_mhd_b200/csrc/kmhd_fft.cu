@@ -182,9 +182,11 @@ __device__ __forceinline__ double2 spec_at(const Plan& P, const double* line, lo
   const bool mirror = k >= N - L, zero = k > L && !mirror;
   const int m = mirror ? N - k : zero ? 0 : k;
   const bool two = 2 * pp + 1 < nc;
-  const double* s = line + (m >> P.mbs) * bs + rtm_pair(P, m, pp, nc);
-  const double2 c0 = *reinterpret_cast<const double2*>(s);
-  double2 c1 = *reinterpret_cast<const double2*>(s + (two ? 2 : 0));
+  const double* s = line + (m >> P.mbs) * bs;
+  int ox, oy;
+  bwd_pair(P, m, pp, nc, bwd_in_order(P.nvb, P.nsb), ox, oy);
+  const double2 c0 = *reinterpret_cast<const double2*>(s + ox);
+  const double2 c1 = *reinterpret_cast<const double2*>(s + (two ? oy : ox));
   const double h = zero ? 0.0 : m == 0 ? 1.0 : 0.5;
   const double h1 = two ? h : 0.0, hs = m == 0 ? 0.0 : mirror ? -h : h, hs1 = m == 0 ? 0.0 : mirror ? -h1 : h1;
   // m = 0: (a_x, a_y); else x / 2 -+ i y / 2 of the two components
@@ -587,6 +589,12 @@ __device__ __forceinline__ void products(double2* z, int zs, int N, const Plan& 
 #pragma unroll
     for (int k = 0; k < MSB; ++k)
       if (k < nsb) sc[k] = *entry(nvb, nvb + k);
+    if (bwd_in_order(nvb, nsb)) {  // (r, theta), (phi, scalar)
+      const double2 w = z[pos];
+      rr[0] = w.x;
+      th[0] = w.y;
+      ph[0] = *entry(nvb, 0);
+    }
     if constexpr (PK > 0) point_products_k<PK>(rr, th, ph, sc, P, orr, oth, oph, os);
     else point_products<MVB, MSB, MVF, MSF, false>(rr, th, ph, sc, P, orr, oth, oph, os);
 #pragma unroll
@@ -729,8 +737,9 @@ __global__ void __launch_bounds__(kGridThreads, 2)
   dif_rest(Z, P);
   const long long nnod = (long long)P.nr * P.nth * N;
   const bool two = 2 * q + 1 < P.ncb;
-  double* f0 = fld + nnod * pair_comp(q, 0, P.nvb) + r0 + (long long)P.nr * th;
-  double* f1 = two ? fld + nnod * pair_comp(q, 1, P.nvb) + r0 + (long long)P.nr * th : nullptr;
+  const bool inorder = bwd_in_order(P.nvb, P.nsb);
+  double* f0 = fld + nnod * (inorder ? 2 * q : pair_comp(q, 0, P.nvb)) + r0 + (long long)P.nr * th;
+  double* f1 = two ? fld + nnod * (inorder ? 2 * q + 1 : pair_comp(q, 1, P.nvb)) + r0 + (long long)P.nr * th : nullptr;
   const long long ps = (long long)P.nr * P.nth;
 #pragma unroll 4
   for (int it = threadIdx.x; it < N << lrad; it += blockDim.x) {
@@ -852,8 +861,8 @@ struct DFT2F_ZM<3, B, SIGN> {
 // inputs (L < k < N - L) is zero and the outer thirds need no range checks.
 // line / bs: the line's block rows, staged or in place (see spec_at).
 template <int N, bool PR, bool INPLACE = false>
-__device__ __forceinline__ void ff_dif_first(const Plan& P, const double* line, long long bs, int nc, double2* z,
-                                             int npair, const double2* __restrict__ tw) {
+__device__ __forceinline__ void ff_dif_first(const Plan& P, const double* line, long long bs, int nc, bool inorder,
+                                             double2* z, int npair, const double2* __restrict__ tw) {
   constexpr int R = ff_first(N), S1 = N / R, NP = N + 1, T3 = R / 3;
   for (int it = threadIdx.x; it < npair * S1; it += blockDim.x) {
     const int pp = it / S1, j = it - pp * S1;
@@ -866,12 +875,16 @@ __device__ __forceinline__ void ff_dif_first(const Plan& P, const double* line, 
       // whole block rows apart.
       static_assert(S1 % kRtmOrders == 0, "orders per rtm block");
       const bool two = 2 * pp + 1 < nc;  // the pair holds two components
-      const int per = two ? 4 : 2;
-      const double* up = line + (j >> kRtmShift) * bs + pp * 4 * kRtmOrders + (j & (kRtmOrders - 1)) * per;
-      const double* dn = line + ((-j) >> kRtmShift) * bs + pp * 4 * kRtmOrders + ((-j) & (kRtmOrders - 1)) * per;
+      int ux, uy, dx, dy;
+      bwd_pair(P, j, pp, nc, inorder, ux, uy);
+      bwd_pair(P, -j, pp, nc, inorder, dx, dy);
+      const double* up = line + (j >> kRtmShift) * bs;
+      const double* dn = line + ((-j) >> kRtmShift) * bs;
       // staged sectors lie 32 bytes apart: lanes 4..7 of each eight read the
       // second half first, so a quarter warp covers all banks
-      const int hu = !INPLACE && two ? (j >> 1) & 2 : 0, hd = !INPLACE && two ? ((-j) >> 1) & 2 : 0;
+      const bool hu = !INPLACE && two && (j & 4), hd = !INPLACE && two && ((-j) & 4);
+      if (!two) uy = ux, dy = dx;
+      const int u0 = hu ? uy : ux, u1 = hu ? ux : uy, d0 = hd ? dy : dx, d1 = hd ? dx : dy;
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         if (r >= T3 && r < 2 * T3) {
@@ -884,10 +897,9 @@ __device__ __forceinline__ void ff_dif_first(const Plan& P, const double* line, 
           continue;
         }
         const double* s = mir ? dn + ((N - r * S1) / kRtmOrders) * bs : up + ((r * S1) / kRtmOrders) * bs;
-        const int h = mir ? hd : hu;
-        double2 c0 = *reinterpret_cast<const double2*>(s + h);
-        double2 c1 = two ? *reinterpret_cast<const double2*>(s + (2 - h)) : make_double2(0.0, 0.0);
-        if (!INPLACE && h) {
+        double2 c0 = *reinterpret_cast<const double2*>(s + (mir ? d0 : u0));
+        double2 c1 = two ? *reinterpret_cast<const double2*>(s + (mir ? d1 : u1)) : make_double2(0.0, 0.0);
+        if (!INPLACE && (mir ? hd : hu)) {
           const double2 t = c0;
           c0 = c1;
           c1 = t;
@@ -1075,11 +1087,17 @@ __device__ __forceinline__ void ff_fused(double2* z, const Plan& P) {
       double rr[VB] = {}, th[VB] = {}, ph[VB] = {}, sc[SB] = {};
       double orr[VF] = {}, oth[VF] = {}, oph[VF] = {}, os[SF] = {};
       auto lst = [&](int f) { return (f & 1) ? v[MVB + f / 2][r].y : v[MVB + f / 2][r].x; };
+      const bool inorder = EX ? bwd_in_order(MVB, MSB) : bwd_in_order(P.nvb, P.nsb);
 #pragma unroll
       for (int q = 0; q < MVB; ++q) {
         rr[q] = lst(q);
         th[q] = v[q][r].x;
         ph[q] = v[q][r].y;
+      }
+      if (MVB > 0 && MSB > 0 && inorder) {  // (r, theta), (phi, scalar)
+        rr[0] = v[0][r].x;
+        th[0] = v[0][r].y;
+        ph[0] = lst(0);
       }
 #pragma unroll
       for (int q = 0; q < MSB; ++q) {
@@ -1183,6 +1201,7 @@ __global__ void __launch_bounds__(NT, kFftThreadsF / NT)
   const int ncb = EX ? 3 * MVB + MSB : P.ncb, ncf = EX ? 3 * MVF + MSF : P.ncf;
   const int npb = (ncb + 1) / 2, npf = (ncf + 1) / 2;
   const int npair = npb > npf ? npb : npf;
+  const bool inorder = EX ? bwd_in_order(MVB, MSB) : bwd_in_order(P.nvb, P.nsb);
   double2* z = reinterpret_cast<double2*>(smraw);
   // staged spectra, 128-byte aligned, then the mbarrier
   double* st = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(z + npair * NP) + 127) & ~static_cast<uintptr_t>(127));
@@ -1208,8 +1227,8 @@ __global__ void __launch_bounds__(NT, kFftThreadsF / NT)
                          reinterpret_cast<uint64_t>(&tmap)),
                      "r"(0), "r"(next % P.nth), "r"(next / P.nth), "r"(0)
                      : "memory");
-      ff_dif_first<N, PR, true>(P, P.rtm_b + rtm_off(P, 0, th, r, ncb), (long long)P.nth * P.nr * row, ncb, z, npb,
-                                P.twid);
+      ff_dif_first<N, PR, true>(P, P.rtm_b + rtm_off(P, 0, th, r, ncb), (long long)P.nth * P.nr * row, ncb,
+                                inorder, z, npb, P.twid);
       __syncthreads();
       rest(th, r);
     }
@@ -1246,7 +1265,7 @@ __global__ void __launch_bounds__(NT, kFftThreadsF / NT)
       }
       return;
     }
-    ff_dif_first<N, PR>(P, st, row, ncb, z, npb, P.twid);
+    ff_dif_first<N, PR>(P, st, row, ncb, inorder, z, npb, P.twid);
     __syncthreads();
     const int next = line + gridDim.x;
     if (next < nlines) stage(next);
@@ -1268,8 +1287,8 @@ __global__ void __launch_bounds__(NT, kFftThreadsF / NT)
 // L = 1023, Nr = 17.  w_N^(h (j + r S1)) = w_N^(h j) w_48^r: the first factor is
 // common to a butterfly and goes into the twiddles, the second is compile-time.
 template <int NH, int H, bool PR>
-__device__ __forceinline__ void ff_half_first(const Plan& P, const double* line, long long bs, int nc, double2* z,
-                                              int npair) {
+__device__ __forceinline__ void ff_half_first(const Plan& P, const double* line, long long bs, int nc, bool inorder,
+                                              double2* z, int npair) {
   constexpr int R = ff_first(NH), S1 = NH / R, NP = NH + 1;
   static_assert(R == 24 && S1 == 64, "w_48 rotations, whole block rows");
   const int L = P.L;
@@ -1277,9 +1296,11 @@ __device__ __forceinline__ void ff_half_first(const Plan& P, const double* line,
   for (int it = threadIdx.x; it < npair * S1; it += blockDim.x) {
     const int pp = it / S1, j = it - pp * S1;
     const bool two = 2 * pp + 1 < nc;
-    const int per = two ? 4 : 2;
-    const double* up = line + (j >> kRtmShift) * bs + pp * 4 * kRtmOrders + (j & (kRtmOrders - 1)) * per;
-    const double* dn = line + ((-j) >> kRtmShift) * bs + pp * 4 * kRtmOrders + ((-j) & (kRtmOrders - 1)) * per;
+    int ux, uy, dx, dy;
+    bwd_pair(P, j, pp, nc, inorder, ux, uy);
+    bwd_pair(P, -j, pp, nc, inorder, dx, dy);
+    const double* up = line + (j >> kRtmShift) * bs;
+    const double* dn = line + ((-j) >> kRtmShift) * bs;
     const double2 zero = make_double2(0.0, 0.0);
     double2 x[R];
     auto input = [&](auto rc) {
@@ -1289,15 +1310,15 @@ __device__ __forceinline__ void ff_half_first(const Plan& P, const double* line,
       double2 u = zero, d = zero;
       if ((!PR || r < 2 * R / 3) && (PR || k <= L)) {
         const double* s = up + (r * S1 / kRtmOrders) * bs;
-        const double2 c0 = *reinterpret_cast<const double2*>(s);
-        const double2 c1 = two ? *reinterpret_cast<const double2*>(s + 2) : zero;
+        const double2 c0 = *reinterpret_cast<const double2*>(s + ux);
+        const double2 c1 = two ? *reinterpret_cast<const double2*>(s + uy) : zero;
         u = r == 0 && j == 0 ? make_double2(c0.x, c1.x)
                              : make_double2(0.5 * c0.x + 0.5 * c1.y, 0.5 * c1.x - 0.5 * c0.y);
       }
       if (PR ? r >= R / 3 && (r > R / 3 || j > 0) : NH - k <= L) {
         const double* s = dn + ((NH - r * S1) / kRtmOrders) * bs;
-        const double2 c0 = *reinterpret_cast<const double2*>(s);
-        const double2 c1 = two ? *reinterpret_cast<const double2*>(s + 2) : zero;
+        const double2 c0 = *reinterpret_cast<const double2*>(s + dx);
+        const double2 c1 = two ? *reinterpret_cast<const double2*>(s + dy) : zero;
         d = make_double2(0.5 * c0.x - 0.5 * c1.y, 0.5 * c0.y + 0.5 * c1.x);
       }
       x[r] = H == 0 ? cadd(u, d) : rot<48, r, +1>(csub(u, d));
@@ -1407,7 +1428,7 @@ __global__ void __launch_bounds__(kFftThreadsF, 1)
     double* dst = P.rtm_f + rtm_off(P, 0, th, r, ncf);
     auto half = [&](auto hc) {
       constexpr int H = decltype(hc)::value;
-      ff_half_first<NH, H, PR>(P, src, bsb, ncb, z, npb);
+      ff_half_first<NH, H, PR>(P, src, bsb, ncb, EX ? bwd_in_order(MVB, MSB) : bwd_in_order(P.nvb, P.nsb), z, npb);
       __syncthreads();
       ff_mid_pass<NH, +1, 2>(z, npb, P.twid);
       __syncthreads();

@@ -17,6 +17,7 @@ TOL = 1e-13  # FP64 tier against the oracle, max-norm per column
 HEAT = dict(nvb=1, nsb=1, nvf=1, nsf=0, products=((1, 0, 0, 1.0),))
 ODD = dict(nvb=2, nsb=2, nvf=2, nsf=2,  # 8 + 8 components, a list no kernel knows
            products=((0, 1, 0, 0.5), (1, 1, 1, 2.0), (2, 0, 1, 1.0), (3, 0, 1, -1.0)))
+ONE2 = dict(nvb=1, nsb=2, nvf=1, nsf=1, products=((1, 0, 1, 0.5), (3, 0, 1, 2.0)))  # components paired in order
 FIVE = dict(nvb=5, nsb=0, nvf=5, nsf=0,
             products=tuple((0, a, (a + 1) % 5, 1.0) for a in range(5)))
 
@@ -54,10 +55,10 @@ LINES = [(3, 6, 8), (7, 12, 16), (8, 13, 20), (9, 15, 40), (15, 24, 90), (16, 26
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("fields", ["default", "heat", "dynamo", "odd"])
+@pytest.mark.parametrize("fields", ["default", "heat", "dynamo", "odd", "one2"])
 @pytest.mark.parametrize("L,nth,nph", LINES)
 def test_cycle_lines(L, nth, nph, fields):
-    sets = dict(FIELD_SETS, heat=HEAT, odd=ODD)
+    sets = dict(FIELD_SETS, heat=HEAT, odd=ODD, one2=ONE2)
     assert run("cycle", SphConfig(L, nth, nph, 3, **sets[fields])) <= TOL
 
 
@@ -71,12 +72,12 @@ def test_cycle_specialised_odd_set(L, nph):
 
 # lines whose grid alone fits (in place), with sets of their own and without, and wide ones
 @pytest.mark.gpu
-@pytest.mark.parametrize("fields", ["dynamo", "full", "five", "odd"])
+@pytest.mark.parametrize("fields", ["dynamo", "full", "five", "odd", "heat", "one2"])
 @pytest.mark.parametrize("L,nph", [(40, 1536), (511, 1536), (60, 1440), (40, 3072)])
 def test_cycle_long_lines(L, nph, fields):
-    sets = dict(FIELD_SETS, odd=ODD, five=FIVE)
+    sets = dict(FIELD_SETS, odd=ODD, five=FIVE, heat=HEAT, one2=ONE2)
     nth = 64 if L < 100 else 96
-    if L == 511 and fields == "odd":
+    if L == 511 and fields in ("odd", "heat", "one2"):
         pytest.skip("staged: covered by the short lines")
     assert run("cycle", SphConfig(L, nth, nph, 3, **sets[fields])) <= TOL
 
@@ -104,9 +105,11 @@ def test_separable_radial_blocks(nr):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("kind", ["b_trans", "f_trans"])
+@pytest.mark.parametrize("fields", ["default", "heat", "one2"])
 @pytest.mark.parametrize("L,nth,nph,nr", [(31, 48, 96, 9), (20, 32, 3072, 5), (20, 32, 1536, 6), (20, 33, 450, 8)])
-def test_separable_lines(kind, L, nth, nph, nr):
-    assert run(kind, SphConfig(L, nth, nph, nr)) <= TOL
+def test_separable_lines(kind, L, nth, nph, nr, fields):
+    sets = dict(FIELD_SETS, heat=HEAT, one2=ONE2)
+    assert run(kind, SphConfig(L, nth, nph, nr, **sets[fields])) <= TOL
 
 
 @pytest.mark.gpu
@@ -148,3 +151,15 @@ def test_noalloc_smaller_record_blocks(fields, back):
     rc, cfg, d, out = call(nr - back)
     assert rc == 0
     assert col_relerr(from_dev_fortran(out), Oracle(cfg, nthreads=8).cycle(d)).max() <= TOL
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("L,nr,fields", [(130, 21, f) for f in ("heat", "convection", "default", "dynamo", "full", "five",
+                                                                "one2")] + [(160, 33, "default"), (255, 9, "default")])
+def test_fp64_sixteen_row_kernels(L, nr, fields):
+    """The FP64 Legendre kernels of large launches: truncations that end inside
+    their 16- and 64-degree blocks, latitudes inside a block of 16 (odd: an equator
+    row), odd radial block counts, every field group."""
+    conv = dict(nvb=2, nsb=1, nvf=2, nsf=1, products=((0, 1, 0, 1.0), (1, 0, 0, 1.0), (2, 0, 1, 1.0)))
+    sets = dict(FIELD_SETS, heat=HEAT, convection=conv, five=FIVE, one2=ONE2)
+    assert run("cycle", SphConfig(L, 3 * (L + 1) // 2 + 1, 3 * (L + 1) if L == 255 else 480, nr, **sets[fields])) <= TOL
