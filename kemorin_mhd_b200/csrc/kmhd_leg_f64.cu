@@ -43,67 +43,54 @@ struct BwdGeo {
 };
 
 // ---------------------------------------------------------------------------
-// d_rj -> SB packing.  CTA = (m, 32-wide l chunk, r block); both parities.
-__global__ void k_pack_b(Plan p, const double* __restrict__ d_rj, long long ld,
-                         const int* __restrict__ cols, int nv, int ns, int CB) {
+// d_rj -> SB packing.  CTA = (m, 32-wide l chunk, r block); both parities.  Warp
+// (slot, radius u), lane = degree: the loads of every column go out together,
+// the scaled values meet in shared memory and leave as whole SB rows.
+// One item per thread in turn, with run-time divisions and a dependent chain of
+// loads each, took 0.478 ms at L = 511, Nr = 17 where this takes 0.153.
+template <int NV, int NS>
+__global__ void __launch_bounds__(kThreads) k_pack_b(const __grid_constant__ Plan p, const double* __restrict__ d_rj,
+                                                     long long ld, const int* __restrict__ cols) {
+  constexpr int CB = 24 * NV + 8 * NS, ST = CB + 1;  // odd row stride: lanes (degrees) in different banks
   extern __shared__ double sm[];
   const int m = blockIdx.y;
-  const int nlc = p.kpad[2 * m] / kKC;  // chunks of 32 l (16 k per parity)
   const int nrbw = win_nrb(p);
   const int lc = blockIdx.x / nrbw;
   const int rb = win_rb0(p) + blockIdx.x % nrbw;
-  if (lc >= nlc) return;
-  const int nc = 3 * nv + ns;
+  if (lc >= p.kpad[2 * m] / kKC) return;  // chunks of 32 l (16 k per parity)
   const int L = p.L;
-  // smem tile [slot][u][q][32]
-  const int nitems = 2 * kRB * nc * 32;
-  for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
-    const int lo = it & 31;
-    int rest = it >> 5;
-    const int q = rest % nc;
-    rest /= nc;
-    const int u = rest % kRB;
-    const int slot = rest / kRB;
-    const int l = m + 32 * lc + lo;
-    const int r = kRB * rb + u;
-    double v = 0.0;
-    if (l <= L && r < p.nr && (slot == 0 || m > 0)) {
-      const int j = p.jmap[((long long)m * 2 + slot) * (L + 1) + l];
-      const int col = q < 3 * nv ? cols[q / 3] + q % 3 : cols[nv + (q - 3 * nv)];
-      v = d_rj[(long long)j + p.J * r + ld * col];
-    }
-    sm[it] = v;
+  const int warp = threadIdx.x >> 5, lo = threadIdx.x & 31;
+  static_assert(kWarps == 2 * kRB, "one warp per slot and radius");
+  const int slot = warp / kRB, u = warp % kRB;
+  const int l = m + 32 * lc + lo, r = kRB * rb + u;
+  const bool ok = l <= L && r < p.nr && (slot == 0 || m > 0);
+  const double* src = d_rj + (ok ? p.jmap[((long long)m * 2 + slot) * (L + 1) + l] + p.J * r : 0);
+  double x[NV > 0 ? NV : 1][3], xs[NS > 0 ? NS : 1];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    const double* c = src + ld * __ldg(cols + v);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) x[v][q] = ok ? __ldg(c + q * ld) : 0.0;
   }
+#pragma unroll
+  for (int s = 0; s < NS; ++s) xs[s] = ok ? __ldg(src + ld * __ldg(cols + NV + s)) : 0.0;
+  const double ar = r < p.nr ? 1.0 / p.radius[r] : 0.0;
+  double* row = sm + lo * ST + 2 * u + slot;
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    row[24 * v] = x[v][1] * ar;                        // dpoldt = dS/dr / r
+    row[24 * v + 8] = x[v][2] * ar;                    // dtordt = T / r
+    row[24 * v + 16] = x[v][0] * (ar * ar) * g3_of(l);  // pol = S / r^2 * g3
+  }
+#pragma unroll
+  for (int s = 0; s < NS; ++s) row[24 * NV + 8 * s] = xs[s];
   __syncthreads();
-  const int nout = 2 * kKC * CB;
-  for (int it = threadIdx.x; it < nout; it += blockDim.x) {
-    const int c = it % CB;
-    const int rest = it / CB;
-    const int kk = rest % kKC;
-    const int par = rest / kKC;
-    const int k = kKC * lc + kk;
-    if (k >= p.kpad[2 * m + par]) continue;
-    const int lo = 2 * kk + par;
-    const int l = m + 32 * lc + lo;
-    double v;
-    int u, slot;
-    if (c < 24 * nv) {
-      const int vv = c / 24, t = c % 24, tile = t / 8, w = t % 8;
-      u = w >> 1;
-      slot = w & 1;
-      const int r = kRB * rb + u;
-      const double ar = r < p.nr ? 1.0 / p.radius[r] : 0.0;
-      const double* s = sm + ((slot * kRB + u) * nc) * 32;
-      if (tile == 0) v = s[(3 * vv + 1) * 32 + lo] * ar;                   // dpoldt = dS/dr / r
-      else if (tile == 1) v = s[(3 * vv + 2) * 32 + lo] * ar;              // dtordt = T / r
-      else v = s[(3 * vv + 0) * 32 + lo] * (ar * ar) * g3_of(l);            // pol = S / r^2 * g3
-    } else {
-      const int cc = c - 24 * nv, ss = cc / 8, w = cc % 8;
-      u = w >> 1;
-      slot = w & 1;
-      v = sm[((slot * kRB + u) * nc + 3 * nv + ss) * 32 + lo];
-    }
-    p.SB[p.sboff[2 * m + par] + (long long)k * (p.nrb * CB) + rb * CB + c] = v;
+#pragma unroll 5
+  for (int it = threadIdx.x; it < 32 * CB; it += kThreads) {
+    const int ll = it / CB, c = it - ll * CB;
+    const int par = ll & 1, k = kKC * lc + (ll >> 1);
+    if (k < p.kpad[2 * m + par])
+      p.SB[p.sboff[2 * m + par] + (long long)k * (p.nrb * CB) + rb * CB + c] = sm[ll * ST + c];
   }
 }
 
@@ -1123,6 +1110,14 @@ cudaError_t run_fwd(const Plan& p, double* d_rj, long long ld, const int* cols, 
                : run_fwd_t<NV, NS, false>(p, d_rj, ld, cols, s, m_count);
 }
 
+template <int NV, int NS>
+cudaError_t run_pack(const Plan& p, int nlc_max, const double* d_rj, long long ld, const int* cols, cudaStream_t s) {
+  if (win_nrb(p) <= 0) return cudaSuccess;
+  constexpr size_t smem = sizeof(double) * 32 * (24 * NV + 8 * NS + 1);  // at most 35 KB
+  k_pack_b<NV, NS><<<dim3(nlc_max * win_nrb(p), p.L + 1), kThreads, smem, s>>>(p, d_rj, ld, cols);
+  return cudaGetLastError();
+}
+
 #define KMHD_DISPATCH(NVv, NSv, FN, ...)                                   \
   switch (NVv * 3 + NSv) {                                                 \
     case 1: return FN<0, 1>(__VA_ARGS__);                                  \
@@ -1149,14 +1144,7 @@ cudaError_t run_fwd(const Plan& p, double* d_rj, long long ld, const int* cols, 
 
 cudaError_t launch_pack_b(const Plan& p, int nlc_max, const double* d_rj, long long ld,
                                const int* cols, int nv, int ns, cudaStream_t s) {
-  const int nc = 3 * nv + ns;
-  const int CB = 24 * nv + 8 * ns;
-  const size_t smem = sizeof(double) * 2 * kRB * nc * 32;
-  cudaFuncSetAttribute(k_pack_b, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (win_nrb(p) <= 0) return cudaSuccess;
-  dim3 grid(nlc_max * win_nrb(p), p.L + 1);
-  k_pack_b<<<grid, kThreads, smem, s>>>(p, d_rj, ld, cols, nv, ns, CB);
-  return cudaGetLastError();
+  KMHD_DISPATCH(nv, ns, run_pack, p, nlc_max, d_rj, ld, cols, s);
 }
 
 cudaError_t launch_leg_bwd_f64(const Plan& p, cudaStream_t s) {
@@ -1175,7 +1163,9 @@ cudaError_t launch_leg_fwd_f64(const Plan& p, double* d_rj, long long ld, const 
   if (m_count <= 0 || m_count > p.L + 1) m_count = p.L + 1;
   // 64 degrees per parity and a whole SM per CTA: for truncations that fill them
   // and launches with several CTAs per SM (not the few orders of the split
-  // tiers' dipole modes).  FWDMEAS
+  // tiers' dipole modes).  ms 32-degree kernel -> this one: L = 255, Nr = 129 3.94 ->
+  // 3.62; L = 511, Nr = 17 4.00 -> 3.61; L = 1023, Nr = 17 29.0 -> 25.9; but L = 106,
+  // Nr = 47 0.252 -> 0.259, L = 31, Nr = 33 0.031 -> 0.043 (most warps without a degree).
   const long long ctas = (long long)((kcount(p.L, 0, 0) + kLB16 - 1) / kLB16) * win_nrb(p) * m_count;
   if (!p.otf && p.L >= 128 && ctas >= 4 * 148) return run_fwd16(p, d_rj, ld, cols, s, m_count);
   KMHD_DISPATCH(p.nvf, p.nsf, run_fwd, p, d_rj, ld, cols, s, m_count);
