@@ -340,7 +340,7 @@ __device__ __forceinline__ void digits4(const double (&v)[4], uint32_t (&w)[NS])
 // in shared memory, one thread per theta row (forward) or degree l
 // (backward), with the sym/asym combination, weights and factors of each
 // column written out explicitly (the same algebra as the FP64 tier's operand
-// loaders).  Pass 2 takes the column maxima, pass 3 cuts the digits.
+// loaders) and takes the column maxima, pass 3 cuts the digits.
 template <bool FWD, int NS>
 __global__ void __launch_bounds__(kSliceThreads) k_slice_mr(Plan P, SliceTabs S, const double* __restrict__ d_rj, long long ld,
                                                    const int* __restrict__ cols) {
@@ -368,12 +368,17 @@ __global__ void __launch_bounds__(kSliceThreads) k_slice_mr(Plan P, SliceTabs S,
   const int* dxa = S.dexp + S.deoff[m * kNT + t0];
   const int* dxb = S.dexp + S.deoff[m * kNT + t0 + 1];
   const int nx = ncolg * kst;
+  // column maxima: the high word of |x| (ordered like x), 0 for an all-zero column
+  int* colmax = reinterpret_cast<int*>(X + ((nx + 1) & ~1));
+  if (threadIdx.x < kGrpCols) colmax[threadIdx.x] = 0;
+  auto hiword = [](double x) { return __double2hiint(x) & 0x7fffffff; };
+  int mx[8] = {};  // vector groups: this thread's maxima of the eight columns
   // Forward with m > 0 and no theta padding, pass 1 writes every X entry
   // (both parts of the vector types, both slots of every field)
   if (!(FWD && m > 0 && P.nh % kTK == 0)) {
     for (int i = threadIdx.x; i < nx; i += blockDim.x) X[i] = 0.0;
-    __syncthreads();
   }
+  __syncthreads();
   const double ar = 1.0 / P.radius[r];
 
   // ---- pass 1: derived columns
@@ -429,17 +434,21 @@ __global__ void __launch_bounds__(kSliceThreads) k_slice_mr(Plan P, SliceTabs S,
           const TypeGeo& g = p ? gb : ga;
           const double s0 = p ? sb : sa;
           double* x = X + (4 * p) * kst;
-          x[0 * kst + th] = A0[0] * s0;
-          x[1 * kst + th] = A0[1] * s0;
-          x[2 * kst + th] = -A0[2] * s0;
-          x[3 * kst + th] = -A0[3] * s0;
+          auto put = [&](int q, int k, double v) {
+            x[q * kst + k] = v;
+            mx[4 * p + q] = max(mx[4 * p + q], hiword(v));
+          };
+          put(0, th, A0[0] * s0);
+          put(1, th, A0[1] * s0);
+          put(2, th, -A0[2] * s0);
+          put(3, th, -A0[3] * s0);
           if (m > 0) {
             const int k1 = g.kpart0 + th;
             const double s1 = pow2(-__ldg((p ? dxb : dxa) + k1)) * ai;
-            x[0 * kst + k1] = -A1[3] * s1;
-            x[1 * kst + k1] = A1[2] * s1;
-            x[2 * kst + k1] = -A1[1] * s1;
-            x[3 * kst + k1] = A1[0] * s1;
+            put(0, k1, -A1[3] * s1);
+            put(1, k1, A1[2] * s1);
+            put(2, k1, -A1[1] * s1);
+            put(3, k1, A1[0] * s1);
           }
         }
       } else {
@@ -497,16 +506,12 @@ __global__ void __launch_bounds__(kSliceThreads) k_slice_mr(Plan P, SliceTabs S,
           const int k = (part1 ? g.kpart0 : 0) + kk;
           const double sc = pow2(-__ldg((t ? dxb : dxa) + k));
           double* x = X + (4 * t) * kst + k;
-          if (!part1) {
-            x[0 * kst] = x10 * sc;
-            x[1 * kst] = x11 * sc;
-            x[2 * kst] = -x20 * sc;
-            x[3 * kst] = -x21 * sc;
-          } else {
-            x[0 * kst] = x21 * sc;
-            x[1 * kst] = -x20 * sc;
-            x[2 * kst] = x11 * sc;
-            x[3 * kst] = -x10 * sc;
+          const double y[4] = {(part1 ? x21 : x10) * sc, (part1 ? -x20 : x11) * sc, (part1 ? x11 : -x20) * sc,
+                               (part1 ? -x10 : -x21) * sc};
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            x[q * kst] = y[q];
+            mx[4 * t + q] = max(mx[4 * t + q], hiword(y[q]));
           }
         }
       } else {
@@ -522,31 +527,39 @@ __global__ void __launch_bounds__(kSliceThreads) k_slice_mr(Plan P, SliceTabs S,
       }
     }
   }
-  __syncthreads();
-
-  double* colmax = X + ((nx + 1) & ~1);
-  int* colexp = reinterpret_cast<int*>(colmax + kGrpCols);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nw = blockDim.x >> 5;
-  // ---- pass 2: column maxima
-  for (int c = warp; c < ncolg; c += nw) {
-    const int t = ctype(c);
-    const int kp = (t == t0) ? ga.kpad : gb.kpad;
-    double mx = 0.0;
-    for (int k = 2 * lane; k < kp; k += 64) {
-      const double2 x2 = *reinterpret_cast<const double2*>(X + c * kst + k);
-      mx = fmax(mx, fmax(fabs(x2.x), fabs(x2.y)));
-    }
-    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) {
-      const int e = mx > 0.0 ? exp_above(mx) : 0;
-      colmax[c] = mx;
-      colexp[c] = e;
-      const ColRef cr = FWD ? colref_fwd(P, S, r, i0 + c) : colref_bwd(P, S, r, i0 + c);
-      S.bexp[S.beoff[m * kNT + t] + cr.col] = e - (8 * NS - 2);
+  // ---- column maxima: of a vector group from the registers (one warp maximum
+  // and one shared atomic per column; a second sweep over X took 15 to 22% of a
+  // CTA's time), of the radial / scalar group from X
+  if (vgrp) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const int w = (int)__reduce_max_sync(0xffffffffu, (unsigned)mx[c]);
+      if (lane == 0) atomicMax(colmax + c, w);
     }
   }
   __syncthreads();
+  if (!vgrp) {
+    for (int c = warp; c < ncolg; c += nw) {
+      const int kp = ctype(c) == t0 ? ga.kpad : gb.kpad;
+      int w = 0;
+      for (int k = 2 * lane; k < kp; k += 64) {
+        const double2 x2 = *reinterpret_cast<const double2*>(X + c * kst + k);
+        w = max(w, max(hiword(x2.x), hiword(x2.y)));
+      }
+      w = (int)__reduce_max_sync(0xffffffffu, (unsigned)w);
+      if (lane == 0) colmax[c] = w;
+    }
+    __syncthreads();
+  }
+  // exponent of a column: smallest e with |x| < 2^e
+  auto colexp = [&](int c) { return colmax[c] > 0 ? (colmax[c] >> 20) - 1022 : 0; };
+  if (threadIdx.x < ncolg) {
+    const int c = threadIdx.x;
+    const ColRef cr = FWD ? colref_fwd(P, S, r, i0 + c) : colref_bwd(P, S, r, i0 + c);
+    S.bexp[S.beoff[m * kNT + ctype(c)] + cr.col] = colexp(c) - (8 * NS - 2);
+  }
   // ---- pass 3: digits.  Work item = (column group, 32-wide K chunk).  A
   // column group is the set of columns that share one 256-byte block of a
   // core-matrix tile: 8 rows (one radius of types 2..5) or 4 rows (one radius
@@ -562,7 +575,7 @@ __global__ void __launch_bounds__(kSliceThreads) k_slice_mr(Plan P, SliceTabs S,
   // staging blocks cost the backward CTAs one resident CTA per SM).
   unsigned char* wb = nullptr;
   if constexpr (FWD)
-    wb = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(colexp + kGrpCols) + 15) &
+    wb = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(colmax + kGrpCols) + 15) &
                                           ~static_cast<uintptr_t>(15)) +
          warp * (NS * kSlab);
   int item0 = 0;
@@ -588,8 +601,8 @@ __global__ void __launch_bounds__(kSliceThreads) k_slice_mr(Plan P, SliceTabs S,
         if (!eight) c = 4 * (t - t0) + q;
         else if (4 * fg + (q >> 1) < nF) c = 4 * (4 * fg + (q >> 1)) + 2 * (t - t0) + (q & 1);
         uint32_t wd[NS];
-        if (c >= 0 && colmax[c] > 0.0) {
-          const double sc = pow2((8 * NS - 2) - colexp[c]);
+        if (c >= 0 && colmax[c] > 0) {
+          const double sc = pow2((8 * NS - 2) - colexp(c));
           const double2 x01 = *reinterpret_cast<const double2*>(X + c * kst + k);
           const double2 x23 = *reinterpret_cast<const double2*>(X + c * kst + k + 2);
           const double xv[4] = {x01.x * sc, x01.y * sc, x23.x * sc, x23.y * sc};
@@ -1395,7 +1408,7 @@ static int select_work(const SplitState* s, const Plan& p, bool fwd, const Work*
 
 // dynamic shared memory of one slicer CTA (largest field group): the derived
 // columns X[col][k] (k up to the padded K of the group's types), the column
-// maxima and exponents, and (forward) eight per-warp slice staging blocks
+// maxima, and (forward) eight per-warp slice staging blocks
 size_t slice_smem(const Plan& p, bool fwd, int ns) {
   // K shrinks with m for the backward types and is m-independent forward: m = 0 is the largest
   const int nF = fwd ? p.nvf + p.nsf : p.nvb + p.nsb;
@@ -1404,7 +1417,7 @@ size_t slice_smem(const Plan& p, bool fwd, int ns) {
   const size_t kr = std::max(type_geo(tr, p.L, 0, p.nh).kpad, type_geo(tr + 1, p.L, 0, p.nh).kpad);
   const size_t nx = std::max(8 * kv, 4 * (size_t)nF * kr);
   const size_t stage = fwd ? (kSliceThreads / 32) * (size_t)ns * kSlab + 16 : 0;
-  return sizeof(double) * (nx + 1 + kGrpCols) + kGrpCols * sizeof(int) + stage;
+  return sizeof(double) * (nx + 1) + kGrpCols * sizeof(int) + stage;
 }
 
 int split_slicer(SplitState* s, const Plan& p, bool fwd, const double* d_rj, long long ld, const int* cols,
