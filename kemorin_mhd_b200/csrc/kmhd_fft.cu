@@ -175,18 +175,17 @@ struct Seqs {
 // X[m] = (a - i b)/2 for m > 0, X[0] = a, X[N-m] = conj(X[m]).
 // line: the line's block rows, bs doubles apart (staged: rtm_row; in place in
 // rtm: rtm_row nr nth).
-__device__ __forceinline__ double2 spec_at(const Plan& P, const double* line, long long bs, int nc, int pp, int k) {
+// src: where the pair's components are; two: it holds two.
+__device__ __forceinline__ double2 spec_at(const Plan& P, const double* line, long long bs, const PairSrc& src, bool two,
+                                           int k) {
   // no branch around the loads: a butterfly's loads go out together (zero-band
   // frequencies load order 0)
   const int N = P.nph, L = P.L;
   const bool mirror = k >= N - L, zero = k > L && !mirror;
   const int m = mirror ? N - k : zero ? 0 : k;
-  const bool two = 2 * pp + 1 < nc;
   const double* s = line + (m >> P.mbs) * bs;
-  int ox, oy;
-  bwd_pair(P, m, pp, nc, bwd_in_order(P.nvb, P.nsb), ox, oy);
-  const double2 c0 = *reinterpret_cast<const double2*>(s + ox);
-  const double2 c1 = *reinterpret_cast<const double2*>(s + (two ? oy : ox));
+  const double2 c0 = *reinterpret_cast<const double2*>(s + src.x(m));
+  const double2 c1 = *reinterpret_cast<const double2*>(s + (two ? src.y(m) : src.x(m)));
   const double h = zero ? 0.0 : m == 0 ? 1.0 : 0.5;
   const double h1 = two ? h : 0.0, hs = m == 0 ? 0.0 : mirror ? -h : h, hs1 = m == 0 ? 0.0 : mirror ? -h1 : h1;
   // m = 0: (a_x, a_y); else x / 2 -+ i y / 2 of the two components
@@ -323,8 +322,10 @@ __device__ __forceinline__ void dif_first(const Seqs Z, const Plan& P, const dou
   for (int it = threadIdx.x; it < Z.n * s; it += blockDim.x) {
     const int pp = it / s, j = it - pp * s;
     double2 x[R];
+    const int q = q0 + pp * dq;
+    const PairSrc src(P, q, nc, bwd_in_order(P.nvb, P.nsb));
 #pragma unroll
-    for (int r = 0; r < R; ++r) x[r] = spec_at(P, line + pp * ls, bs, nc, q0 + pp * dq, j + r * s);
+    for (int r = 0; r < R; ++r) x[r] = spec_at(P, line + pp * ls, bs, src, 2 * q + 1 < nc, j + r * s);
     DFT<R, +1>::run(x);
     double2* base = Z.z + pp * Z.zs;
     TwiddleRun<+1> tr(P.twid, j);
@@ -875,9 +876,8 @@ __device__ __forceinline__ void ff_dif_first(const Plan& P, const double* line, 
       // whole block rows apart.
       static_assert(S1 % kRtmOrders == 0, "orders per rtm block");
       const bool two = 2 * pp + 1 < nc;  // the pair holds two components
-      int ux, uy, dx, dy;
-      bwd_pair(P, j, pp, nc, inorder, ux, uy);
-      bwd_pair(P, -j, pp, nc, inorder, dx, dy);
+      const PairSrc src(P, pp, nc, inorder);
+      int ux = src.x(j), uy = src.y(j), dx = src.x(-j), dy = src.y(-j);
       const double* up = line + (j >> kRtmShift) * bs;
       const double* dn = line + ((-j) >> kRtmShift) * bs;
       // staged sectors lie 32 bytes apart: lanes 4..7 of each eight read the
@@ -913,8 +913,9 @@ __device__ __forceinline__ void ff_dif_first(const Plan& P, const double* line, 
       }
       DFT2F_ZM<3, T3, +1>::run(x);
     } else {
+      const PairSrc src(P, pp, nc, inorder);
 #pragma unroll
-      for (int r = 0; r < R; ++r) x[r] = spec_at(P, line, bs, nc, pp, j + r * S1);
+      for (int r = 0; r < R; ++r) x[r] = spec_at(P, line, bs, src, 2 * pp + 1 < nc, j + r * S1);
       DFT<R, +1>::run(x);
     }
     double2* zp = z + pp * NP;
@@ -1296,9 +1297,8 @@ __device__ __forceinline__ void ff_half_first(const Plan& P, const double* line,
   for (int it = threadIdx.x; it < npair * S1; it += blockDim.x) {
     const int pp = it / S1, j = it - pp * S1;
     const bool two = 2 * pp + 1 < nc;
-    int ux, uy, dx, dy;
-    bwd_pair(P, j, pp, nc, inorder, ux, uy);
-    bwd_pair(P, -j, pp, nc, inorder, dx, dy);
+    const PairSrc src(P, pp, nc, inorder);
+    const int ux = src.x(j), uy = src.y(j), dx = src.x(-j), dy = src.y(-j);
     const double* up = line + (j >> kRtmShift) * bs;
     const double* dn = line + ((-j) >> kRtmShift) * bs;
     const double2 zero = make_double2(0.0, 0.0);

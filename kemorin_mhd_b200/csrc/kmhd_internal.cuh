@@ -130,18 +130,23 @@ __host__ __device__ __forceinline__ int rtm_pair(const Plan& P, int m, int q, in
 // (r, theta), (phi, scalar), (scalar) -- instead of by sector: the two sequences
 // of a complex FFT share their rounding error, and u_r is larger than a scalar by
 // a factor of l, u_phi is not (u T at L = 333: 2.9e-15 against 5.0e-14).  Only
-// the reads of the first pass know: pair pp's components start at ox and oy
+// the reads of the first pass know: PairSrc, where pair pp's components start
 // inside order m's block row.
 __host__ __device__ __forceinline__ bool bwd_in_order(int nv, int ns) { return nv == 1 && ns >= 1; }
-__device__ __forceinline__ void bwd_pair(const Plan& P, int m, int pp, int nc, bool in_order, int& ox, int& oy) {
-  if (!in_order) {
-    ox = rtm_pair(P, m, pp, nc);
-    oy = ox + 2;
-  } else {
-    ox = pp == 0 ? rtm_pair(P, m, 1, nc) : pp == 1 ? rtm_pair(P, m, 0, nc) + 2 : rtm_pair(P, m, pp, nc);
-    oy = pp == 0 ? rtm_pair(P, m, 0, nc) : rtm_pair(P, m, 1, nc) + 2;
+struct PairSrc {
+  int x0, xp, y0, yp, msk;  // component x of order m starts at x0 + (m & msk) xp
+  __device__ __forceinline__ PairSrc(const Plan& P, int pp, int nc, bool in_order) {
+    const int qx = in_order && pp < 2 ? 1 - pp : pp, hx = in_order && pp == 1 ? 2 : 0;
+    const int qy = pp, hy = in_order && pp == 0 ? 0 : 2;
+    msk = (1 << P.mbs) - 1;
+    x0 = (qx << (P.mbs + 2)) + hx;
+    xp = 2 * qx + 1 < nc ? 4 : 2;
+    y0 = (qy << (P.mbs + 2)) + hy;
+    yp = xp;
   }
-}
+  __device__ __forceinline__ int x(int m) const { return x0 + (m & msk) * xp; }
+  __device__ __forceinline__ int y(int m) const { return y0 + (m & msk) * yp; }
+};
 // doubles of all records of one direction
 __host__ __device__ __forceinline__ size_t rtm_size(const Plan& P, int nc) {
   return (size_t)rtm_blocks(P) * P.nr * P.nth * rtm_row(P, nc);
