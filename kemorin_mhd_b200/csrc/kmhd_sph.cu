@@ -58,6 +58,7 @@ struct kmhd_sph {
   double2* twid = nullptr;
   int *cols_b_d = nullptr, *cols_f_d = nullptr;
   int* err = nullptr;  // device error word (bounded waits of the FFT and tcgen05 kernels)
+  int* err_h = nullptr;  // its page-locked copy, read back with each call's last synchronisation
   // divergence post-processing: FDM / normalisation coefficients, host-pointer staging
   double *div_coef = nullptr, *div_stage = nullptr, *rot_stage = nullptr;
   // Coriolis curl: coupled modes (4 per j), coefficients (12 per j), staging
@@ -251,6 +252,7 @@ int kmhd_sph_destroy(kmhd_sph* h) {
     delete h->batch;
   }
   for (void* p : h->allocs) cudaFree(p);
+  if (h->err_h) cudaFreeHost(h->err_h);
   for (auto& e : h->ev)
     if (e) cudaEventDestroy(e);
   for (auto& e : h->ev_mid)
@@ -292,6 +294,7 @@ int kmhd_sph_create(const kmhd_sph_desc* d, kmhd_sph** out) {
     if (cudaEventCreate(&e) != cudaSuccess) return fail(KMHD_ERR_CUDA);
   for (auto& e : h->ev_mid)
     if (cudaEventCreate(&e) != cudaSuccess) return fail(KMHD_ERR_CUDA);
+  if (cudaHostAlloc(&h->err_h, sizeof(int), cudaHostAllocDefault) != cudaSuccess) return fail(KMHD_ERR_NOMEM);
 
   Plan& p = h->plan;
   std::memset(&p, 0, sizeof(p));
@@ -591,13 +594,19 @@ int enqueue_cycle(kmhd_sph* h, const double* in, int64_t ld_in, double* out, int
   return run_fwd_spectral(h, out, ld_out, false);
 }
 
-// The instance's device error word (KMHD_ERR_TIMEOUT from a bounded wait of
-// the FFT or tcgen05 kernels); synchronises the handle's stream.
+// Queues the read-back of the instance's device error word (KMHD_ERR_TIMEOUT from
+// a bounded wait of the FFT or tcgen05 kernels) behind the call's work; valid
+// in *err_h once the stream is synchronised.  Read after the synchronisation
+// as a copy of its own it cost a second round trip (10 us of a 135 us call).
+int queue_dev_err(kmhd_sph* h) {
+  KCHECK(cudaMemcpyAsync(h->err_h, h->err, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  return KMHD_OK;
+}
 int check_dev_err(kmhd_sph* h) {
-  int v = 0;
-  KCHECK(cudaMemcpyAsync(&v, h->err, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  const int st = queue_dev_err(h);
+  if (st) return st;
   KCHECK(cudaStreamSynchronize(h->stream));
-  return v;
+  return *h->err_h;
 }
 
 // The registered Coriolis curl of radii [r0, r1): vel / vort point at the S
@@ -703,7 +712,6 @@ int cycle_host_chunked(kmhd_sph* h, const double* d_rj_in, int64_t ld_in, const 
   KCHECK(cudaEventRecord(h->ev[1], h->s_out));
   KCHECK(cudaStreamWaitEvent(h->stream, h->ev[1], 0));
   KCHECK(cudaEventRecord(h->ev[3], h->stream));
-  KCHECK(cudaEventSynchronize(h->ev[3]));
   {
     const int e = check_dev_err(h);
     if (e != KMHD_OK) return e;
@@ -717,8 +725,8 @@ int cycle_host_chunked(kmhd_sph* h, const double* d_rj_in, int64_t ld_in, const 
   return KMHD_OK;
 }
 
+// Ends a call: waits for its stream, reports the device error word, reads the stage timers.
 int finish_timing(kmhd_sph* h) {
-  KCHECK(cudaEventSynchronize(h->ev[3]));
   {
     const int e = check_dev_err(h);
     if (e != KMHD_OK) return e;
@@ -796,7 +804,6 @@ int kmhd_sph_b_trans(kmhd_sph* h, const double* d_rj, int64_t ld, const int32_t*
   KCHECK(cudaEventRecord(h->ev[3], h->stream));
   if (ptr_kind == KMHD_PTR_HOST)
     KCHECK(cudaMemcpyAsync(fld_rtp, grid, sizeof(double) * nnod * p.ncb, cudaMemcpyDeviceToHost, h->stream));
-  KCHECK(cudaStreamSynchronize(h->stream));
   return finish_timing(h);
 }
 
@@ -852,7 +859,6 @@ int kmhd_sph_f_trans(kmhd_sph* h, const double* frc_rtp, double* d_rj, int64_t l
                              h->stream));
     h->cor_pending = 0;
   }
-  KCHECK(cudaStreamSynchronize(h->stream));
   return finish_timing(h);
 }
 
@@ -923,7 +929,6 @@ int kmhd_sph_cycle(kmhd_sph* h, const double* d_rj_in, int64_t ld_in, const int3
         KCHECK(cudaMemcpyAsync(d_rj_out + ld_out * (h->cor_col + 2 * q), h->cor_cyc + nrj * q,
                                sizeof(double) * nrj, cudaMemcpyDeviceToHost, h->stream));
   }
-  KCHECK(cudaStreamSynchronize(h->stream));
   if ((st = finish_timing(h))) return st;
   return finish_kernel_timing(h);
 }
@@ -1831,9 +1836,11 @@ int batch_cycle_impl(kmhd_sph** hs, int32_t n, const double* const* d_rj_in, con
       return st;
     }
   }
-  for (int i = 0; i < n; ++i) {
-    const int e = check_dev_err(hs[i]);
-    if (e != KMHD_OK) return e;
-  }
+  // every word's copy is queued before the first wait
+  for (int i = 0; i < n; ++i)
+    if ((st = queue_dev_err(hs[i]))) return st;
+  for (int i = 0; i < n; ++i) KCHECK(cudaStreamSynchronize(hs[i]->stream));
+  for (int i = 0; i < n; ++i)
+    if (*hs[i]->err_h != KMHD_OK) return *hs[i]->err_h;
   return KMHD_OK;
 }
