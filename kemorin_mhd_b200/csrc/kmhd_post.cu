@@ -8,6 +8,8 @@
 // fixed-field boundary rows as cal_sph_div_flux_4_fix_in / _fix_out
 // (MHD_src/sph_MHD/cal_sph_exp_fixed_scalar.f90:381-456); the FDM coefficients
 // are built on the host (kmhd_sph.cu) as the reference builds them.
+#include <algorithm>
+
 #include "kmhd_internal.cuh"
 
 namespace kmhd {
@@ -44,8 +46,32 @@ __global__ void k_div_flux(long long J, int nr, const double* __restrict__ S, co
   }
 }
 
-// Curl of a vector (S, dS/dr, T) into (pol, dpol/dr, tor), one thread per
-// (j, k).  Interior rows as cal_sph_nod_vect_w_div_rot2
+// The rows of the curls are walked by one thread per mode j over a range of
+// radii [k0, k1) with a window of three radii in registers: every element is
+// loaded once, coalesced over j.  Bound by HBM.  us at L = 255, Nr = 129, one
+// thread per (j, k) before -> ranges of eight radii here (one radius, two,
+// four): curl of a field 119 -> 82 (102, 92, 83), of a force 104 -> 98 (117, 106,
+// 99), buoyancy 40.6 -> 35.1 (43, 40, 36).  The divergence, with one column to
+// difference and one to read, is faster by points (56 against 70).
+struct Window {
+  double m, c, p;  // radii k - 1, k, k + 1
+  const double* f;
+  long long J;
+  int nr;
+  __device__ __forceinline__ Window(const double* f_, long long j, long long J_, int nr_, int k) : f(f_ + j), J(J_), nr(nr_) {
+    m = k > 0 ? f[(k - 1) * J] : 0.0;
+    c = f[k * J];
+    p = k + 1 < nr ? f[(k + 1) * J] : 0.0;
+  }
+  __device__ __forceinline__ void step(int k) {  // from radius k to k + 1
+    m = c;
+    c = p;
+    p = k + 2 < nr ? f[(k + 2) * J] : 0.0;
+  }
+  __device__ __forceinline__ double at(int k) const { return f[k * J]; }
+};
+
+// Curl of a vector (S, dS/dr, T) into (pol, dpol/dr, tor).  Interior rows as cal_sph_nod_vect_w_div_rot2
 // (MHD_src/sph_MHD/cal_sph_exp_rotation.f90:207-248).  Boundary rows per side:
 // - insulating (curl of u x B): cal_sph_nod_icb_ins_vp_rot2 /
 //   cal_sph_nod_cmb_ins_vp_rot2 (cal_sph_exp_nod_icb_ins.f90:135-160,
@@ -57,63 +83,68 @@ __global__ void k_div_flux(long long J, int nr, const double* __restrict__ S, co
 //   cal_sph_nod_icb_free_rot2 / cal_sph_nod_cmb_free_rot2).
 // coef as k_div_flux, then ar1[nr] = 1/r, gl[J] = l and d2[3 nr] (second
 // derivative, offsets -1, 0, +1).
-__global__ void k_rot_vec(long long J, int nr, const double* __restrict__ S, const double* __restrict__ dS,
+// X: the column whose radial derivative the interior rows take, S (second
+// derivative, D2) or dS/dr (first).
+template <bool D2>
+__global__ void k_rot_vec(long long J, int nr, int kchunk, const double* __restrict__ S, const double* __restrict__ dS,
                           const double* __restrict__ T, double* __restrict__ pol, double* __restrict__ dpol,
                           double* __restrict__ tor, const double* __restrict__ coef, const RotBnd b) {
+  const long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (j >= J) return;
   const double* d1 = coef;
   const double* ar2 = coef + 3 * nr + 6;
-  const double* g3 = ar2 + nr;
-  const double* ar1 = g3 + J;
-  const double* gl = ar1 + nr;
-  const double* d2 = gl + J;  // interior 3-point second derivative
-  const long long n = J * nr;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const int k = (int)(i / J);
-    const long long j = i - (long long)k * J;
-    const double t = T[i];
-    // g_sph_rj(j,3) = l(l+1), 0 at l = 0 (the rj copy has no l = 0 override;
-    // the coefficient array holds max(l(l+1), 1/2) for the divergence)
-    const double g3j = gl[j] > 0.0 ? g3[j] : 0.0;
+  const double* g3a = ar2 + nr;
+  const double* ar1 = g3a + J;
+  const double* gla = ar1 + nr;
+  const double* dx = D2 ? gla + J : d1;  // interior rows of X
+  // g_sph_rj(j,3) = l(l+1), 0 at l = 0 (the rj copy has no l = 0 override;
+  // the coefficient array holds max(l(l+1), 1/2) for the divergence)
+  const double gl = gla[j], g3j = gl > 0.0 ? g3a[j] : 0.0;
+  const int k0 = blockIdx.y * kchunk, k1 = min(nr, k0 + kchunk);
+  Window t(T, j, J, nr, k0), x(D2 ? S : dS, j, J, nr, k0);
+  for (int k = k0; k < k1; ++k) {
+    const long long i = k * J + j;
+    const double s = D2 ? x.c : S[i];
     double dp, tr;
     if (k == 0) {
       if (b.qvac_in) {  // pseudo-vacuum (radial field): cal_sph_nod_icb_qvc_vp_rot2
         dp = 0.0;
         tr = 0.0;
       } else if (b.insulating_in) {
-        dp = (gl[j] + 1.0) * ar1[0] * t;
+        dp = (gl + 1.0) * ar1[0] * t.c;
         tr = 0.0;
       } else {
-        const double s0 = b.ins_s_in ? (gl[j] + 1.0) * ar1[0] * b.cdr_in + b.s_in[0] : b.s_in[0];
-        const double d2s = s0 * S[i] + b.s_in[1] * S[i + J];
-        dp = b.t_in[0] * t + b.t_in[1] * T[i + J] + b.t_in[2] * T[i + 2 * J];
-        tr = -(d2s - g3j * ar2[0] * S[i]);
+        const double s0 = b.ins_s_in ? (gl + 1.0) * ar1[0] * b.cdr_in + b.s_in[0] : b.s_in[0];
+        const double d2s = s0 * s + b.s_in[1] * (D2 ? x.p : S[i + J]);
+        dp = b.t_in[0] * t.c + b.t_in[1] * t.p + b.t_in[2] * t.at(2);
+        tr = -(d2s - g3j * ar2[0] * s);
       }
     } else if (k == nr - 1) {
       if (b.qvac_out) {  // cal_sph_nod_cmb_qvc_vp_rot2
         dp = 0.0;
         tr = 0.0;
       } else if (b.insulating_out) {
-        dp = -gl[j] * ar1[k] * t;
+        dp = -gl * ar1[k] * t.c;
         tr = 0.0;
       } else {
-        const double s0 = b.ins_s_out ? b.s_out[0] - gl[j] * ar1[k] * b.cdr_out : b.s_out[0];
-        const double d2s = b.s_out[1] * S[i - J] + s0 * S[i];
-        dp = b.t_out[2] * T[i - 2 * J] + b.t_out[1] * T[i - J] + b.t_out[0] * t;
-        tr = -(d2s - g3j * ar2[k] * S[i]);
+        const double s0 = b.ins_s_out ? b.s_out[0] - gl * ar1[k] * b.cdr_out : b.s_out[0];
+        const double d2s = b.s_out[1] * (D2 ? x.m : S[i - J]) + s0 * s;
+        dp = b.t_out[2] * t.at(k - 2) + b.t_out[1] * t.m + b.t_out[0] * t.c;
+        tr = -(d2s - g3j * ar2[k] * s);
       }
     } else {
-      dp = d1[3 * k] * T[i - J] + d1[3 * k + 1] * t + d1[3 * k + 2] * T[i + J];
-      if (b.d2_interior) {  // cal_sph_nod_vect_rot2 (cal_sph_exp_rotation.f90:157-203)
-        const double d2s = d2[3 * k] * S[i - J] + d2[3 * k + 1] * S[i] + d2[3 * k + 2] * S[i + J];
-        tr = -d2s + g3j * ar2[k] * S[i];
-      } else {
-        const double d1d = d1[3 * k] * dS[i - J] + d1[3 * k + 1] * dS[i] + d1[3 * k + 2] * dS[i + J];
-        tr = -d1d + g3j * ar2[k] * S[i];
-      }
+      dp = d1[3 * k] * t.m + d1[3 * k + 1] * t.c + d1[3 * k + 2] * t.p;
+      // cal_sph_nod_vect_rot2 (cal_sph_exp_rotation.f90:157-203), or the first derivative of dS/dr
+      const double dd = dx[3 * k] * x.m + dx[3 * k + 1] * x.c + dx[3 * k + 2] * x.p;
+      tr = -dd + g3j * ar2[k] * s;
     }
-    pol[i] = t;
+    pol[i] = t.c;
     dpol[i] = dp;
     tor[i] = tr;
+    if (k + 1 < k1) {
+      t.step(k);
+      x.step(k);
+    }
   }
 }
 
@@ -258,41 +289,55 @@ __global__ void k_b_trans_center(Plan P, const double* __restrict__ d_rj, long l
 // Curl of the radial buoyancy (toroidal part): out = coef_t T r, or
 // (coef_t T + coef_c C) r with a second scalar (cal_rot_buoyancy_sph_MHD /
 // cal_rot_double_buoyancy_sph_MHD, MHD_src/sph_MHD/cal_rot_buoyancies_sph_MHD.f90:106-165).
-__global__ void k_rot_buoyancy(long long J, int nr, const double* __restrict__ T, double coef_t,
+__global__ void k_rot_buoyancy(long long J, int nr, int kchunk, const double* __restrict__ T, double coef_t,
                                const double* __restrict__ C, double coef_c, double* __restrict__ out,
                                const double* __restrict__ radius) {
-  const long long n = J * nr;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const int k = (int)(i / J);
+  const long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (j >= J) return;
+  const int k0 = blockIdx.y * kchunk, k1 = min(nr, k0 + kchunk);
+#pragma unroll 4
+  for (int k = k0; k < k1; ++k) {
+    const long long i = k * J + j;
     out[i] = C ? (coef_t * T[i] + coef_c * C[i]) * radius[k] : coef_t * T[i] * radius[k];
   }
+}
+
+// Blocks of 256 modes times ranges of at most eight radii, fewer where that
+// leaves less than eight CTAs per SM (Coriolis curl, L = 255, Nr = 129: 127 us;
+// four radii 135, sixteen 133, the whole shell's share of eight CTAs per SM 149).
+struct RadialGrid {
+  dim3 grid;
+  int kchunk;
+};
+RadialGrid radial_grid(long long J, int nr) {
+  int dev = 0, nsm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  const long long jb = (J + 255) / 256;
+  long long ks = std::max<long long>(1, (8LL * nsm + jb - 1) / std::max<long long>(jb, 1));
+  if (ks > nr) ks = nr;
+  RadialGrid g;
+  g.kchunk = std::min((int)((nr + ks - 1) / ks), 8);
+  g.grid = dim3((unsigned)jb, (unsigned)((nr + g.kchunk - 1) / g.kchunk));
+  return g;
 }
 
 }  // namespace
 
 cudaError_t launch_rot_vec(long long J, int nr, const double* S, const double* dS, const double* T, double* pol,
                            double* dpol, double* tor, const double* coef, const RotBnd& b, cudaStream_t s) {
-  const long long n = J * nr;
-  int dev = 0, nsm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const long long want = (n + 255) / 256;
-  const int grid = (int)(want < 8LL * nsm ? want : 8LL * nsm);
-  if (grid <= 0) return cudaSuccess;
-  k_rot_vec<<<grid, 256, 0, s>>>(J, nr, S, dS, T, pol, dpol, tor, coef, b);
+  if (J <= 0 || nr <= 0) return cudaSuccess;
+  const RadialGrid g = radial_grid(J, nr);
+  if (b.d2_interior) k_rot_vec<true><<<g.grid, 256, 0, s>>>(J, nr, g.kchunk, S, dS, T, pol, dpol, tor, coef, b);
+  else k_rot_vec<false><<<g.grid, 256, 0, s>>>(J, nr, g.kchunk, S, dS, T, pol, dpol, tor, coef, b);
   return cudaGetLastError();
 }
 
 cudaError_t launch_rot_buoyancy(long long J, int nr, const double* T, double coef_t, const double* C, double coef_c,
                                 double* out, const double* radius, cudaStream_t s) {
-  const long long n = J * nr;
-  int dev = 0, nsm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const long long want = (n + 255) / 256;
-  const int grid = (int)(want < 8LL * nsm ? want : 8LL * nsm);
-  if (grid <= 0) return cudaSuccess;
-  k_rot_buoyancy<<<grid, 256, 0, s>>>(J, nr, T, coef_t, C, coef_c, out, radius);
+  if (J <= 0 || nr <= 0) return cudaSuccess;
+  const RadialGrid g = radial_grid(J, nr);
+  k_rot_buoyancy<<<g.grid, 256, 0, s>>>(J, nr, g.kchunk, T, coef_t, C, coef_c, out, radius);
   return cudaGetLastError();
 }
 
@@ -314,19 +359,10 @@ cudaError_t launch_b_trans_center(const Plan& p, const double* d_rj, long long l
 cudaError_t launch_rot_coriolis(long long J, int nr, const double* vel, const double* vort, long long ld,
                                 double* pol, double* tor, const int* idx, const double* cf, const double* radius,
                                 double coef_cor, cudaStream_t s) {
-  int dev = 0, nsm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const long long jb = (J + 255) / 256;
-  if (jb <= 0 || nr <= 0) return cudaSuccess;
-  // enough blocks for 8 per SM; each block walks a contiguous range of radii
-  long long ks = (8LL * nsm + jb - 1) / jb;
-  if (ks > nr) ks = nr;
-  const int kchunk = (int)((nr + ks - 1) / ks);
-  const int ky = (nr + kchunk - 1) / kchunk;
-  k_rot_coriolis<<<dim3((unsigned)jb, (unsigned)ky), 256, 0, s>>>(J, nr, kchunk, vel, vel + ld, vort, vort + ld,
-                                                                   vort + 2 * ld, pol, tor, idx, cf, radius,
-                                                                   coef_cor);
+  if (J <= 0 || nr <= 0) return cudaSuccess;
+  const RadialGrid g = radial_grid(J, nr);
+  k_rot_coriolis<<<g.grid, 256, 0, s>>>(J, nr, g.kchunk, vel, vel + ld, vort, vort + ld, vort + 2 * ld, pol, tor, idx, cf,
+                                        radius, coef_cor);
   return cudaGetLastError();
 }
 
