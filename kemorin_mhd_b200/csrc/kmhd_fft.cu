@@ -766,12 +766,22 @@ __global__ void __launch_bounds__(kGridThreads, 2)
   const double* __restrict__ f0 = frc + nnod * pair_comp(q, 0, P.nvf) + r0 + (long long)P.nr * th;
   const double* __restrict__ f1 = two ? frc + nnod * pair_comp(q, 1, P.nvf) + r0 + (long long)P.nr * th : nullptr;
   const long long ps = (long long)P.nr * P.nth;
-#pragma unroll 4
-  for (int it = threadIdx.x; it < N << lrad; it += blockDim.x) {
-    const int r = it & (rad - 1), pos = it >> lrad;
-    if (r >= nrad) continue;
-    const long long o = ps * __ldg(P.digrev + pos) + r;
-    Z.z[r * Z.zs + Z.ix(pos)] = make_double2(__ldg(f0 + o), two ? __ldg(f1 + o) : 0.0);
+  // eight grid loads of a thread in flight
+  constexpr int U = 4;
+  for (int it = threadIdx.x; it < N << lrad; it += U * blockDim.x) {
+    double lo[U], hi[U];
+    int ix[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int e = it + u * blockDim.x, r = e & (rad - 1), pos = e >> lrad;
+      ix[u] = e < N << lrad && r < nrad ? r * Z.zs + Z.ix(pos) : -1;
+      const long long o = ix[u] >= 0 ? ps * __ldg(P.digrev + pos) + r : 0;
+      lo[u] = __ldg(f0 + o);
+      hi[u] = two ? __ldg(f1 + o) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (ix[u] >= 0) Z.z[ix[u]] = make_double2(lo[u], hi[u]);
   }
   __syncthreads();
   dit_all(Z, P);
@@ -1411,7 +1421,6 @@ template <int NH, int MVB, int MSB, int MVF, int MSF, bool EX, bool PR, int PK>
 __global__ void __launch_bounds__(kFftThreadsF, 1)
     k_fft_cycle_half(const __grid_constant__ Plan P, int line0, int nlines, const __grid_constant__ CUtensorMap tmap) {
   extern __shared__ double4 smraw[];
-  constexpr int NP = NH + 1;
   const int ncb = EX ? 3 * MVB + MSB : P.ncb, ncf = EX ? 3 * MVF + MSF : P.ncf;
   const int npb = (ncb + 1) / 2, npf = (ncf + 1) / 2;
   double2* z = reinterpret_cast<double2*>(smraw);
