@@ -1162,12 +1162,13 @@ cudaError_t launch_leg_fwd_f64(const Plan& p, double* d_rj, long long ld, const 
                                cudaStream_t s, int m_count) {
   if (m_count <= 0 || m_count > p.L + 1) m_count = p.L + 1;
   // 64 degrees per parity and a whole SM per CTA: for truncations that fill them
-  // and launches with several CTAs per SM (not the few orders of the split
-  // tiers' dipole modes).  ms 32-degree kernel -> this one: L = 255, Nr = 129 3.94 ->
-  // 3.62; L = 511, Nr = 17 4.00 -> 3.61; L = 1023, Nr = 17 29.0 -> 25.9; but L = 106,
-  // Nr = 47 0.252 -> 0.259, L = 31, Nr = 33 0.031 -> 0.043 (most warps without a degree).
+  // and launches of at least one CTA per SM (not the few orders of the split
+  // tiers' dipole modes at small Nr).  ms 32-degree kernel -> this one: L = 127, Nr =
+  // 65 0.447 -> 0.409, Nr = 5 (256 CTAs) 0.081 -> 0.060; L = 255, Nr = 3 0.168 ->
+  // 0.142, Nr = 129 3.94 -> 3.62; L = 1023, Nr = 17 29.0 -> 25.9; the same at L = 95
+  // and 106; but L = 63, Nr = 33 0.051 -> 0.065 (most warps without a degree).
   const long long ctas = (long long)((kcount(p.L, 0, 0) + kLB16 - 1) / kLB16) * win_nrb(p) * m_count;
-  if (!p.otf && p.L >= 128 && ctas >= 4 * 148) return run_fwd16(p, d_rj, ld, cols, s, m_count);
+  if (!p.otf && p.L >= 112 && ctas >= 148) return run_fwd16(p, d_rj, ld, cols, s, m_count);
   KMHD_DISPATCH(p.nvf, p.nsf, run_fwd, p, d_rj, ld, cols, s, m_count);
 }
 
