@@ -8,7 +8,7 @@
 //   V(theta, col) = sum_k Ptab[m][p][k][theta] * SB[m][p][k][col]
 // for P and dP, then the N/S (sym +/- asym) recombination and the +-m cross
 // terms are applied in registers and the grid spectra are written to
-// rtm_b[m][theta][r][comp][cos,sin].
+// the rtm_b records (layout: rtm_off, rtm_pair).
 //
 // Forward (leg_f_trans_vec_sym_dgemm, legendre_fwd_sym_matmul.f90:315-452,
 // pack set_vr_rtm_for_leg_matmul.f90:170-364, unpack cal_sp_rlm_by_matmul.f90:172-360):
@@ -22,6 +22,7 @@
 // backward direction (a = S g3 / r^2, b = dS/dr / r, c = T / r), so the m8n8
 // accumulator fragment of a thread (row g, columns 2t, 2t+1) holds the cos and
 // sin slots of one radius.
+#include <algorithm>
 #include <type_traits>
 
 #include "kmhd_internal.cuh"
@@ -92,6 +93,22 @@ __global__ void __launch_bounds__(kThreads) k_pack_b(const __grid_constant__ Pla
     if (k < p.kpad[2 * m + par])
       p.SB[p.sboff[2 * m + par] + (long long)k * (p.nrb * CB) + rb * CB + c] = sm[ll * ST + c];
   }
+}
+
+// +-m cross terms of a vector: products a(tile, parity, slot), tiles XP, XdP, YP, YdP, ZP, slots cos, sin ->
+// (theta cos, theta sin, phi cos, phi sin), equator-symmetric and antisymmetric.
+// theta: own slot dP*b, mirror slot -/+ m/sin * P*c;
+// phi: own slot -dP*c, mirror slot +/- m/sin * P*b
+template <typename F>
+__device__ __forceinline__ void cross_terms(F a, double ms, double (&sy)[4], double (&as)[4]) {
+  sy[0] = a(1, 1, 0) + ms * a(2, 0, 1);
+  sy[1] = a(1, 1, 1) - ms * a(2, 0, 0);
+  sy[2] = -a(3, 1, 0) + ms * a(0, 0, 1);
+  sy[3] = -a(3, 1, 1) - ms * a(0, 0, 0);
+  as[0] = a(1, 0, 0) + ms * a(2, 1, 1);
+  as[1] = a(1, 0, 1) - ms * a(2, 1, 0);
+  as[2] = -a(3, 0, 0) + ms * a(0, 1, 1);
+  as[3] = -a(3, 0, 1) - ms * a(0, 1, 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -308,12 +325,8 @@ __global__ void __launch_bounds__(kThreads + (OTF ? kGenThreadsB : 0), 1) k_leg_
   };
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
-    // theta: own slot dP*b, mirror slot -/+ m/sin * P*c;
-    // phi: own slot -dP*c, mirror slot +/- m/sin * P*b
-    const double sy[4] = {acc[v][1][1][0] + ms * acc[v][2][0][1], acc[v][1][1][1] - ms * acc[v][2][0][0],
-                          -acc[v][3][1][0] + ms * acc[v][0][0][1], -acc[v][3][1][1] - ms * acc[v][0][0][0]};
-    const double as[4] = {acc[v][1][0][0] + ms * acc[v][2][1][1], acc[v][1][0][1] - ms * acc[v][2][1][0],
-                          -acc[v][3][0][0] + ms * acc[v][0][1][1], -acc[v][3][0][1] - ms * acc[v][0][1][0]};
+    double sy[4], as[4];
+    cross_terms([&](int tile, int par, int slot) { return acc[v][tile][par][slot]; }, ms, sy, as);
     put(v, sy, as);
   }
   // radial components and scalars, two list entries per pair
@@ -619,7 +632,8 @@ k_leg_fwd_f64(Plan p, double* __restrict__ d_rj, long long ld, const int* __rest
 // buffered, so a chunk costs one barrier and its staging runs beside the other
 // warps' DMMAs.  A field group holds at most three vectors (16 accumulator tiles
 // of four doubles per lane; more would spill): groups share nothing but the A
-// operand, so larger sets run group by group.
+// operand, so larger sets run group by group.  The sums are those of the 8-row
+// kernel in the same order, so the two agree bit for bit.
 constexpr int kLB16 = 64;  // degrees per parity of a CTA
 
 template <int NV, int NS>
@@ -846,46 +860,48 @@ cudaError_t run_fwd16(const Plan& p, double* d_rj, long long ld, const int* cols
   return cudaGetLastError();
 }
 // ---------------------------------------------------------------------------
-// Backward kernel of the stored tables.  CTA = (m, 64 latitudes, 8 radii, field
-// group); 8 warps = (16 latitudes, 4 radii).  The +-m cross terms are summed
-// inside the accumulators: m/sin P is a third A operand and the mirror slot's
-// columns are B fragments of the neighbouring column with a sign, so a vector
-// needs six output tiles (sym / asym of r, theta, phi) where separate P and dP
-// products of each parity take ten, and 16 latitudes per warp (m16n8k4) fit the
-// registers: one B fragment serves 16 rows.  Operands come through a ring of
-// four cp.async stages, one barrier per chunk.  A field group holds at most
-// three vectors (see k_leg_fwd16); groups start at even vectors, so no record
-// pair is split between two of them.
+// Backward kernel of the stored tables.  8 warps of m16n8k4: one B fragment serves
+// 16 rows where the 8-row kernel reads it twice.  The products and their order
+// are the 8-row kernel's (P and dP of each parity summed on their own, the +-m
+// terms scaled and added at the end), and both DMMA shapes round alike, so the
+// two kernels agree bit for bit: which one a launch takes does not show in the
+// results of a radial window or slab.  (Summing the +-m terms into the same
+// accumulators, m/sin P as a third operand, takes 3% less time at L = 255, Nr =
+// 129, but its theta and phi sums have 1.3 times the rounding error at L = 63 ..
+// 511.)  Operands come through a ring of four
+// cp.async stages, one barrier per chunk.  A CTA takes one field group, at most
+// two vectors (20 accumulator tiles of four doubles per lane, and two per
+// scalar); groups start at even vectors, so no record pair is split between two
+// of them.  A group of one vector takes twice the radii, so that its warps have
+// as many columns to share the A fragments (default set at L = 255, Nr = 129,
+// two launches: 2.83 ms with eight radii, 2.74 so; one launch 2.72).
 constexpr int kRing16 = 4;
 
+// group: CTA = (m, 64 latitudes, 8 RB radii), warp = (16 latitudes, 4 RB radii)
 template <int NV, int NS>
 struct Bwd16Geo {
+  static constexpr int RB = NV == 1 && NS <= 1 ? 2 : 1;
   static constexpr int CB = 24 * NV + 8 * NS;
   static constexpr int CBp = CB + ((4 - CB % 16) + 16) % 16;
   static constexpr int AS = kThBlk + 4;
   static constexpr int A_STAGE = 2 * kKC * AS;
-  static constexpr int B_STAGE = 2 * kKC * CBp;  // two radial blocks
+  static constexpr int B_STAGE = 2 * RB * kKC * CBp;
   static constexpr size_t SMEM = sizeof(double) * kRing16 * (A_STAGE + B_STAGE);
+  __host__ __device__ static int radial_ctas(const Plan& p) { return (win_nrb(p) + 2 * RB - 1) / (2 * RB); }
 };
 
+// order m, latitudes from th0, radial CTA rp of the group of vectors v0 .. v0 + NV - 1 and scalars 0 .. NS - 1
 template <int NV, int NS>
-__global__ void __launch_bounds__(kThreads, 1) k_leg_bwd16(const __grid_constant__ Plan p, int v0, int s0) {
+__device__ __forceinline__ void bwd16_group(const Plan& p, double* sm, int m, int th0, int rp, int v0) {
   using G = Bwd16Geo<NV, NS>;
-  extern __shared__ double sm[];
+  constexpr int RB = G::RB;
   double* sA = sm;                            // [ring][P, dP][kKC][AS]
-  double* sB = sm + kRing16 * G::A_STAGE;     // [ring][2 radial blocks][kKC][CBp]
-  const int nthb = p.nh_pad / kThBlk;
-  const int nrbw = win_nrb(p), nrp = (nrbw + 1) / 2;
-  int b = blockIdx.x;
-  const int rp = b % nrp;
-  b /= nrp;
-  const int th0 = (b % nthb) * kThBlk;
-  const int m = b / nthb;
+  double* sB = sm + kRing16 * G::A_STAGE;     // [ring][2 RB radial blocks][kKC][CBp]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int tg = warp & 3, rbi = warp >> 2;
-  const int nrb_here = min(2, nrbw - 2 * rp);  // radial blocks of this CTA
-  const int rb0 = win_rb0(p) + 2 * rp;
+  const int tg = warp & 3, rbi = warp >> 2;  // radial blocks rbi, rbi + 2, ...
+  const int nrb_here = min(2 * RB, win_nrb(p) - 2 * RB * rp);  // of this CTA
+  const int rb0 = win_rb0(p) + 2 * RB * rp;
   const int n0 = p.kpad[2 * m] / kKC, n1 = p.kpad[2 * m + 1] / kKC;
   const int total = n0 + n1;
   const int CBt = 24 * p.nvb + 8 * p.nsb;     // columns of one radial block in SB
@@ -908,61 +924,60 @@ __global__ void __launch_bounds__(kThreads, 1) k_leg_bwd16(const __grid_constant
     const double* Bg = p.SB + p.sboff[2 * m + par] + (long long)(ch * kKC) * rowB + (long long)rb0 * CBt;
     double* bs = sB + st * G::B_STAGE;
     constexpr int NV2 = 12 * NV, NP2 = 12 * NV + 4 * NS;  // 16-byte pieces of a row: vectors, all
-    for (int it = tid; it < 2 * kKC * NP2; it += kThreads) {
+    for (int it = tid; it < 2 * RB * kKC * NP2; it += kThreads) {
       const int rr = it / NP2, c2 = it - rr * NP2;  // rr = radial block * kKC + row
       const int q = rr / kKC, row = rr % kKC;
       if (q >= nrb_here) break;
-      const int src = c2 < NV2 ? 24 * v0 + 2 * c2 : 24 * p.nvb + 8 * s0 + 2 * (c2 - NV2);
+      const int src = c2 < NV2 ? 24 * v0 + 2 * c2 : 24 * p.nvb + 2 * (c2 - NV2);
       cp_async16(bs + rr * G::CBp + 2 * c2, Bg + row * rowB + q * CBt + src);
     }
   };
 
-  // tiles of a vector: [r, theta, phi][sym, asym]; of a scalar: [sym, asym]
-  double acc[NV > 0 ? NV : 1][3][2][4];
-  double accS[NS > 0 ? NS : 1][2][4];
+  // accumulators: [radial block][field][tile][parity][row g, g + 8: cos, sin]; tiles XP, XdP, YP, YdP, ZP
+  double acc[RB][NV][5][2][4];
+  double accS[RB][NS > 0 ? NS : 1][2][4];
 #pragma unroll
-  for (int v = 0; v < (NV > 0 ? NV : 1); ++v)
+  for (int u = 0; u < RB; ++u) {
 #pragma unroll
-    for (int q = 0; q < 3; ++q)
+    for (int v = 0; v < NV; ++v)
+#pragma unroll
+      for (int q = 0; q < 5; ++q)
+#pragma unroll
+        for (int s = 0; s < 2; ++s)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[u][v][q][s][e] = 0.0;
+#pragma unroll
+    for (int v = 0; v < (NS > 0 ? NS : 1); ++v)
 #pragma unroll
       for (int s = 0; s < 2; ++s)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc[v][q][s][e] = 0.0;
-#pragma unroll
-  for (int v = 0; v < (NS > 0 ? NS : 1); ++v)
-#pragma unroll
-    for (int s = 0; s < 2; ++s)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) accS[v][s][e] = 0.0;
+        for (int e = 0; e < 4; ++e) accS[u][v][s][e] = 0.0;
+  }
 
-  const int i0 = th0 + 16 * tg + g;  // latitudes i0, i0 + 8
-  const double ms0 = i0 < p.nh ? (double)m * p.asin_t[i0] : 0.0;
-  const double ms1 = i0 + 8 < p.nh ? (double)m * p.asin_t[i0 + 8] : 0.0;
-  const double sg = (g & 1) ? -1.0 : 1.0;  // mirror slot: cos takes +sin, sin takes -cos
-
-  // chunk of parity par: P feeds sym (par = 0) or asym r, dP asym or sym, m/sin P sym or asym theta / phi
-  auto compute = [&](int st, auto parc) {
-    constexpr int par = decltype(parc)::value;
+  // nu: radial blocks of this warp
+  auto compute = [&](int st, auto parc, auto nuc) {
+    constexpr int par = decltype(parc)::value, nu = decltype(nuc)::value;
     const double* a = sA + st * G::A_STAGE + t * G::AS + 16 * tg + g;
-    const double* bs = sB + st * G::B_STAGE + (rbi * kKC + t) * G::CBp;
+    const double* bs = sB + st * G::B_STAGE + (rbi * kKC + t) * G::CBp + g;
 #pragma unroll
     for (int kk = 0; kk < kKC / 4; ++kk) {
       const double p0 = a[4 * kk * G::AS], p1 = a[4 * kk * G::AS + 8];
       const double d0 = a[(kKC + 4 * kk) * G::AS], d1 = a[(kKC + 4 * kk) * G::AS + 8];
-      const double q0 = ms0 * p0, q1 = ms1 * p1;
-      const double* br = bs + 4 * kk * G::CBp;
 #pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        const double bX = br[24 * v + g], bY = br[24 * v + 8 + g], bZ = br[24 * v + 16 + g];
-        const double mX = sg * br[24 * v + (g ^ 1)], mY = sg * br[24 * v + 8 + (g ^ 1)];
-        dmma16(acc[v][0][par], p0, p1, bZ);
-        dmma16(acc[v][1][1 - par], d0, d1, bX);
-        dmma16(acc[v][1][par], q0, q1, mY);
-        dmma16(acc[v][2][1 - par], d0, d1, -bY);
-        dmma16(acc[v][2][par], q0, q1, mX);
+      for (int u = 0; u < nu; ++u) {
+        const double* br = bs + (2 * u * kKC + 4 * kk) * G::CBp;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+          const double bX = br[24 * v], bY = br[24 * v + 8], bZ = br[24 * v + 16];
+          dmma16(acc[u][v][0][par], p0, p1, bX);
+          dmma16(acc[u][v][1][par], d0, d1, bX);
+          dmma16(acc[u][v][2][par], p0, p1, bY);
+          dmma16(acc[u][v][3][par], d0, d1, bY);
+          dmma16(acc[u][v][4][par], p0, p1, bZ);
+        }
+#pragma unroll
+        for (int s = 0; s < NS; ++s) dmma16(accS[u][s][par], p0, p1, br[24 * NV + 8 * s]);
       }
-#pragma unroll
-      for (int s = 0; s < NS; ++s) dmma16(accS[s][par], p0, p1, br[24 * NV + 8 * s + g]);
     }
   };
 
@@ -976,104 +991,146 @@ __global__ void __launch_bounds__(kThreads, 1) k_leg_bwd16(const __grid_constant
     __syncthreads();  // stage step has landed; every warp is done with the stage that load() overwrites
     if (step + kRing16 - 1 < total) load(step + kRing16 - 1);
     cp_async_commit();
-    if (active) {
-      if (step < n0) compute(step % kRing16, std::integral_constant<int, 0>());
-      else compute(step % kRing16, std::integral_constant<int, 1>());
+    if (!active) continue;
+    using One = std::integral_constant<int, 1>;
+    using All = std::integral_constant<int, RB>;
+    const bool all = rbi + 2 * (RB - 1) < nrb_here;
+    if (step < n0) {
+      if (all) compute(step % kRing16, std::integral_constant<int, 0>(), All());
+      else compute(step % kRing16, std::integral_constant<int, 0>(), One());
+    } else {
+      if (all) compute(step % kRing16, std::integral_constant<int, 1>(), All());
+      else compute(step % kRing16, std::integral_constant<int, 1>(), One());
     }
   }
   cp_async_wait<0>();
 
-  // ---- epilogue: north = sym + asym, south = sym - asym
-  const int r = kRB * (rb0 + rbi) + t;
-  if (!active || r >= p.nr) return;
+  // ---- epilogue: N/S recombination and +-m cross terms
+  if (!active) return;
   const int nc = p.ncb;
   const bool al = rtm_aligned(p, nc);
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int i = i0 + 8 * h, e = 2 * h;
-    if (i >= p.nh) continue;
-    const bool pair = i < p.nth / 2;
-    double* outN = p.rtm_b + rtm_off(p, m, i, r, nc);
-    double* outS = p.rtm_b + rtm_off(p, m, p.nth - 1 - i, r, nc);
-    // two components x, y: [sym, asym] tiles -> one record sector of each hemisphere
-    auto put = [&](int q, const double(&x)[2][4], const double(&y)[2][4]) {
-      const int o = rtm_pair(p, m, q, nc);
-      if (pair) {
-        st_sector(outN + o, al, x[0][e] + x[1][e], x[0][e + 1] + x[1][e + 1], y[0][e] + y[1][e], y[0][e + 1] + y[1][e + 1]);
-        st_sector(outS + o, al, x[0][e] - x[1][e], x[0][e + 1] - x[1][e + 1], y[0][e] - y[1][e], y[0][e + 1] - y[1][e + 1]);
-      } else {
-        st_sector(outN + o, al, x[0][e], x[0][e + 1], y[0][e], y[0][e + 1]);
+  for (int u = 0; u < RB; ++u) {
+    const int r = kRB * (rb0 + rbi + 2 * u) + t;
+    if (rbi + 2 * u >= nrb_here || r >= p.nr) continue;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int i = th0 + 16 * tg + 8 * h + g, e = 2 * h;
+      if (i >= p.nh) continue;
+      const bool pair = i < p.nth / 2;
+      const double ms = (double)m * p.asin_t[i];
+      double* outN = p.rtm_b + rtm_off(p, m, i, r, nc);
+      double* outS = p.rtm_b + rtm_off(p, m, p.nth - 1 - i, r, nc);
+      // (sym, asym) of two components -> one record sector of each hemisphere
+      auto put = [&](int q, const double(&sy)[4], const double(&as)[4]) {
+        const int o = rtm_pair(p, m, q, nc);
+        if (pair) {
+          st_sector(outN + o, al, sy[0] + as[0], sy[1] + as[1], sy[2] + as[2], sy[3] + as[3]);
+          st_sector(outS + o, al, sy[0] - as[0], sy[1] - as[1], sy[2] - as[2], sy[3] - as[3]);
+        } else {
+          st_sector(outN + o, al, sy[0], sy[1], sy[2], sy[3]);
+        }
+      };
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        double sy[4], as[4];
+        cross_terms([&](int tile, int par, int slot) { return acc[u][v][tile][par][e + slot]; }, ms, sy, as);
+        put(v0 + v, sy, as);
       }
-    };
+      // radial components and scalars, two list entries per pair (v0 is even; the
+      // scalars follow the last group's vectors)
+      constexpr int NF = NV + NS;
 #pragma unroll
-    for (int v = 0; v < NV; ++v) put(v0 + v, acc[v][1], acc[v][2]);
-    // radial components and scalars, two list entries per pair (v0 is even; the
-    // scalars follow the last group's vectors)
-    constexpr int NF = NV + NS;
+      for (int f = 0; f < NF; f += 2) {
+        double sy[4] = {0.0, 0.0, 0.0, 0.0}, as[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-    for (int f = 0; f < NF; f += 2) {
-      const double(&x)[2][4] = f < NV ? acc[f < NV ? f : 0][0] : accS[f < NV ? 0 : f - NV];
-      if (f + 1 < NF) {
-        const double(&y)[2][4] = f + 1 < NV ? acc[f + 1 < NV ? f + 1 : 0][0] : accS[f + 1 < NV ? 0 : (f + 1 < NF ? f + 1 - NV : 0)];
-        put(p.nvb + (v0 + f) / 2, x, y);
-      } else {  // odd count: the last pair holds one component
-        const int o = rtm_pair(p, m, p.nvb + (v0 + f) / 2, nc);
-        *reinterpret_cast<double2*>(outN + o) =
-            pair ? make_double2(x[0][e] + x[1][e], x[0][e + 1] + x[1][e + 1]) : make_double2(x[0][e], x[0][e + 1]);
-        if (pair) *reinterpret_cast<double2*>(outS + o) = make_double2(x[0][e] - x[1][e], x[0][e + 1] - x[1][e + 1]);
+        for (int k = 0; k < 2; ++k) {
+          const int ff = f + k;
+          if (ff >= NF) break;
+          const double(&c)[2][4] = ff < NV ? acc[u][ff < NV ? ff : 0][4] : accS[u][ff < NV ? 0 : ff - NV];
+          sy[2 * k] = c[0][e];
+          sy[2 * k + 1] = c[0][e + 1];
+          as[2 * k] = c[1][e];
+          as[2 * k + 1] = c[1][e + 1];
+        }
+        if (f + 1 < NF) {
+          put(p.nvb + (v0 + f) / 2, sy, as);
+        } else {  // odd count: the last pair holds one component
+          const int o = rtm_pair(p, m, p.nvb + (v0 + f) / 2, nc);
+          *reinterpret_cast<double2*>(outN + o) =
+              pair ? make_double2(sy[0] + as[0], sy[1] + as[1]) : make_double2(sy[0], sy[1]);
+          if (pair) *reinterpret_cast<double2*>(outS + o) = make_double2(sy[0] - as[0], sy[1] - as[1]);
+        }
       }
     }
   }
 }
 
+// One launch for every group: nfull groups of two vectors, then the last one of
+// NV vectors with the scalars.  The groups of one (m, latitudes) are neighbours
+// in the grid: they read the same P and dP (once from HBM at large L).
 template <int NV, int NS>
-cudaError_t run_bwd16(const Plan& p, cudaStream_t s, int v0, int s0) {
-  auto kern = k_leg_bwd16<NV, NS>;
-  const size_t smem = Bwd16Geo<NV, NS>::SMEM;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  const long long nblk = (long long)(p.L + 1) * (p.nh_pad / kThBlk) * ((win_nrb(p) + 1) / 2);
-  if (nblk <= 0) return cudaSuccess;
-  kern<<<(unsigned)nblk, kThreads, smem, s>>>(p, v0, s0);
-  return cudaGetLastError();
+__global__ void __launch_bounds__(kThreads, 1) k_leg_bwd16(const __grid_constant__ Plan p, int nfull) {
+  extern __shared__ double sm[];
+  const int full = Bwd16Geo<2, 0>::radial_ctas(p), last = Bwd16Geo<NV, NS>::radial_ctas(p);
+  const int per = nfull * full + last, x = blockIdx.x % per, y = blockIdx.x / per;
+  const int nthb = p.nh_pad / kThBlk, m = y / nthb, th0 = (y - m * nthb) * kThBlk;
+  if (x < nfull * full) bwd16_group<2, 0>(p, sm, m, th0, x % full, 2 * (x / full));
+  else bwd16_group<NV, NS>(p, sm, m, th0, x - nfull * full, 2 * nfull);
 }
 
-// Field groups of the stored-table kernels: two vectors while more than three
-// are left, then the rest with the scalars; fn(nv, ns, v0) launches one group.
-template <typename F>
-cudaError_t for_groups(int nvec, int nscl, F fn) {
+template <int NV, int NS>
+cudaError_t run_bwd16(const Plan& p, cudaStream_t s) {
+  auto kern = k_leg_bwd16<NV, NS>;
+  const int nfull = (p.nvb - NV) / 2;
+  const size_t smem = std::max(nfull ? Bwd16Geo<2, 0>::SMEM : 0, Bwd16Geo<NV, NS>::SMEM);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  const long long nblk = (long long)(p.L + 1) * (p.nh_pad / kThBlk) *
+                         (nfull * Bwd16Geo<2, 0>::radial_ctas(p) + Bwd16Geo<NV, NS>::radial_ctas(p));
+  if (nblk <= 0) return cudaSuccess;
+  kern<<<(unsigned)nblk, kThreads, smem, s>>>(p, nfull);
+  return cudaGetLastError();
+}
+cudaError_t run_bwd16(const Plan& p, cudaStream_t s) {  // at least one vector
+  switch ((p.nvb % 2 ? 1 : 2) * 3 + p.nsb) {
+    case 3: return run_bwd16<1, 0>(p, s);
+    case 4: return run_bwd16<1, 1>(p, s);
+    case 5: return run_bwd16<1, 2>(p, s);
+    case 6: return run_bwd16<2, 0>(p, s);
+    case 7: return run_bwd16<2, 1>(p, s);
+    case 8: return run_bwd16<2, 2>(p, s);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+// Field groups of the forward kernel: two vectors while more than three are left,
+// then the rest with the scalars.
+cudaError_t run_fwd16(const Plan& p, double* d_rj, long long ld, const int* cols, cudaStream_t s, int m_count) {
+  auto group = [&](int nv, int ns, int v0) -> cudaError_t {
+    switch (nv * 3 + ns) {
+      case 1: return run_fwd16<0, 1>(p, d_rj, ld, cols, s, m_count, v0, 0);
+      case 2: return run_fwd16<0, 2>(p, d_rj, ld, cols, s, m_count, v0, 0);
+      case 3: return run_fwd16<1, 0>(p, d_rj, ld, cols, s, m_count, v0, 0);
+      case 4: return run_fwd16<1, 1>(p, d_rj, ld, cols, s, m_count, v0, 0);
+      case 5: return run_fwd16<1, 2>(p, d_rj, ld, cols, s, m_count, v0, 0);
+      case 6: return run_fwd16<2, 0>(p, d_rj, ld, cols, s, m_count, v0, 0);
+      case 7: return run_fwd16<2, 1>(p, d_rj, ld, cols, s, m_count, v0, 0);
+      case 8: return run_fwd16<2, 2>(p, d_rj, ld, cols, s, m_count, v0, 0);
+      case 9: return run_fwd16<3, 0>(p, d_rj, ld, cols, s, m_count, v0, 0);
+      case 10: return run_fwd16<3, 1>(p, d_rj, ld, cols, s, m_count, v0, 0);
+      case 11: return run_fwd16<3, 2>(p, d_rj, ld, cols, s, m_count, v0, 0);
+      default: return cudaErrorInvalidValue;
+    }
+  };
   cudaError_t e = cudaSuccess;
   int v0 = 0;
   do {
-    const int nv = nvec - v0 <= 3 ? nvec - v0 : 2;
-    e = fn(nv, v0 + nv == nvec ? nscl : 0, v0);
+    const int nv = p.nvf - v0 <= 3 ? p.nvf - v0 : 2;
+    e = group(nv, v0 + nv == p.nvf ? p.nsf : 0, v0);
     v0 += nv;
-  } while (e == cudaSuccess && v0 < nvec);
+  } while (e == cudaSuccess && v0 < p.nvf);
   return e;
-}
-#define KMHD_GROUP(NVv, NSv, FN, ...)             \
-  switch ((NVv)*3 + (NSv)) {                      \
-    case 1: return FN<0, 1>(__VA_ARGS__);         \
-    case 2: return FN<0, 2>(__VA_ARGS__);         \
-    case 3: return FN<1, 0>(__VA_ARGS__);         \
-    case 4: return FN<1, 1>(__VA_ARGS__);         \
-    case 5: return FN<1, 2>(__VA_ARGS__);         \
-    case 6: return FN<2, 0>(__VA_ARGS__);         \
-    case 7: return FN<2, 1>(__VA_ARGS__);         \
-    case 8: return FN<2, 2>(__VA_ARGS__);         \
-    case 9: return FN<3, 0>(__VA_ARGS__);         \
-    case 10: return FN<3, 1>(__VA_ARGS__);        \
-    case 11: return FN<3, 2>(__VA_ARGS__);        \
-    default: return cudaErrorInvalidValue;        \
-  }
-cudaError_t run_bwd16(const Plan& p, cudaStream_t s) {
-  return for_groups(p.nvb, p.nsb, [&](int nv, int ns, int v0) -> cudaError_t { KMHD_GROUP(nv, ns, run_bwd16, p, s, v0, 0); });
-}
-
-cudaError_t run_fwd16(const Plan& p, double* d_rj, long long ld, const int* cols, cudaStream_t s, int m_count) {
-  return for_groups(p.nvf, p.nsf, [&](int nv, int ns, int v0) -> cudaError_t {
-    KMHD_GROUP(nv, ns, run_fwd16, p, d_rj, ld, cols, s, m_count, v0, 0);
-  });
 }
 
 template <int NV, int NS, bool OTF>
@@ -1147,14 +1204,23 @@ cudaError_t launch_pack_b(const Plan& p, int nlc_max, const double* d_rj, long l
   KMHD_DISPATCH(nv, ns, run_pack, p, nlc_max, d_rj, ld, cols, s);
 }
 
+static int sm_count() {
+  int dev = 0, n = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  return n;
+}
+
 cudaError_t launch_leg_bwd_f64(const Plan& p, cudaStream_t s) {
-  // The 16-latitude kernel takes a whole SM per CTA: it wins when there are
-  // enough CTAs and at least two vectors to share a chunk's operands.  ms old ->
-  // new: L = 255, Nr = 129 3.19 -> 2.64; L = 511, Nr = 17 3.24 -> 2.91; L = 127,
-  // Nr = 17 (768 CTAs) 0.109 -> 0.092; but L = 31, Nr = 33 (160) 0.016 -> 0.019,
-  // L = 63, Nr = 9 (128) 0.018 -> 0.020, one vector at L = 255, Nr = 33 0.309 -> 0.322.
+  // The 16-row kernel takes a whole SM per CTA: it wins when there are two CTAs
+  // (of eight radii) for each and at least two vectors to share a chunk's
+  // operands.  ms 8-row -> 16-row: L = 255, Nr = 129 3.19 -> 2.72; L = 511, Nr = 17
+  // 3.24 -> 3.08; L = 127, Nr = 17 (768 CTAs) 0.109 -> 0.101; but L = 31, Nr = 33
+  // (160) 0.016 -> 0.019, L = 63, Nr = 9 (128) 0.018 -> 0.020, one vector at
+  // L = 255, Nr = 33 0.309 -> 0.322.  The launch is a window or slab of the shell
+  // as often as not; the results are the same on both sides.
   const long long ctas = (long long)(p.L + 1) * (p.nh_pad / kThBlk) * ((win_nrb(p) + 1) / 2);
-  if (!p.otf && p.nvb >= 2 && ctas >= 2 * 148) return run_bwd16(p, s);
+  if (!p.otf && p.nvb >= 2 && ctas >= 2 * sm_count()) return run_bwd16(p, s);
   KMHD_DISPATCH(p.nvb, p.nsb, run_bwd, p, s);
 }
 
@@ -1168,7 +1234,7 @@ cudaError_t launch_leg_fwd_f64(const Plan& p, double* d_rj, long long ld, const 
   // 0.142, Nr = 129 3.94 -> 3.62; L = 1023, Nr = 17 29.0 -> 25.9; the same at L = 95
   // and 106; but L = 63, Nr = 33 0.051 -> 0.065 (most warps without a degree).
   const long long ctas = (long long)((kcount(p.L, 0, 0) + kLB16 - 1) / kLB16) * win_nrb(p) * m_count;
-  if (!p.otf && p.L >= 112 && ctas >= 148) return run_fwd16(p, d_rj, ld, cols, s, m_count);
+  if (!p.otf && p.L >= 112 && ctas >= sm_count()) return run_fwd16(p, d_rj, ld, cols, s, m_count);
   KMHD_DISPATCH(p.nvf, p.nsf, run_fwd, p, d_rj, ld, cols, s, m_count);
 }
 
