@@ -176,7 +176,7 @@ struct Seqs {
 // line: the line's block rows, bs doubles apart (staged: rtm_row; in place in
 // rtm: rtm_row nr nth).
 // src: where the pair's components are; two: it holds two.
-__device__ __forceinline__ double2 spec_at(const Plan& P, const double* line, long long bs, const PairSrc& src, bool two,
+__device__ __forceinline__ double2 spec_at(const Plan& P, const double* line, long long bs, const PairPos& src, bool two,
                                            int k) {
   // no branch around the loads: a butterfly's loads go out together (zero-band
   // frequencies load order 0)
@@ -323,7 +323,7 @@ __device__ __forceinline__ void dif_first(const Seqs Z, const Plan& P, const dou
     const int pp = it / s, j = it - pp * s;
     double2 x[R];
     const int q = q0 + pp * dq;
-    const PairSrc src(P, q, nc, bwd_in_order(P.nvb, P.nsb));
+    const PairPos src(P, q, nc, P.nvb, P.mixb);
 #pragma unroll
     for (int r = 0; r < R; ++r) x[r] = spec_at(P, line + pp * ls, bs, src, 2 * q + 1 < nc, j + r * s);
     DFT<R, +1>::run(x);
@@ -420,7 +420,19 @@ __device__ void prefetch_line(double* st, const double* rtm, int nc, const Plan&
   cp_async_commit();
 }
 
-// Record sector of order m from the natural-order forward spectrum of one pair:
+// Forward records of one order of a pair: (a0, b0) of its first component at dx,
+// (a1, b1) of its second at dy (two: it has one; split: not the same sector; al: sectors are aligned).
+__device__ __forceinline__ void store_rec(double* dx, double* dy, bool two, bool split, bool al, double a0, double b0,
+                                          double a1, double b1) {
+  if (two && !split) {
+    st_sector(dx, al, a0, b0, a1, b1);
+  } else {
+    *reinterpret_cast<double2*>(dx) = make_double2(a0, b0);
+    if (two) *reinterpret_cast<double2*>(dy) = make_double2(a1, b1);
+  }
+}
+
+// Records of order m from the natural-order forward spectrum of one pair:
 // zm = z[m], wm = z[N - m].
 __device__ __forceinline__ void store_pair(double* base, long long bs, const Plan& P, int m, int pp, int nc, bool al,
                                            double2 zm, double2 wm) {
@@ -434,9 +446,9 @@ __device__ __forceinline__ void store_pair(double* base, long long bs, const Pla
     a1 = (zm.y + wm.y) * aN;
     b1 = (zm.x - wm.x) * aN;
   }
-  double* d = base + (m >> P.mbs) * bs + rtm_pair(P, m, pp, nc);
-  if (2 * pp + 1 < nc) st_sector(d, al, a0, b0, a1, b1);
-  else *reinterpret_cast<double2*>(d) = make_double2(a0, b0);
+  const PairPos dst(P, pp, nc, P.nvf, P.mixf);
+  double* d = base + (m >> P.mbs) * bs;
+  store_rec(d + dst.x(m), d + dst.y(m), 2 * pp + 1 < nc, dst.split, al, a0, b0, a1, b1);
 }
 
 // Natural-order forward spectra of the sequences -> records: sequence i is pair
@@ -509,7 +521,8 @@ __device__ __forceinline__ void point_products(const double* rr, const double* t
 }
 
 // Product lists known at compile time (vector-valued products first): the
-// field sets of the reference's MHD, convection and heat runs.  PK = 0: the
+// field sets of the reference's MHD, convection and heat runs.  Where they have a
+// mixed forward pair its scalar is a dot product (Plan::mixf = -1).  PK = 0: the
 // plan's list, read at run time.
 constexpr int kX = KMHD_PROD_CROSS, kVS = KMHD_PROD_VEC_SCALAR, kDot = KMHD_PROD_DOT;
 struct ProdList {
@@ -565,7 +578,7 @@ __device__ __forceinline__ void point_products_k(const double* rr, const double*
 }
 
 // Pointwise products on the digit-reversed grid (sequence zs entries apart),
-// backward pairs in, forward pairs out (pair and list order: see rtm_off); PK: the
+// backward pairs in, forward pairs out (pairs: see rtm_off, mixed_pair); PK: the
 // product list (0: the plan's).
 template <int PK>
 __device__ __forceinline__ void products(double2* z, int zs, int N, const Plan& P) {
@@ -573,6 +586,7 @@ __device__ __forceinline__ void products(double2* z, int zs, int N, const Plan& 
   constexpr int MVB = PK ? q.nvb : kMaxVec, MSB = PK ? q.nsb : kMaxScl, MVF = PK ? q.nvf : kMaxVec,
                 MSF = PK ? q.nsf : kMaxScl;
   const int nvb = PK ? MVB : P.nvb, nsb = PK ? MSB : P.nsb, nvf = PK ? MVF : P.nvf, nsf = PK ? MSF : P.nsf;
+  const bool mixb = PK ? mixed_pair(MVB, MSB) >= 0 : P.mixb >= 0, mixf = PK ? false : P.mixf >= 0;
   for (int pos = threadIdx.x; pos < N; pos += blockDim.x) {
     constexpr int VB = MVB > 0 ? MVB : 1, SB = MSB > 0 ? MSB : 1, VF = MVF > 0 ? MVF : 1, SF = MSF > 0 ? MSF : 1;
     double rr[VB] = {}, th[VB] = {}, ph[VB] = {}, sc[SB] = {};
@@ -583,26 +597,23 @@ __device__ __forceinline__ void products(double2* z, int zs, int N, const Plan& 
     for (int v = 0; v < MVB; ++v)
       if (v < nvb) {
         const double2 w = z[v * zs + pos];
-        rr[v] = *entry(nvb, v);
-        th[v] = w.x;
+        const double e = *entry(nvb, v);
+        const bool sp = mixb && v == nvb - 1;  // (r, phi), (theta, scalar)
+        rr[v] = sp ? w.x : e;
+        th[v] = sp ? e : w.x;
         ph[v] = w.y;
       }
 #pragma unroll
     for (int k = 0; k < MSB; ++k)
       if (k < nsb) sc[k] = *entry(nvb, nvb + k);
-    if (bwd_in_order(nvb, nsb)) {  // (r, theta), (phi, scalar)
-      const double2 w = z[pos];
-      rr[0] = w.x;
-      th[0] = w.y;
-      ph[0] = *entry(nvb, 0);
-    }
     if constexpr (PK > 0) point_products_k<PK>(rr, th, ph, sc, P, orr, oth, oph, os);
     else point_products<MVB, MSB, MVF, MSF, false>(rr, th, ph, sc, P, orr, oth, oph, os);
 #pragma unroll
     for (int v = 0; v < MVF; ++v)
       if (v < nvf) {
-        z[v * zs + pos] = make_double2(oth[v], oph[v]);
-        *entry(nvf, v) = orr[v];
+        const bool sp = mixf && v == nvf - 1;
+        z[v * zs + pos] = make_double2(sp ? orr[v] : oth[v], oph[v]);
+        *entry(nvf, v) = sp ? oth[v] : orr[v];
       }
 #pragma unroll
     for (int k = 0; k < MSF; ++k)
@@ -708,8 +719,10 @@ __global__ void __launch_bounds__(kFftThreads) k_fft_cycle_wide(const __grid_con
 
 constexpr int kGridThreads = 256;  // separable kernels: at most, at 128 registers
 
-// Component of part c (0, 1) of pair pp (the inverse of comp_pair).
-__device__ __forceinline__ int pair_comp(int pp, int c, int nv) {
+// Component of part c (0, 1) of FFT pair pp (mixed: see mixed_pair).
+__device__ __forceinline__ int pair_comp(int pp, int c, int nv, int mixed) {
+  if (mixed >= 0 && pp == nv - 1) return 3 * pp + 2 * c;
+  if (pp == mixed) return c ? 3 * nv : 3 * nv - 2;
   if (pp < nv) return 3 * pp + 1 + c;
   const int f = 2 * (pp - nv) + c;
   return f < nv ? 3 * f : 2 * nv + f;
@@ -738,9 +751,9 @@ __global__ void __launch_bounds__(kGridThreads, 2)
   dif_rest(Z, P);
   const long long nnod = (long long)P.nr * P.nth * N;
   const bool two = 2 * q + 1 < P.ncb;
-  const bool inorder = bwd_in_order(P.nvb, P.nsb);
-  double* f0 = fld + nnod * (inorder ? 2 * q : pair_comp(q, 0, P.nvb)) + r0 + (long long)P.nr * th;
-  double* f1 = two ? fld + nnod * (inorder ? 2 * q + 1 : pair_comp(q, 1, P.nvb)) + r0 + (long long)P.nr * th : nullptr;
+  const int mixed = P.mixb;
+  double* f0 = fld + nnod * pair_comp(q, 0, P.nvb, mixed) + r0 + (long long)P.nr * th;
+  double* f1 = two ? fld + nnod * pair_comp(q, 1, P.nvb, mixed) + r0 + (long long)P.nr * th : nullptr;
   const long long ps = (long long)P.nr * P.nth;
 #pragma unroll 4
   for (int it = threadIdx.x; it < N << lrad; it += blockDim.x) {
@@ -763,8 +776,9 @@ __global__ void __launch_bounds__(kGridThreads, 2)
   const Seqs Z(reinterpret_cast<double2*>(smraw), nrad, N + 1, N);
   const long long nnod = (long long)P.nr * P.nth * N;
   const bool two = 2 * q + 1 < P.ncf;
-  const double* __restrict__ f0 = frc + nnod * pair_comp(q, 0, P.nvf) + r0 + (long long)P.nr * th;
-  const double* __restrict__ f1 = two ? frc + nnod * pair_comp(q, 1, P.nvf) + r0 + (long long)P.nr * th : nullptr;
+  const int mixed = P.mixf;
+  const double* __restrict__ f0 = frc + nnod * pair_comp(q, 0, P.nvf, mixed) + r0 + (long long)P.nr * th;
+  const double* __restrict__ f1 = two ? frc + nnod * pair_comp(q, 1, P.nvf, mixed) + r0 + (long long)P.nr * th : nullptr;
   const long long ps = (long long)P.nr * P.nth;
   // eight grid loads of a thread in flight
   constexpr int U = 4;
@@ -872,7 +886,7 @@ struct DFT2F_ZM<3, B, SIGN> {
 // inputs (L < k < N - L) is zero and the outer thirds need no range checks.
 // line / bs: the line's block rows, staged or in place (see spec_at).
 template <int N, bool PR, bool INPLACE = false>
-__device__ __forceinline__ void ff_dif_first(const Plan& P, const double* line, long long bs, int nc, bool inorder,
+__device__ __forceinline__ void ff_dif_first(const Plan& P, const double* line, long long bs, int nc, int nv, int mixed,
                                              double2* z, int npair, const double2* __restrict__ tw) {
   constexpr int R = ff_first(N), S1 = N / R, NP = N + 1, T3 = R / 3;
   for (int it = threadIdx.x; it < npair * S1; it += blockDim.x) {
@@ -886,12 +900,13 @@ __device__ __forceinline__ void ff_dif_first(const Plan& P, const double* line, 
       // whole block rows apart.
       static_assert(S1 % kRtmOrders == 0, "orders per rtm block");
       const bool two = 2 * pp + 1 < nc;  // the pair holds two components
-      const PairSrc src(P, pp, nc, inorder);
+      const PairPos src(P, pp, nc, nv, mixed);
       int ux = src.x(j), uy = src.y(j), dx = src.x(-j), dy = src.y(-j);
       const double* up = line + (j >> kRtmShift) * bs;
       const double* dn = line + ((-j) >> kRtmShift) * bs;
       // staged sectors lie 32 bytes apart: lanes 4..7 of each eight read the
-      // second half first, so a quarter warp covers all banks
+      // second half first, so a quarter warp covers all banks (a split pair's
+      // components are the two halves of two sectors)
       const bool hu = !INPLACE && two && (j & 4), hd = !INPLACE && two && ((-j) & 4);
       if (!two) uy = ux, dy = dx;
       const int u0 = hu ? uy : ux, u1 = hu ? ux : uy, d0 = hd ? dy : dx, d1 = hd ? dx : dy;
@@ -923,7 +938,7 @@ __device__ __forceinline__ void ff_dif_first(const Plan& P, const double* line, 
       }
       DFT2F_ZM<3, T3, +1>::run(x);
     } else {
-      const PairSrc src(P, pp, nc, inorder);
+      const PairPos src(P, pp, nc, nv, mixed);
 #pragma unroll
       for (int r = 0; r < R; ++r) x[r] = spec_at(P, line, bs, src, 2 * pp + 1 < nc, j + r * S1);
       DFT<R, +1>::run(x);
@@ -955,7 +970,7 @@ __device__ __forceinline__ void ff_dif_first(const Plan& P, const double* line, 
 // mirrors.
 template <int N, bool PR>
 __device__ __forceinline__ void ff_dit_store(const double2* z, int npair, const Plan& P, double* base, long long bs,
-                                             int nc, const double2* __restrict__ tw) {
+                                             int nc, int nv, int mixed, const double2* __restrict__ tw) {
   constexpr int R = ff_first(N), S1 = N / R, NP = N + 1;
   constexpr int QM = PR ? R / 3 : (R + 1) / 2;  // orders j + q S1 <= L < N / 2 have q < QM
   static_assert(S1 == 64 || S1 == 16, "lane arrangement");
@@ -988,7 +1003,9 @@ __device__ __forceinline__ void ff_dit_store(const double2* z, int npair, const 
     }
     DFT<R, -1>::run(x);
     const bool two = 2 * pp + 1 < nc;
-    double* d = base + (j >> kRtmShift) * bs + pp * 4 * kRtmOrders + (j & (kRtmOrders - 1)) * (two ? 4 : 2);
+    const PairPos dst(P, pp, nc, nv, mixed);
+    double* dx = base + (j >> kRtmShift) * bs + dst.x(j);
+    double* dy = base + (j >> kRtmShift) * bs + dst.y(j);
     const double aN = 1.0 / (double)N;
 #pragma unroll
     for (int q = 0; q < QM; ++q) {
@@ -999,11 +1016,10 @@ __device__ __forceinline__ void ff_dit_store(const double2* z, int npair, const 
       const double2 zm = x[q];
       const bool m0 = q == 0 && j == 0;
       if (!ok || (!PR && j + q * S1 > L)) continue;
-      double* dq = d + (q * S1 / kRtmOrders) * bs;
+      const long long o = (q * S1 / kRtmOrders) * bs;
       const double a0 = m0 ? zm.x * aN : (zm.x + wm.x) * aN, b0 = m0 ? 0.0 : (wm.y - zm.y) * aN;
       const double a1 = m0 ? zm.y * aN : (zm.y + wm.y) * aN, b1 = m0 ? 0.0 : (zm.x - wm.x) * aN;
-      if (two) st_global_v4(dq, a0, b0, a1, b1);
-      else *reinterpret_cast<double2*>(dq) = make_double2(a0, b0);
+      store_rec(dx + o, dy + o, two, dst.split, true, a0, b0, a1, b1);
     }
   }
 }
@@ -1078,6 +1094,7 @@ __device__ __forceinline__ void ff_fused(double2* z, const Plan& P) {
   const int nvb = EX ? MVB : P.nvb, nvf = EX ? MVF : P.nvf;
   const int nlb = EX ? (FB + 1) / 2 : (P.nvb + P.nsb + 1) / 2, nlf = EX ? (FF + 1) / 2 : (P.nvf + P.nsf + 1) / 2;
   const int nff = EX ? FF : P.nvf + P.nsf;
+  const bool mixb = (EX ? mixed_pair(MVB, MSB) : P.mixb) >= 0, mixf = PK > 0 ? false : P.mixf >= 0;
   for (int b = threadIdx.x; b < N / 4; b += blockDim.x) {
     const int e0 = (4 * b) ^ (((b >> 1) ^ (b >> 4)) & 7);  // swf(4b + r) = e0 ^ r
     double2 v[NPM][4];
@@ -1098,17 +1115,12 @@ __device__ __forceinline__ void ff_fused(double2* z, const Plan& P) {
       double rr[VB] = {}, th[VB] = {}, ph[VB] = {}, sc[SB] = {};
       double orr[VF] = {}, oth[VF] = {}, oph[VF] = {}, os[SF] = {};
       auto lst = [&](int f) { return (f & 1) ? v[MVB + f / 2][r].y : v[MVB + f / 2][r].x; };
-      const bool inorder = EX ? bwd_in_order(MVB, MSB) : bwd_in_order(P.nvb, P.nsb);
 #pragma unroll
       for (int q = 0; q < MVB; ++q) {
-        rr[q] = lst(q);
-        th[q] = v[q][r].x;
+        const bool sp = mixb && q == nvb - 1;  // (r, phi), (theta, scalar)
+        rr[q] = sp ? v[q][r].x : lst(q);
+        th[q] = sp ? lst(q) : v[q][r].x;
         ph[q] = v[q][r].y;
-      }
-      if (MVB > 0 && MSB > 0 && inorder) {  // (r, theta), (phi, scalar)
-        rr[0] = v[0][r].x;
-        th[0] = v[0][r].y;
-        ph[0] = lst(0);
       }
 #pragma unroll
       for (int q = 0; q < MSB; ++q) {
@@ -1122,17 +1134,19 @@ __device__ __forceinline__ void ff_fused(double2* z, const Plan& P) {
       }
       if constexpr (PK > 0) point_products_k<PK>(rr, th, ph, sc, P, orr, oth, oph, os);
       else point_products<MVB, MSB, MVF, MSF, EX>(rr, th, ph, sc, P, orr, oth, oph, os);
-      // forward list entry f: r of a vector, scalar or (odd count) zero
+      // forward list entry f: r of a vector (theta in the mixed pair), scalar or (odd count) zero
       auto out = [&](int f) {
-        if (EX) return f < MVF ? orr[f < MVF ? f : 0] : f < FF ? os[f < MVF ? 0 : (f < FF ? f - MVF : 0)] : 0.0;
-        double x = f < nvf && f < MVF ? orr[f < MVF ? f : 0] : 0.0;
+        const int c = f < MVF ? f : 0;
+        const double ve = mixf && f == nvf - 1 ? oth[c] : orr[c];
+        if (EX) return f < MVF ? ve : f < FF ? os[f < MVF ? 0 : (f < FF ? f - MVF : 0)] : 0.0;
+        double x = f < nvf && f < MVF ? ve : 0.0;
 #pragma unroll
         for (int q = 0; q < MSF; ++q)
           if (f == nvf + q && f < nff) x = os[q];
         return x;
       };
 #pragma unroll
-      for (int q = 0; q < MVF; ++q) v[q][r] = make_double2(oth[q], oph[q]);
+      for (int q = 0; q < MVF; ++q) v[q][r] = make_double2(mixf && q == nvf - 1 ? orr[q] : oth[q], oph[q]);
 #pragma unroll
       for (int k = 0; k < (FF + 1) / 2; ++k) v[MVF + k][r] = make_double2(out(2 * k), out(2 * k + 1));
     }
@@ -1212,7 +1226,8 @@ __global__ void __launch_bounds__(NT, kFftThreadsF / NT)
   const int ncb = EX ? 3 * MVB + MSB : P.ncb, ncf = EX ? 3 * MVF + MSF : P.ncf;
   const int npb = (ncb + 1) / 2, npf = (ncf + 1) / 2;
   const int npair = npb > npf ? npb : npf;
-  const bool inorder = EX ? bwd_in_order(MVB, MSB) : bwd_in_order(P.nvb, P.nsb);
+  const int nvb = EX ? MVB : P.nvb, nvf = EX ? MVF : P.nvf;
+  const int mixb = EX ? mixed_pair(MVB, MSB) : P.mixb, mixf = PK > 0 ? -1 : P.mixf;
   double2* z = reinterpret_cast<double2*>(smraw);
   // staged spectra, 128-byte aligned, then the mbarrier
   double* st = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(z + npair * NP) + 127) & ~static_cast<uintptr_t>(127));
@@ -1227,7 +1242,8 @@ __global__ void __launch_bounds__(NT, kFftThreadsF / NT)
     __syncthreads();
     ff_mid_pass<N, -1>(z, npf, P.twid);
     __syncthreads();
-    ff_dit_store<N, PR>(z, npf, P, P.rtm_f + rtm_off(P, 0, th, r, ncf), (long long)P.nth * P.nr * (2 * kRtmOrders) * ncf, ncf, P.twid);
+    ff_dit_store<N, PR>(z, npf, P, P.rtm_f + rtm_off(P, 0, th, r, ncf),
+                        (long long)P.nth * P.nr * (2 * kRtmOrders) * ncf, ncf, nvf, mixf, P.twid);
     __syncthreads();
   };
   if constexpr (!STG) {
@@ -1239,7 +1255,7 @@ __global__ void __launch_bounds__(NT, kFftThreadsF / NT)
                      "r"(0), "r"(next % P.nth), "r"(next / P.nth), "r"(0)
                      : "memory");
       ff_dif_first<N, PR, true>(P, P.rtm_b + rtm_off(P, 0, th, r, ncb), (long long)P.nth * P.nr * row, ncb,
-                                inorder, z, npb, P.twid);
+                                nvb, mixb, z, npb, P.twid);
       __syncthreads();
       rest(th, r);
     }
@@ -1276,7 +1292,7 @@ __global__ void __launch_bounds__(NT, kFftThreadsF / NT)
       }
       return;
     }
-    ff_dif_first<N, PR>(P, st, row, ncb, inorder, z, npb, P.twid);
+    ff_dif_first<N, PR>(P, st, row, ncb, nvb, mixb, z, npb, P.twid);
     __syncthreads();
     const int next = line + gridDim.x;
     if (next < nlines) stage(next);
@@ -1298,7 +1314,7 @@ __global__ void __launch_bounds__(NT, kFftThreadsF / NT)
 // L = 1023, Nr = 17.  w_N^(h (j + r S1)) = w_N^(h j) w_48^r: the first factor is
 // common to a butterfly and goes into the twiddles, the second is compile-time.
 template <int NH, int H, bool PR>
-__device__ __forceinline__ void ff_half_first(const Plan& P, const double* line, long long bs, int nc, bool inorder,
+__device__ __forceinline__ void ff_half_first(const Plan& P, const double* line, long long bs, int nc, int nv, int mixed,
                                               double2* z, int npair) {
   constexpr int R = ff_first(NH), S1 = NH / R, NP = NH + 1;
   static_assert(R == 24 && S1 == 64, "w_48 rotations, whole block rows");
@@ -1307,7 +1323,7 @@ __device__ __forceinline__ void ff_half_first(const Plan& P, const double* line,
   for (int it = threadIdx.x; it < npair * S1; it += blockDim.x) {
     const int pp = it / S1, j = it - pp * S1;
     const bool two = 2 * pp + 1 < nc;
-    const PairSrc src(P, pp, nc, inorder);
+    const PairPos src(P, pp, nc, nv, mixed);
     const int ux = src.x(j), uy = src.y(j), dx = src.x(-j), dy = src.y(-j);
     const double* up = line + (j >> kRtmShift) * bs;
     const double* dn = line + ((-j) >> kRtmShift) * bs;
@@ -1353,7 +1369,7 @@ __device__ __forceinline__ void ff_half_first(const Plan& P, const double* line,
 // order m = j + q S1 takes X[N - m] from butterfly S1 - j, entry R - 1 - q).
 template <int NH, int H, bool PR>
 __device__ __forceinline__ void ff_half_store(const double2* z, int npair, const Plan& P, double2* __restrict__ sc,
-                                              double* base, long long bs, int nc) {
+                                              double* base, long long bs, int nc, int nv, int mixed) {
   constexpr int R = ff_first(NH), S1 = NH / R, NP = NH + 1;
   constexpr int QM = PR ? 2 * R / 3 : R;  // orders j + q S1 <= L < NH
   const double2* __restrict__ tw = P.twid;
@@ -1386,16 +1402,17 @@ __device__ __forceinline__ void ff_half_store(const double2* z, int npair, const
       };
       for_constants(turn, std::make_integer_sequence<int, R>{});
       const bool two = 2 * pp + 1 < nc;
-      double* d = base + (j >> kRtmShift) * bs + pp * 4 * kRtmOrders + (j & (kRtmOrders - 1)) * (two ? 4 : 2);
+      const PairPos dst(P, pp, nc, nv, mixed);
+      double* dx = base + (j >> kRtmShift) * bs + dst.x(j);
+      double* dy = base + (j >> kRtmShift) * bs + dst.y(j);
       const double aN = 1.0 / (double)(2 * NH);
       auto put = [&](int q, double2 zm, double2 wm) {
         if (!PR && j + q * S1 > L) return;
         const bool m0 = q == 0 && j == 0;
-        double* dq = d + (q * S1 / kRtmOrders) * bs;
+        const long long o = (q * S1 / kRtmOrders) * bs;
         const double c0 = m0 ? zm.x * aN : (zm.x + wm.x) * aN, s0 = m0 ? 0.0 : (wm.y - zm.y) * aN;
         const double c1 = m0 ? zm.y * aN : (zm.y + wm.y) * aN, s1 = m0 ? 0.0 : (zm.x - wm.x) * aN;
-        if (two) st_global_v4(dq, c0, s0, c1, s1);
-        else *reinterpret_cast<double2*>(dq) = make_double2(c0, s0);
+        store_rec(dx + o, dy + o, two, dst.split, true, c0, s0, c1, s1);
       };
       auto from_mate = [&](double2 v) {
         return make_double2(__shfl_sync(0xffffffffu, v.x, mate), __shfl_sync(0xffffffffu, v.y, mate));
@@ -1423,6 +1440,8 @@ __global__ void __launch_bounds__(kFftThreadsF, 1)
   extern __shared__ double4 smraw[];
   const int ncb = EX ? 3 * MVB + MSB : P.ncb, ncf = EX ? 3 * MVF + MSF : P.ncf;
   const int npb = (ncb + 1) / 2, npf = (ncf + 1) / 2;
+  const int nvb = EX ? MVB : P.nvb, nvf = EX ? MVF : P.nvf;
+  const int mixb = EX ? mixed_pair(MVB, MSB) : P.mixb, mixf = PK > 0 ? -1 : P.mixf;
   double2* z = reinterpret_cast<double2*>(smraw);
   double2* sc = P.fft_scratch + (long long)blockIdx.x * (npb > npf ? npb : npf) * P.nph;
   const long long bsb = (long long)P.nth * P.nr * (2 * kRtmOrders) * ncb, bsf = (long long)P.nth * P.nr * (2 * kRtmOrders) * ncf;
@@ -1437,7 +1456,7 @@ __global__ void __launch_bounds__(kFftThreadsF, 1)
     double* dst = P.rtm_f + rtm_off(P, 0, th, r, ncf);
     auto half = [&](auto hc) {
       constexpr int H = decltype(hc)::value;
-      ff_half_first<NH, H, PR>(P, src, bsb, ncb, EX ? bwd_in_order(MVB, MSB) : bwd_in_order(P.nvb, P.nsb), z, npb);
+      ff_half_first<NH, H, PR>(P, src, bsb, ncb, nvb, mixb, z, npb);
       __syncthreads();
       ff_mid_pass<NH, +1, 2>(z, npb, P.twid);
       __syncthreads();
@@ -1445,7 +1464,7 @@ __global__ void __launch_bounds__(kFftThreadsF, 1)
       __syncthreads();
       ff_mid_pass<NH, -1, 2>(z, npf, P.twid);
       __syncthreads();
-      ff_half_store<NH, H, PR>(z, npf, P, sc, dst, bsf, ncf);
+      ff_half_store<NH, H, PR>(z, npf, P, sc, dst, bsf, ncf, nvf, mixf);
       __syncthreads();
     };
     half(std::integral_constant<int, 0>());

@@ -30,6 +30,7 @@ constexpr long long kSelfTestSpinCap = 1ll << 16;  // bounded-wait rounds of the
 struct Plan {
   int L, nth, nph, nr, nh, nh_pad, nr4, nrb;
   int mbs;  // orders per rtm block, log2 (see rtm_off)
+  int mixb, mixf;  // FFT pairs that are not record pairs (see mixed_pair)
   // radial window [r_lo, r_hi) of the cycle launches (0, nr: every radius);
   // r_lo is a multiple of 16, so the window covers whole radial blocks and
   // whole split-GEMM column tiles
@@ -103,7 +104,7 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 
 // rtm records.  The nc components of one (m, theta, r) are taken in pairs, the
-// two real sequences that one complex longitudinal FFT carries: pair v < nv is
+// two real sequences that one complex longitudinal FFT carries (but see mixed_pair): pair v < nv is
 // (theta, phi) of vector v; pair nv + k is entries 2k, 2k + 1 of the list (r of
 // every vector, scalars).  One pair of one order is one 32-byte sector
 // (a_x, b_x, a_y, b_y) (cos, sin); with an odd component count the last pair is
@@ -126,41 +127,47 @@ __host__ __device__ __forceinline__ long long rtm_off(const Plan& P, int m, int 
 __host__ __device__ __forceinline__ int rtm_pair(const Plan& P, int m, int q, int nc) {
   return (q << (P.mbs + 2)) + (m & ((1 << P.mbs) - 1)) * (2 * q + 1 < nc ? 4 : 2);
 }
-// A backward set of one vector pairs its components in order for the FFT --
-// (r, theta), (phi, scalar), (scalar) -- instead of by sector: the two sequences
-// of a complex FFT share their rounding error, and u_r is larger than a scalar by
-// a factor of l, u_phi is not (u T at L = 333: 2.9e-15 against 5.0e-14).  Only
-// the reads of the first pass know: PairSrc, where pair pp's components start
-// inside order m's block row.
-__host__ __device__ __forceinline__ bool bwd_in_order(int nv, int ns) { return nv == 1 && ns >= 1; }
-struct PairSrc {
-  int x0, xp, y0, yp, msk;  // component x of order m starts at x0 + (m & msk) xp
-  __device__ __forceinline__ PairSrc(const Plan& P, int pp, int nc, bool in_order) {
-    const int qx = in_order && pp < 2 ? 1 - pp : pp, hx = in_order && pp == 1 ? 2 : 0;
-    const int qy = pp, hy = in_order && pp == 0 ? 0 : 2;
+// The two sequences of a complex FFT share their rounding error, and u_r is larger
+// than a scalar by a factor of l, u_theta is not.  So where a record pair holds r of
+// the last vector and the first scalar (an odd number of vectors), the FFT may take
+// the last vector's pair as (r, phi) and the mixed pair as (theta, scalar).  Only
+// the reads of the first inverse pass, the products and the stores of the last
+// forward pass know; the records stay as they are.
+// Backward always (Plan::mixb): T of the default set takes an error (2-norm) of 5.6,
+// 5.6, 21 and 21e-15 at L = 127, 255, 511 and 1023 from B_r, 0.9, 0.5, 1.5 and
+// 1.3e-15 from B_theta.
+// Forward (Plan::mixf) unless the scalar is a dot product, which is as large as a
+// cross product's r: u T's columns at L = 511 have 18.2, 3.0 and 5.8e-15 with
+// (r, u . omega) in one FFT, 18.0, 15.4 and 28.5e-15 with (phi, u . omega), and the two
+// half sectors of each store cost 5% of the FFT's time.
+// The mixed pair's index, -1 without one.
+__host__ __device__ __forceinline__ constexpr int mixed_pair(int nv, int ns) {
+  return (nv & 1) && ns > 0 ? nv + (nv >> 1) : -1;
+}
+inline void set_mixed_pairs(Plan& P) {
+  P.mixb = mixed_pair(P.nvb, P.nsb);
+  P.mixf = P.nprod > 0 && P.pkind[P.nvf] == KMHD_PROD_DOT ? -1 : mixed_pair(P.nvf, P.nsf);
+}
+// Where the two components of FFT pair pp lie inside the block row of order m:
+// at x(m) and y(m); split: not in one sector.
+struct PairPos {
+  int x0, y0, stride, msk;
+  bool split;
+  __device__ __forceinline__ PairPos(const Plan& P, int pp, int nc, int nv, int mixed) {
+    const bool last = mixed >= 0 && pp == nv - 1, mix = pp == mixed;
+    split = last || mix;
+    const int qx = last ? mixed : mix ? nv - 1 : pp;
     msk = (1 << P.mbs) - 1;
-    x0 = (qx << (P.mbs + 2)) + hx;
-    xp = 2 * qx + 1 < nc ? 4 : 2;
-    y0 = (qy << (P.mbs + 2)) + hy;
-    yp = xp;
+    stride = 2 * qx + 1 < nc ? 4 : 2;
+    x0 = qx << (P.mbs + 2);
+    y0 = (pp << (P.mbs + 2)) + 2;
   }
-  __device__ __forceinline__ int x(int m) const { return x0 + (m & msk) * xp; }
-  __device__ __forceinline__ int y(int m) const { return y0 + (m & msk) * yp; }
+  __device__ __forceinline__ int x(int m) const { return x0 + (m & msk) * stride; }
+  __device__ __forceinline__ int y(int m) const { return y0 + (m & msk) * stride; }
 };
 // doubles of all records of one direction
 __host__ __device__ __forceinline__ size_t rtm_size(const Plan& P, int nc) {
   return (size_t)rtm_blocks(P) * P.nr * P.nth * rtm_row(P, nc);
-}
-// pair and part (0: x, 1: y) of component c (three per vector, then scalars)
-__host__ __device__ __forceinline__ int comp_pair(int c, int nv, int* part) {
-  if (c < 3 * nv) {
-    const int v = c / 3, q = c - 3 * v;
-    *part = q == 0 ? (v & 1) : q - 1;
-    return q == 0 ? nv + (v >> 1) : v;
-  }
-  const int f = c - 2 * nv;  // list entry nv + (c - 3 nv)
-  *part = f & 1;
-  return nv + (f >> 1);
 }
 // 32-byte sectors are aligned unless one-order blocks hold an odd count
 __host__ __device__ __forceinline__ bool rtm_aligned(const Plan& P, int nc) { return ((nc << P.mbs) & 1) == 0; }

@@ -172,6 +172,7 @@ int na_plan(const kmhd_sph_desc* d, Plan& p, NaHost& H) {
       p.pcoef[p.nprod] = q.coef;
       ++p.nprod;
     }
+  set_mixed_pairs(p);
   return KMHD_OK;
 }
 

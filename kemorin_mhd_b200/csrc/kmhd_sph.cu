@@ -399,6 +399,7 @@ int kmhd_sph_create(const kmhd_sph_desc* d, kmhd_sph** out) {
       p.pcoef[p.nprod] = q.coef;
       ++p.nprod;
     }
+  set_mixed_pairs(p);
 
   // ---- device allocations
   const size_t nP = (size_t)po, nSB = (size_t)so;
