@@ -135,15 +135,22 @@ __device__ __forceinline__ double2 twd(const double2* __restrict__ tw, int idx) 
 }
 
 // Twiddles w^(j q), q = 0, 1, ..., of one radix-R butterfly (w = e^{2 pi i / N})
-// with a table load every eighth q only: a running product w^(j q) =
-// w^(j (q - 1)) w^j, restarted from the table at q = 8, 16, ..., so at most
-// seven products separate a twiddle from a table value (within 2e-15 of
-// e^{2 pi i j q / N} for N = 48 .. 3072, checked against exact values).
-// Used by the first and last passes of the specialised kernels, whose lanes
-// read 32 different table entries per load (at L = 511 the FFT kernel takes
-// 20.6 ms this way, 21.7 ms restarting every fourth q, 23.5 ms loading every
-// twiddle).
-template <int SIGN>
+// with a table load every K-th q only: a running product w^(j q) = w^(j (q - 1)) w^j,
+// restarted from the table at q = K, 2 K, ..., so at most K - 1 products separate
+// a twiddle from a table value (K = 8: within 2e-15 of e^{2 pi i j q / N} for
+// N = 48 .. 3072, checked against exact values).
+// K = 8 in the first and last passes of the specialised kernels, whose lanes
+// read 32 different table entries per load (at L = 511 an FFT kernel of 20.6 ms
+// took 21.7 ms restarting every fourth q, 23.5 ms loading every twiddle; that
+// kernel has since been rebuilt).
+// K = 4 in the run-time passes and at N = 3072.  One frequency alone (b_trans, rms in
+// 2^-53 at N = 384, 450, 768): 0.76, 0.85, 0.76; with K = 8 1.05, 1.07, 1.01, with every
+// twiddle from the table 0.64, 0.78, 0.65.  What T of the default set takes from its
+// partner at L = 127: 5.2e-16, 8.5e-16, 4.6e-16; smooth spectra show no difference
+// between K = 4 and the table.  The table alone costs 6 to 7% of a separable
+// transform at L = 127 (0.78 -> 0.83 ms), K = 4 less than 1%.
+constexpr int kTwSpecial = 8, kTwRun = 4;
+template <int SIGN, int K>
 struct TwiddleRun {
   const double2* tw;
   int j;
@@ -154,7 +161,7 @@ struct TwiddleRun {
   }
   // w^(j q) for the next q (called for q = 1, 2, ... in order)
   __device__ __forceinline__ double2 next(int q) {
-    cur = (q & 7) == 0 ? twd<SIGN>(tw, j * q) : (q == 1 ? w1 : cmul(cur, w1));
+    cur = q % K == 0 ? twd<SIGN>(tw, j * q) : (q == 1 ? w1 : cmul(cur, w1));
     return cur;
   }
 };
@@ -328,7 +335,7 @@ __device__ __forceinline__ void dif_first(const Seqs Z, const Plan& P, const dou
     for (int r = 0; r < R; ++r) x[r] = spec_at(P, line + pp * ls, bs, src, 2 * q + 1 < nc, j + r * s);
     DFT<R, +1>::run(x);
     double2* base = Z.z + pp * Z.zs;
-    TwiddleRun<+1> tr(P.twid, j);
+    TwiddleRun<+1, kTwRun> tr(P.twid, j);
 #pragma unroll
     for (int q = 0; q < R; ++q) base[Z.ix(j + q * s)] = q == 0 ? x[0] : cmul(x[q], tr.next(q));
   }
@@ -359,7 +366,7 @@ __device__ __forceinline__ void mid_pass(const Seqs Z, int span, const double2* 
       for (int q = 0; q < R; ++q) base[Z.ix(i0 + q)] = x[q];
       continue;
     }
-    TwiddleRun<SIGN> tr(tw, j * stw);
+    TwiddleRun<SIGN, kTwRun> tr(tw, j * stw);
     if constexpr (SIGN > 0) {
 #pragma unroll
       for (int r = 0; r < R; ++r) x[r] = base[Z.ix(i0 + r * s)];
@@ -944,7 +951,7 @@ __device__ __forceinline__ void ff_dif_first(const Plan& P, const double* line, 
       DFT<R, +1>::run(x);
     }
     double2* zp = z + pp * NP;
-    TwiddleRun<+1> tr(tw, j);
+    TwiddleRun<+1, kTwSpecial> tr(tw, j);
     if constexpr (S1 % 64 == 0) {
       const int jj = j ^ ((j >> 3) & 7);
 #pragma unroll
@@ -994,7 +1001,7 @@ __device__ __forceinline__ void ff_dit_store(const double2* z, int npair, const 
     const bool ok = pp < npair;
     const double2* zp = z + (ok ? pp : 0) * NP;
     double2 x[R];
-    TwiddleRun<-1> tr(tw, j);
+    TwiddleRun<-1, kTwSpecial> tr(tw, j);
     const int jj = j ^ ((j >> 3) & 7);
 #pragma unroll
     for (int q = 0; q < R; ++q) {
@@ -1352,13 +1359,13 @@ __device__ __forceinline__ void ff_half_first(const Plan& P, const double* line,
     for_constants(input, std::make_integer_sequence<int, R>{});
     DFT<R, +1>::run(x);
     double2* zp = z + pp * NP;
-    // w_N^(j (2 q + H)): running product, restarted from the table every eighth q
+    // w_N^(j (2 q + H)): running product (see TwiddleRun)
     const double2 w1 = twd<+1>(tw, 2 * j);
     double2 cur = make_double2(1.0, 0.0);
     const int jj = j ^ ((j >> 3) & 7);
 #pragma unroll
     for (int q = 0; q < R; ++q) {
-      cur = (q & 7) == 0 ? (H == 0 && q == 0 ? cur : twd<+1>(tw, j * (2 * q + H))) : cmul(cur, w1);
+      cur = q % kTwRun == 0 ? (H == 0 && q == 0 ? cur : twd<+1>(tw, j * (2 * q + H))) : cmul(cur, w1);
       zp[(jj ^ (((q * S1) >> 6) & 7)) + q * S1] = H == 0 && q == 0 ? x[0] : cmul(x[q], cur);
     }
   }
@@ -1385,7 +1392,7 @@ __device__ __forceinline__ void ff_half_store(const double2* z, int npair, const
     const int jj = j ^ ((j >> 3) & 7);
 #pragma unroll
     for (int q = 0; q < R; ++q) {
-      cur = q == 0 ? cur : (q & 7) == 0 ? twd<-1>(tw, 2 * j * q) : cmul(cur, w1);
+      cur = q == 0 ? cur : q % kTwRun == 0 ? twd<-1>(tw, 2 * j * q) : cmul(cur, w1);
       const double2 v = zp[(jj ^ (((q * S1) >> 6) & 7)) + q * S1];
       x[q] = q == 0 ? v : cmul(v, cur);
     }
