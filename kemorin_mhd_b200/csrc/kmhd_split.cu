@@ -368,11 +368,14 @@ __global__ void __launch_bounds__(kSliceThreads) k_slice_mr(Plan P, SliceTabs S,
   const int* dxa = S.dexp + S.deoff[m * kNT + t0];
   const int* dxb = S.dexp + S.deoff[m * kNT + t0 + 1];
   const int nx = ncolg * kst;
-  // column maxima: the high word of |x| (ordered like x), 0 for an all-zero column
-  int* colmax = reinterpret_cast<int*>(X + ((nx + 1) & ~1));
+  // column maxima as keys: the high word of |x| times two (ordered like |x|) plus
+  // kZeroKey, which takes NaN and infinities (exponent field 0x7ff) round to
+  // below zero's key: a column is scaled by its finite entries
+  constexpr unsigned kZeroKey = 1u << 21;
+  unsigned* colmax = reinterpret_cast<unsigned*>(X + ((nx + 1) & ~1));
   if (threadIdx.x < kGrpCols) colmax[threadIdx.x] = 0;
-  auto hiword = [](double x) { return __double2hiint(x) & 0x7fffffff; };
-  int mx[8] = {};  // vector groups: this thread's maxima of the eight columns
+  auto key = [](double x) { return ((unsigned)__double2hiint(x) << 1) + kZeroKey; };
+  unsigned mx[8] = {};  // vector groups: this thread's maxima of the eight columns
   // Forward with m > 0 and no theta padding, pass 1 writes every X entry
   // (both parts of the vector types, both slots of every field)
   if (!(FWD && m > 0 && P.nh % kTK == 0)) {
@@ -436,7 +439,7 @@ __global__ void __launch_bounds__(kSliceThreads) k_slice_mr(Plan P, SliceTabs S,
           double* x = X + (4 * p) * kst;
           auto put = [&](int q, int k, double v) {
             x[q * kst + k] = v;
-            mx[4 * p + q] = max(mx[4 * p + q], hiword(v));
+            mx[4 * p + q] = max(mx[4 * p + q], key(v));
           };
           put(0, th, A0[0] * s0);
           put(1, th, A0[1] * s0);
@@ -511,7 +514,7 @@ __global__ void __launch_bounds__(kSliceThreads) k_slice_mr(Plan P, SliceTabs S,
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             x[q * kst] = y[q];
-            mx[4 * t + q] = max(mx[4 * t + q], hiword(y[q]));
+            mx[4 * t + q] = max(mx[4 * t + q], key(y[q]));
           }
         }
       } else {
@@ -535,7 +538,7 @@ __global__ void __launch_bounds__(kSliceThreads) k_slice_mr(Plan P, SliceTabs S,
   if (vgrp) {
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
-      const int w = (int)__reduce_max_sync(0xffffffffu, (unsigned)mx[c]);
+      const unsigned w = __reduce_max_sync(0xffffffffu, mx[c]);
       if (lane == 0) atomicMax(colmax + c, w);
     }
   }
@@ -543,18 +546,18 @@ __global__ void __launch_bounds__(kSliceThreads) k_slice_mr(Plan P, SliceTabs S,
   if (!vgrp) {
     for (int c = warp; c < ncolg; c += nw) {
       const int kp = ctype(c) == t0 ? ga.kpad : gb.kpad;
-      int w = 0;
+      unsigned w = 0;
       for (int k = 2 * lane; k < kp; k += 64) {
         const double2 x2 = *reinterpret_cast<const double2*>(X + c * kst + k);
-        w = max(w, max(hiword(x2.x), hiword(x2.y)));
+        w = max(w, max(key(x2.x), key(x2.y)));
       }
-      w = (int)__reduce_max_sync(0xffffffffu, (unsigned)w);
+      w = __reduce_max_sync(0xffffffffu, w);
       if (lane == 0) colmax[c] = w;
     }
     __syncthreads();
   }
   // exponent of a column: smallest e with |x| < 2^e
-  auto colexp = [&](int c) { return colmax[c] > 0 ? (colmax[c] >> 20) - 1022 : 0; };
+  auto colexp = [&](int c) { return colmax[c] > kZeroKey ? (int)(colmax[c] >> 21) - 1023 : 0; };
   if (threadIdx.x < ncolg) {
     const int c = threadIdx.x;
     const ColRef cr = FWD ? colref_fwd(P, S, r, i0 + c) : colref_bwd(P, S, r, i0 + c);
@@ -601,7 +604,7 @@ __global__ void __launch_bounds__(kSliceThreads) k_slice_mr(Plan P, SliceTabs S,
         if (!eight) c = 4 * (t - t0) + q;
         else if (4 * fg + (q >> 1) < nF) c = 4 * (4 * fg + (q >> 1)) + 2 * (t - t0) + (q & 1);
         uint32_t wd[NS];
-        if (c >= 0 && colmax[c] > 0) {
+        if (c >= 0 && colmax[c] > kZeroKey) {
           const double sc = pow2((8 * NS - 2) - colexp(c));
           const double2 x01 = *reinterpret_cast<const double2*>(X + c * kst + k);
           const double2 x23 = *reinterpret_cast<const double2*>(X + c * kst + k + 2);
@@ -1417,7 +1420,7 @@ size_t slice_smem(const Plan& p, bool fwd, int ns) {
   const size_t kr = std::max(type_geo(tr, p.L, 0, p.nh).kpad, type_geo(tr + 1, p.L, 0, p.nh).kpad);
   const size_t nx = std::max(8 * kv, 4 * (size_t)nF * kr);
   const size_t stage = fwd ? (kSliceThreads / 32) * (size_t)ns * kSlab + 16 : 0;
-  return sizeof(double) * (nx + 1) + kGrpCols * sizeof(int) + stage;
+  return sizeof(double) * (nx + 1) + kGrpCols * sizeof(unsigned) + stage;
 }
 
 int split_slicer(SplitState* s, const Plan& p, bool fwd, const double* d_rj, long long ld, const int* cols,
