@@ -1193,21 +1193,36 @@ static EncodeTiledFn encode_tiled() {
   return fn;
 }
 
-// Tensor map of rtm_b for the staging of k_fft_cycle_f: [block][r][theta][block
-// row], box (block row, 1, 1, all blocks) = one line.  False when a line is not
-// one box (the caller then takes a kernel that does not stage by TMA).
+// Boxes of a line: a box has at most 256 doubles along the block row (16
+// components; 17, the most there are, take two).
+__host__ __device__ constexpr int line_boxes(int row) { return row > 256 ? 2 : 1; }
+
+// Tensor map of rtm_b for k_fft_cycle_f and _half: [block][r][theta][block row],
+// box (block row or half of it, 1, 1, all blocks).  False when a line is not
+// line_boxes() boxes (the caller then takes a kernel without the map).
 bool make_rtm_map(const Plan& p, CUtensorMap* map) {
-  const int row = rtm_row(p, p.ncb), nblk = rtm_blocks(p);
-  if (row > 256 || nblk > 256 || !p.rtm_b) return false;
+  const int row = rtm_row(p, p.ncb), nblk = rtm_blocks(p), nx = row / line_boxes(row);
+  if (nx > 256 || nblk > 256 || !p.rtm_b) return false;
   const cuuint64_t dims[4] = {(cuuint64_t)row, (cuuint64_t)p.nth, (cuuint64_t)p.nr, (cuuint64_t)nblk};
   const cuuint64_t strides[3] = {8ull * row, 8ull * row * p.nth, 8ull * row * p.nth * p.nr};
-  const cuuint32_t box[4] = {(cuuint32_t)row, 1, 1, (cuuint32_t)nblk};
+  const cuuint32_t box[4] = {(cuuint32_t)nx, 1, 1, (cuuint32_t)nblk};
   const cuuint32_t es[4] = {1, 1, 1, 1};
   const EncodeTiledFn enc = encode_tiled();
   if (!enc) return false;
   return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, const_cast<double*>(p.rtm_b), dims, strides, box, es,
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// L2 prefetch of a line's spectra (row: its block row); x of the second box is a
+// multiple of 16 bytes
+__device__ __forceinline__ void prefetch_l2(const CUtensorMap& tmap, int row, int th, int r) {
+  const int nx = row / line_boxes(row);
+  for (int x = 0; x < row; x += nx)
+    asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];\n" ::"l"(
+                     reinterpret_cast<uint64_t>(&tmap)),
+                 "r"(x), "r"(th), "r"(r), "r"(0)
+                 : "memory");
 }
 
 // fn(integral_constant<int, I>) for every I of the sequence
@@ -1256,11 +1271,7 @@ __global__ void __launch_bounds__(NT, kFftThreadsF / NT)
   if constexpr (!STG) {
     for (; line < nlines; line += gridDim.x) {
       const int th = line % P.nth, r = line / P.nth, next = line + gridDim.x;
-      if (threadIdx.x == 0 && next < nlines)
-        asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];\n" ::"l"(
-                         reinterpret_cast<uint64_t>(&tmap)),
-                     "r"(0), "r"(next % P.nth), "r"(next / P.nth), "r"(0)
-                     : "memory");
+      if (threadIdx.x == 0 && next < nlines) prefetch_l2(tmap, row, next % P.nth, next / P.nth);
       ff_dif_first<N, PR, true>(P, P.rtm_b + rtm_off(P, 0, th, r, ncb), (long long)P.nth * P.nr * row, ncb,
                                 nvb, mixb, z, npb, P.twid);
       __syncthreads();
@@ -1454,11 +1465,7 @@ __global__ void __launch_bounds__(kFftThreadsF, 1)
   const long long bsb = (long long)P.nth * P.nr * (2 * kRtmOrders) * ncb, bsf = (long long)P.nth * P.nr * (2 * kRtmOrders) * ncf;
   for (int line = line0 + blockIdx.x; line < nlines; line += gridDim.x) {
     const int th = line % P.nth, r = line / P.nth, next = line + gridDim.x;
-    if (threadIdx.x == 0 && next < nlines)
-      asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];\n" ::"l"(
-                       reinterpret_cast<uint64_t>(&tmap)),
-                   "r"(0), "r"(next % P.nth), "r"(next / P.nth), "r"(0)
-                   : "memory");
+    if (threadIdx.x == 0 && next < nlines) prefetch_l2(tmap, 2 * kRtmOrders * ncb, next % P.nth, next / P.nth);
     const double* src = P.rtm_b + rtm_off(P, 0, th, r, ncb);
     double* dst = P.rtm_f + rtm_off(P, 0, th, r, ncf);
     auto half = [&](auto hc) {

@@ -163,3 +163,24 @@ def test_fp64_sixteen_row_kernels(L, nr, fields):
     conv = dict(nvb=2, nsb=1, nvf=2, nsf=1, products=((0, 1, 0, 1.0), (1, 0, 0, 1.0), (2, 0, 1, 1.0)))
     sets = dict(FIELD_SETS, heat=HEAT, convection=conv, five=FIVE, one2=ONE2)
     assert run("cycle", SphConfig(L, 3 * (L + 1) // 2 + 1, 3 * (L + 1) if L == 255 else 480, nr, **sets[fields])) <= TOL
+
+
+# 17 components back, the most a set can have: the same line kernels as with 16,
+# so a scalar that no product uses changes no bit; against the oracle with it used
+@pytest.mark.gpu
+@pytest.mark.parametrize("L,nph", [(300, 1536), (40, 3072)])  # in place, half lines
+def test_seventeen_components(L, nph):
+    import torch
+    from kemorin_mhd_b200.sph_trans import SphTransform
+    prods = tuple((0, a, (a + 1) % 5, 1.0) for a in range(5)) + ((2, 0, 1, 1.0),)
+    res = []
+    for nsb in (1, 2):
+        cfg = SphConfig(L, 64, nph, 3, nvb=5, nsb=nsb, nvf=5, nsf=1, products=prods)
+        d = make_d_rj(SphConfig(L, 64, nph, 3, nvb=5, nsb=2, nvf=5, nsf=1, products=prods), seed=24)[:, :cfg.ncb]
+        out = torch.zeros((cfg.ncf, cfg.J * cfg.nr), dtype=torch.float64, device="cuda")
+        SphTransform(cfg).nonlinear_cycle(to_dev_fortran(np.asfortranarray(d)), out)
+        res.append(out)
+    assert torch.equal(res[0], res[1])
+    used = dict(nvb=5, nsb=2, nvf=4, nsf=2, products=((0, 0, 4, 1.0), (0, 1, 2, 1.0), (1, 3, 1, 1.0), (1, 4, 0, 1.0),
+                                                       (2, 0, 3, 1.0), (3, 0, 1, 1.0)))
+    assert run("cycle", SphConfig(L, 64, nph, 3, **used)) <= TOL
