@@ -304,7 +304,8 @@ __global__ void k_rot_buoyancy(long long J, int nr, int kchunk, const double* __
 
 // Blocks of 256 modes times ranges of at most eight radii, fewer where that
 // leaves less than eight CTAs per SM (Coriolis curl, L = 255, Nr = 129: 127 us;
-// four radii 135, sixteen 133, the whole shell's share of eight CTAs per SM 149).
+// four radii 135, sixteen 133, the whole shell's share of eight CTAs per SM 149);
+// more than eight where the ranges would pass the grid's 65535 rows.
 struct RadialGrid {
   dim3 grid;
   int kchunk;
@@ -317,7 +318,7 @@ RadialGrid radial_grid(long long J, int nr) {
   long long ks = std::max<long long>(1, (8LL * nsm + jb - 1) / std::max<long long>(jb, 1));
   if (ks > nr) ks = nr;
   RadialGrid g;
-  g.kchunk = std::min((int)((nr + ks - 1) / ks), 8);
+  g.kchunk = std::max(std::min((int)((nr + ks - 1) / ks), 8), (nr + 65534) / 65535);
   g.grid = dim3((unsigned)jb, (unsigned)((nr + g.kchunk - 1) / g.kchunk));
   return g;
 }

@@ -303,3 +303,22 @@ def test_rot_buoyancy_matches_oracle(double, host):
         tr.rot_buoyancy(t, 0, 2.5, 2, **kw)
         got = from_dev_fortran(t)[:, 2]
     assert _relerr(got, ref) <= 1e-14
+
+
+@pytest.mark.gpu
+def test_operators_on_many_radii():
+    """More radii than 65535 ranges of eight: the operators take longer ranges."""
+    import torch
+    from kemorin_mhd_b200.sph_trans import SphTransform
+    nr = 8 * 65535 + 9
+    cfg = SphConfig(1, 2, 4, nr, nvb=1, nsb=1, nvf=1, nsf=0, products=((1, 0, 0, 1.0),))
+    r = 1.0 + np.arange(nr) / nr
+    tr = SphTransform(cfg, radius=r)
+    d = torch.randn((8, cfg.J * nr), dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(5))
+    torch.cuda.synchronize()  # the handle has a stream of its own
+    tr.rot_buoyancy(d, 3, 1.5, 4)
+    rt = torch.from_numpy(r).cuda().repeat_interleave(cfg.J)
+    assert torch.equal(d[4], 1.5 * d[3] * rt)
+    tr.vorticity(d, 0, 5)  # its poloidal part is the toroidal part of the field
+    assert torch.equal(d[5], d[2])
+    tr.close()
