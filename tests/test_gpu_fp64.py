@@ -18,7 +18,7 @@ CFGS = [
     SphConfig(47, 73, 144, 6, name="L47_odd_nth"),          # odd N_theta: equator row
     SphConfig(16, 26, 40, 5, nvb=1, nsb=2, nvf=1, nsf=1,     # nph = 40 = 8*5
               products=((1, 0, 1, 0.5), (3, 0, 1, 2.0)), name="L16_mixed"),
-    SphConfig(63, 96, 3072, 3, name="L63_wide_nph3072"),    # line too wide for shared memory: pair by pair
+    SphConfig(63, 96, 3072, 3, name="L63_wide_nph3072"),    # line too wide for shared memory: in two halves
 ]
 
 

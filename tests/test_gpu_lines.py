@@ -2,7 +2,7 @@
 wrong: truncations that do not fill the eight-order blocks of the rtm records,
 odd component counts (a half pair at the end of a record), composite FFT radices
 (every one of them, first, middle and last), the short, staged, in-place and
-wide line kernels, and radial blocks of the separable transforms that end inside
+half line kernels, and radial blocks of the separable transforms that end inside
 a block.  Reference: the CPU FP64 oracle; bounds as in the FP64 tier's tests."""
 import numpy as np
 import pytest
@@ -70,15 +70,15 @@ def test_cycle_specialised_odd_set(L, nph):
                                   products=((0, 1, 0, 1.0), (1, 0, 0, 1.0), (2, 0, 1, 1.0)))) <= TOL
 
 
-# lines whose grid alone fits (in place), with sets of their own and without, and wide ones
+# lines whose grid alone fits (in place), with sets of their own and without, and
+# unpruned half lines (3072); lines that go pair by pair: test_gpu_wide.py
 @pytest.mark.gpu
-@pytest.mark.parametrize("fields", ["dynamo", "full", "five", "odd", "heat", "one2"])
-@pytest.mark.parametrize("L,nph", [(40, 1536), (511, 1536), (60, 1440), (40, 3072)])
+@pytest.mark.parametrize("L,nph,fields", [(L, nph, f) for L, nph in ((40, 1536), (511, 1536), (60, 1440), (40, 3072))
+                                          for f in ("dynamo", "full", "five", "odd", "heat", "one2")
+                                          if L != 511 or f not in ("odd", "heat", "one2")])  # those are staged
 def test_cycle_long_lines(L, nph, fields):
     sets = dict(FIELD_SETS, odd=ODD, five=FIVE, heat=HEAT, one2=ONE2)
     nth = 64 if L < 100 else 96
-    if L == 511 and fields in ("odd", "heat", "one2"):
-        pytest.skip("staged: covered by the short lines")
     assert run("cycle", SphConfig(L, nth, nph, 3, **sets[fields])) <= TOL
 
 

@@ -115,9 +115,10 @@ def test_split_dipole_modes_fp64(tier):
 @pytest.mark.gpu
 def test_split_vs_fp64_L1023():
     """cfg5 angular grid (L=1023, Ntheta=1536, Nphi=3072; wide lines go through
-    the FFT pair by pair): split tier against the FP64 GPU tier on the same
+    the FFT in two halves): split tier against the FP64 GPU tier on the same
     input (the CPU oracle at this L takes minutes; the FP64 tier is pinned to
-    the oracle at L <= 511 and on the wide-line path at L=63)."""
+    the oracle at L <= 511 and on unpruned half lines at L=63, and the pruned ones
+    of this grid to the separable transforms in test_gpu_wide.py)."""
     import torch
     from kemorin_mhd_b200.config import TIER_FP64
     from kemorin_mhd_b200.sph_trans import SphTransform
