@@ -866,16 +866,18 @@ cudaError_t run_fwd16(const Plan& p, double* d_rj, long long ld, const int* cols
 // terms scaled and added at the end), and both DMMA shapes round alike, so the
 // two kernels agree bit for bit: which one a launch takes does not show in the
 // results of a radial window or slab.  (Summing the +-m terms into the same
-// accumulators, m/sin P as a third operand, takes 3% less time at L = 255, Nr =
+// accumulators, m/sin P as a third operand, takes 1% less time at L = 255, Nr =
 // 129, but its theta and phi sums have 1.3 times the rounding error at L = 63 ..
-// 511.)  Operands come through a ring of four
-// cp.async stages, one barrier per chunk.  A CTA takes one field group, at most
+// 511.)  Operands come through a ring of six
+// cp.async stages, one barrier per two chunks.  A CTA takes one field group, at most
 // two vectors (20 accumulator tiles of four doubles per lane, and two per
 // scalar); groups start at even vectors, so no record pair is split between two
 // of them.  A group of one vector takes twice the radii, so that its warps have
-// as many columns to share the A fragments (default set at L = 255, Nr = 129,
-// two launches: 2.83 ms with eight radii, 2.74 so; one launch 2.72).
-constexpr int kRing16 = 4;
+// as many columns to share the A fragments.  Default set, ms at L = 255, Nr = 129
+// and L = 1023, Nr = 17: a launch per group, eight radii each 2.83, 22.8; sixteen for
+// the last 2.74, 23.7; one launch 2.72, 22.6; six stages and half the barriers
+// (four and one per chunk before) 2.67, 22.1.
+constexpr int kRing16 = 6;
 
 // group: CTA = (m, 64 latitudes, 8 RB radii), warp = (16 latitudes, 4 RB radii)
 template <int NV, int NS>
@@ -981,27 +983,34 @@ __device__ __forceinline__ void bwd16_group(const Plan& p, double* sm, int m, in
     }
   };
 
-#pragma unroll
-  for (int q = 0; q < kRing16 - 1; ++q) {
-    if (q < total) load(q);
-    cp_async_commit();
-  }
-  for (int step = 0; step < total; ++step) {
-    cp_async_wait<kRing16 - 2>();
-    __syncthreads();  // stage step has landed; every warp is done with the stage that load() overwrites
-    if (step + kRing16 - 1 < total) load(step + kRing16 - 1);
-    cp_async_commit();
-    if (!active) continue;
-    using One = std::integral_constant<int, 1>;
-    using All = std::integral_constant<int, RB>;
-    const bool all = rbi + 2 * (RB - 1) < nrb_here;
+  using One = std::integral_constant<int, 1>;
+  using All = std::integral_constant<int, RB>;
+  const bool all = RB == 1 || rbi + 2 * (RB - 1) < nrb_here;
+  auto compute_step = [&](int step) {
+    const int st = step % kRing16;
     if (step < n0) {
-      if (all) compute(step % kRing16, std::integral_constant<int, 0>(), All());
-      else compute(step % kRing16, std::integral_constant<int, 0>(), One());
+      if (all) compute(st, std::integral_constant<int, 0>(), All());
+      else compute(st, std::integral_constant<int, 0>(), One());
     } else {
-      if (all) compute(step % kRing16, std::integral_constant<int, 1>(), All());
-      else compute(step % kRing16, std::integral_constant<int, 1>(), One());
+      if (all) compute(st, std::integral_constant<int, 1>(), All());
+      else compute(st, std::integral_constant<int, 1>(), One());
     }
+  };
+  // two chunks per commit group and barrier
+  auto load2 = [&](int step) {
+    if (step < total) load(step);
+    if (step + 1 < total) load(step + 1);
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int q = 0; q < kRing16 - 2; q += 2) load2(q);
+  for (int step = 0; step < total; step += 2) {
+    cp_async_wait<kRing16 / 2 - 2>();
+    __syncthreads();  // both chunks have landed; every warp is done with the stages that load2() overwrites
+    load2(step + kRing16 - 2);
+    if (!active) continue;
+#pragma unroll 1  // the body is large
+    for (int q = step; q < min(step + 2, total); ++q) compute_step(q);
   }
   cp_async_wait<0>();
 
@@ -1214,8 +1223,8 @@ static int sm_count() {
 cudaError_t launch_leg_bwd_f64(const Plan& p, cudaStream_t s) {
   // The 16-row kernel takes a whole SM per CTA: it wins when there are two CTAs
   // (of eight radii) for each and at least two vectors to share a chunk's
-  // operands.  ms 8-row -> 16-row: L = 255, Nr = 129 3.19 -> 2.72; L = 511, Nr = 17
-  // 3.24 -> 3.08; L = 127, Nr = 17 (768 CTAs) 0.109 -> 0.101; but L = 31, Nr = 33
+  // operands.  ms 8-row -> 16-row: L = 255, Nr = 129 3.19 -> 2.67; L = 511, Nr = 17
+  // 3.24 -> 3.01; L = 127, Nr = 17 (768 CTAs) 0.109 -> 0.101; but L = 31, Nr = 33
   // (160) 0.016 -> 0.019, L = 63, Nr = 9 (128) 0.018 -> 0.020, one vector at
   // L = 255, Nr = 33 0.309 -> 0.322.  The launch is a window or slab of the shell
   // as often as not; the results are the same on both sides.
