@@ -740,7 +740,7 @@ __device__ __forceinline__ int pair_comp(int pp, int c, int nv, int mixed) {
 // takes one pair of rad neighbouring radii of one latitude: its grid accesses
 // are rad contiguous doubles (with one radius per CTA every lane of a grid
 // access was a sector of its own: at L = 127, Nr = 65 the inverse took 0.65 ms
-// and the forward 0.52 ms; see grid_radii for the present ones).  Sequences lie
+// and the forward 0.52 ms, now 0.35 and 0.33).  Sequences lie
 // N + 1 entries apart, so the radii of one point are in different banks.
 // Block order: pair fastest, then radial block, then latitude.
 __global__ void __launch_bounds__(kGridThreads, 2)
@@ -835,10 +835,10 @@ constexpr int kFftThreadsF = 384;
 // shared memory, so one CTA has them all; the shorter lines leave room for
 // several CTAs per SM, whose barriers and record stores then overlap, and a
 // pass of theirs has fewer items than 384 threads could take (N / F0 or N / M
-// per pair).  FFT ms at 384 threads -> here: L = 255, Nr = 129 (N = 768)
-// 2.64 -> 2.42 (160 threads 2.53); L = 127, Nr = 65 (N = 384) 0.390 -> 0.292
-// (128 threads 0.296); L = 63, Nr = 65 (N = 192) 0.153 -> 0.081 (96 threads
-// 0.085); L = 31, Nr = 33 (N = 96) 0.034 -> 0.016 (64 threads 0.018).
+// per pair).  FFT ms at 384 threads -> here: L = 255, Nr = 129 (N = 768) 2.04 ->
+// 1.75; L = 127, Nr = 65 (N = 384) 0.306 -> 0.234; L = 63, Nr = 65 (N = 192) 0.118 ->
+// 0.071; L = 31, Nr = 33 (N = 96) 0.027 -> 0.015.  (160, 128, 96 and 64 threads were
+// slower than these, before the passes were rebuilt.)
 __host__ __device__ constexpr int ff_threads(int n) { return n == 768 ? 192 : n == 384 ? 96 : n == 192 ? 64 : n == 96 ? 32 : kFftThreadsF; }
 
 __host__ __device__ constexpr int ff_mid(int n) { return (n % 64 == 0 && (n / 64 == 3 || n / 64 == 6 || n / 64 == 12 || n / 64 == 24)) ? 16 : 4; }
@@ -1637,11 +1637,6 @@ cudaError_t launch_selftest_fft_wait(int* err, cudaStream_t s) {
 
 bool fft_line_fits(const Plan& p) {
   return smem_cycle(p) <= 227 * 1024 || smem_cycle_f(p) <= 227 * 1024;
-}
-
-size_t fft_smem_bytes(const Plan& p, int npair) {
-  (void)npair;
-  return smem_cycle(p);
 }
 
 size_t smem_direct(const Plan& p) {

@@ -13,7 +13,6 @@
 
 namespace kmhd {
 size_t bwd_smem_bytes(int nv, int ns);
-size_t fft_smem_bytes(const Plan& p, int npair);
 }  // namespace kmhd
 
 using namespace kmhd;
