@@ -134,11 +134,11 @@ __host__ __device__ __forceinline__ int rtm_pair(const Plan& P, int m, int q, in
 // the reads of the first inverse pass, the products and the stores of the last
 // forward pass know; the records stay as they are.
 // Backward always (Plan::mixb): T of the default set takes an error (2-norm) of 5.6,
-// 5.6, 21 and 21e-15 at L = 127, 255, 511 and 1023 from B_r, 0.9, 0.5, 1.5 and
-// 1.3e-15 from B_theta.
+// 5.6, 21 and 21e-15 at L = 127, 255, 511 and 1023 from B_r, 0.5, 0.4, 1.2 and
+// 0.8e-15 from B_theta.
 // Forward (Plan::mixf) unless the scalar is a dot product, which is as large as a
 // cross product's r: u T's columns at L = 511 have 18.2, 3.0 and 5.8e-15 with
-// (r, u . omega) in one FFT, 18.0, 15.4 and 28.5e-15 with (phi, u . omega), and the two
+// (r, u . omega) in one FFT, 18.0, 15.4 and 28.5e-15 with (phi, u . omega); and the two
 // half sectors of each store cost 5% of the FFT's time.
 // The mixed pair's index, -1 without one.
 __host__ __device__ __forceinline__ constexpr int mixed_pair(int nv, int ns) {
